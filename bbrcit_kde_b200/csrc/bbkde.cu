@@ -76,14 +76,23 @@ struct PackCache {
   DevBuf rec, ext;
 };
 
-// Morton-sorted FP32 records of the reference set and their culling tiles,
-// valid for the packed records with the same key.
-struct CullCache {
+// Curve-sorted FP32 records of the reference set (valid for the packed records
+// with the same key) and their culling tiles at one size (valid likewise): [0]
+// kRefTile references (the factored grid kernels), [1] kCullUnit (the pair form).
+struct CullLevel {
   PackKey key;
-  DevBuf rec, ext, tiles, groups;
+  DevBuf tiles, groups;
   int n_tiles = 0;
   int n_groups = 0;
 };
+struct CullCache {
+  PackKey key;
+  DevBuf rec, ext;
+  CullLevel level[2];
+  DevBuf perm;                      // curve order of the coordinates
+  uint64_t perm_version = ~0ull;    // ... at this coordinate version
+};
+constexpr int kCullLevelSize[2] = {kRefTile, kCullUnit};
 
 struct QueryCache {
   int set = -1;
@@ -125,8 +134,8 @@ struct bbkde_ctx {
   // culled evaluation: sorted references, sort scratch, sorted queries, per-block
   // bounds; dense-grid pipeline buffers
   CullCache cull;
-  DevBuf ms_keys, ms_keys2, ms_perm, ms_perm2, ms_box, ms_tmp, cq_x, cq_y, cq_out, cb_bound,
-      cb_smin, cb_tiles, cb_stats, cb_key, cb_key2, cb_sched;
+  DevBuf ms_keys, ms_keys2, ms_perm, ms_perm2, ms_box, ms_tmp, cq_out, cb_bound, cb_smin,
+      cb_tiles, cb_stats, cb_key, cb_key2, cb_sched;
   DevBuf gr_pred, gr_order, gr_tmin, gr_tmax, gr_bad, gr_terr, gr_flag, gr_flag_ord, gr_list,
       gr_nsel, gr_counts, gr_gmax, gr_lat_order, gr_lat_exact, gr_lat_net, gr_q_order, gr_q_exact,
       gr_q_net, gr_resid, gr_cand_ord, gr_cand_xy, gr_cand_net, gr_out, gr_part, gr_rl_idx,
@@ -741,9 +750,10 @@ int bbkde_ctx_destroy(bbkde_ctx *c) {
                     &c->cv_counter, &c->cv_h, &c->cv_lut, &c->cv_part, &c->cv_hist,
                     &c->cv_out, &c->cv_parts})
     release(*b);
-  for (DevBuf *b : {&c->cull.rec, &c->cull.ext, &c->cull.tiles, &c->cull.groups, &c->ms_keys,
-                    &c->ms_keys2, &c->ms_perm, &c->ms_perm2, &c->ms_box, &c->ms_tmp, &c->cq_x,
-                    &c->cq_y, &c->cq_out, &c->cb_bound, &c->cb_smin, &c->cb_tiles, &c->cb_stats,
+  for (DevBuf *b : {&c->cull.rec, &c->cull.ext, &c->cull.perm, &c->cull.level[0].tiles,
+                    &c->cull.level[0].groups, &c->cull.level[1].tiles, &c->cull.level[1].groups,
+                    &c->ms_keys, &c->ms_keys2, &c->ms_perm, &c->ms_perm2, &c->ms_box, &c->ms_tmp,
+                    &c->cq_out, &c->cb_bound, &c->cb_smin, &c->cb_tiles, &c->cb_stats,
                     &c->cb_key, &c->cb_key2, &c->cb_sched,
                     &c->gr_pred, &c->gr_order, &c->gr_tmin, &c->gr_tmax, &c->gr_bad,
                     &c->gr_terr, &c->gr_flag, &c->gr_flag_ord, &c->gr_list, &c->gr_nsel,
@@ -1416,6 +1426,11 @@ namespace {
 // Near-field width of the culled sum in log2 units: the first pass sums every
 // tile whose bound is within 2^-24 of the block's largest.
 constexpr float kCullCut = 24.0f;
+// The same for the pair form: the near-field sum only sets the far threshold, and a
+// narrower first pass leaves queries in thin regions, whose absolute allowance
+// needs nothing more, with fewer tiles (24 measured 1-5% slower at 20,011-400,000
+// references).
+constexpr float kCullCutPair = 10.0f;
 
 // Automatic probe set of the grid pipeline (bbkde_grid_config.probes = 0): 5 probes
 // while the tile span is at most this many narrowest kernel widths, else 9.
@@ -1428,86 +1443,93 @@ constexpr double kGridProbeSpan = 0.75;
 // 10 narrowest widths 20% faster, of 33 and 80 widths 5-7% slower).
 constexpr double kGridLatticeSpan = 16.0;
 
-// Morton order of n points (x[i * stride], y[i * stride]; y null for 1-D):
-// *perm_out = the sorted permutation (valid until the next sort).
-int morton_sort(bbkde_ctx *c, const float *x, const float *y, int stride, int64_t n,
-                const int **perm_out) {
+// Curve order of n points (x[i * stride], y[i * stride]; y null for 1-D) into
+// `perm` (n ints).
+int curve_sort(bbkde_ctx *c, const float *x, const float *y, int stride, int64_t n,
+               DevBuf &perm) {
   if (n > INT32_MAX) return fail(c, BBKDE_OUT_OF_RANGE, "more than 2^31 - 1 points");
   TRY(ensure(c, c->ms_keys, (size_t)n * sizeof(unsigned)));
   TRY(ensure(c, c->ms_keys2, (size_t)n * sizeof(unsigned)));
   TRY(ensure(c, c->ms_perm, (size_t)n * sizeof(int)));
-  TRY(ensure(c, c->ms_perm2, (size_t)n * sizeof(int)));
+  TRY(ensure(c, perm, (size_t)n * sizeof(int)));
   TRY(ensure(c, c->ms_box, 4 * sizeof(unsigned)));
   CUDA_TRY(c, cudaMemsetAsync(c->ms_box.p, 0xff, 2 * sizeof(unsigned), c->stream));
   CUDA_TRY(c, cudaMemsetAsync(c->ms_box.as<unsigned>() + 2, 0, 2 * sizeof(unsigned), c->stream));
-  const unsigned gb = std::min<unsigned>(grid1d(n), (unsigned)c->sm_count * 8);
+  const unsigned gb = std::min<unsigned>(grid1d(n), (unsigned)c->sm_count);
   k_bbox<<<gb, 256, 0, c->stream>>>(x, y, stride, n, c->ms_box.as<unsigned>());
   COUNT_LAUNCH(c);
-  k_morton<<<grid1d(n), 256, 0, c->stream>>>(x, y, stride, n, c->ms_box.as<unsigned>(),
-                                             c->ms_keys.as<unsigned>(), c->ms_perm.as<int>());
+  k_curve_keys<<<grid1d(n), 256, 0, c->stream>>>(x, y, stride, n, c->ms_box.as<unsigned>(),
+                                                 c->ms_keys.as<unsigned>(), c->ms_perm.as<int>());
   COUNT_LAUNCH(c);
   CUDA_TRY(c, cudaGetLastError());
   size_t tmp = 0;
   CUDA_TRY(c, cub::DeviceRadixSort::SortPairs(nullptr, tmp, c->ms_keys.as<unsigned>(),
                                               c->ms_keys2.as<unsigned>(), c->ms_perm.as<int>(),
-                                              c->ms_perm2.as<int>(), (int)n, 0, 32, c->stream));
+                                              perm.as<int>(), (int)n, 0, 32, c->stream));
   TRY(ensure(c, c->ms_tmp, tmp));
   CUDA_TRY(c, cub::DeviceRadixSort::SortPairs(c->ms_tmp.p, tmp, c->ms_keys.as<unsigned>(),
                                               c->ms_keys2.as<unsigned>(), c->ms_perm.as<int>(),
-                                              c->ms_perm2.as<int>(), (int)n, 0, 32, c->stream));
+                                              perm.as<int>(), (int)n, 0, 32, c->stream));
   c->launch_total += 4;   // CUB's onesweep radix sort: histogram + passes
-  *perm_out = c->ms_perm2.as<int>();
   return BBKDE_OK;
 }
 
-// Sorted records and culling tiles of the reference set for `r` (cached).
-int ensure_culled(bbkde_ctx *c, const Resolved &r) {
+// Sorted records and culling tiles (of kCullLevelSize[level] references) of the
+// reference set for `r`, cached. The order depends on the coordinates alone, so
+// new masses, local bandwidths or kernels re-gather the records without a sort.
+int ensure_culled(bbkde_ctx *c, const Resolved &r, int level) {
   TRY(ensure_pack(c, r, false));
   CullCache &cc = c->cull;
-  if (cc.key == c->pack32.key) return BBKDE_OK;
-  const int64_t n = c->sets[BBKDE_REFERENCE].n;
-  cc.n_tiles = (int)((n + kRefTile - 1) / kRefTile);
-  cc.n_groups = (cc.n_tiles + kGroupTiles - 1) / kGroupTiles;
-  if (n > 0) {
-    TRY(ensure(c, cc.rec, (size_t)n * sizeof(float4)));
-    TRY(ensure(c, cc.ext, (size_t)n * sizeof(float)));
-    TRY(ensure(c, cc.tiles, (size_t)cc.n_tiles * sizeof(RefTile)));
-    TRY(ensure(c, cc.groups, (size_t)cc.n_groups * sizeof(RefTile)));
-    const float *rx = c->pack32.rec.as<float>();
-    const int *perm = nullptr;
-    TRY(morton_sort(c, rx, r.dim == 2 ? rx + 1 : nullptr, 4, n, &perm));
-    k_gather_rec<<<grid1d(n), 256, 0, c->stream>>>(c->pack32.rec.as<float4>(),
-                                                   c->pack32.ext.as<float>(), perm, n,
-                                                   cc.rec.as<float4>(), cc.ext.as<float>());
-    COUNT_LAUNCH(c);
-    const float *tex = (op_has_extra(r.op) && r.dim == 2) ? cc.ext.as<float>() : nullptr;
-    const unsigned tb = grid1d((int64_t)cc.n_tiles * 32);
-    if (r.dim == 2)
-      k_ref_tiles<2><<<tb, 256, 0, c->stream>>>(cc.rec.as<float4>(), tex, n, cc.n_tiles,
-                                                cc.tiles.as<RefTile>());
-    else
-      k_ref_tiles<1><<<tb, 256, 0, c->stream>>>(cc.rec.as<float4>(), tex, n, cc.n_tiles,
-                                                cc.tiles.as<RefTile>());
-    COUNT_LAUNCH(c);
-    k_ref_groups<<<grid1d(cc.n_groups), 256, 0, c->stream>>>(
-        cc.tiles.as<RefTile>(), cc.n_tiles, cc.n_groups, cc.groups.as<RefTile>());
-    COUNT_LAUNCH(c);
-    CUDA_TRY(c, cudaGetLastError());
+  CullLevel &lv = cc.level[level];
+  const PointSet &s = c->sets[BBKDE_REFERENCE];
+  const int64_t n = s.n;
+  if (!(cc.key == c->pack32.key)) {
+    if (n > 0) {
+      TRY(ensure(c, cc.rec, (size_t)n * sizeof(float4)));
+      TRY(ensure(c, cc.ext, (size_t)n * sizeof(float)));
+      if (cc.perm_version != s.coord_version) {
+        const float *rx = c->pack32.rec.as<float>();
+        cc.perm_version = ~0ull;
+        TRY(curve_sort(c, rx, r.dim == 2 ? rx + 1 : nullptr, 4, n, cc.perm));
+        cc.perm_version = s.coord_version;
+      }
+      k_gather_rec<<<grid1d(n), 256, 0, c->stream>>>(c->pack32.rec.as<float4>(),
+                                                     c->pack32.ext.as<float>(), cc.perm.as<int>(),
+                                                     n, cc.rec.as<float4>(), cc.ext.as<float>());
+      COUNT_LAUNCH(c);
+      CUDA_TRY(c, cudaGetLastError());
+    }
+    cc.key = c->pack32.key;
   }
-  cc.key = c->pack32.key;
+  if (!(lv.key == cc.key)) {
+    const int size = kCullLevelSize[level];
+    lv.n_tiles = (int)((n + size - 1) / size);
+    lv.n_groups = (lv.n_tiles + kGroupTiles - 1) / kGroupTiles;
+    if (n > 0) {
+      TRY(ensure(c, lv.tiles, (size_t)lv.n_tiles * sizeof(RefTile)));
+      TRY(ensure(c, lv.groups, (size_t)lv.n_groups * sizeof(RefTile)));
+      const float *tex = (op_has_extra(r.op) && r.dim == 2) ? cc.ext.as<float>() : nullptr;
+      const unsigned tb = grid1d((int64_t)lv.n_tiles * 32);
+      if (r.dim == 2)
+        k_ref_tiles<2><<<tb, 256, 0, c->stream>>>(cc.rec.as<float4>(), tex, n, size, lv.n_tiles,
+                                                  lv.tiles.as<RefTile>());
+      else
+        k_ref_tiles<1><<<tb, 256, 0, c->stream>>>(cc.rec.as<float4>(), tex, n, size, lv.n_tiles,
+                                                  lv.tiles.as<RefTile>());
+      COUNT_LAUNCH(c);
+      k_ref_groups<<<grid1d((int64_t)lv.n_groups * kGroupTiles), 256, 0, c->stream>>>(
+          lv.tiles.as<RefTile>(), lv.n_tiles, lv.n_groups, lv.groups.as<RefTile>());
+      COUNT_LAUNCH(c);
+      CUDA_TRY(c, cudaGetLastError());
+    }
+    lv.key = cc.key;
+  }
   return BBKDE_OK;
 }
 
-// Launch shapes of the culled sum: 0 = 1024 queries per block (128 threads x 8),
-// 1 = 256 queries per block (64 threads x 4).
-constexpr int kCullQpb[2] = {1024, 256};
-
 template <int OP, int D>
-void launch_cull_op(int shape, unsigned nblk, cudaStream_t st, const CullArgs &a) {
-  if (shape == 0)
-    k_pair_sum_culled<OP, D, 8, 128, 4><<<nblk, 128, 0, st>>>(a);
-  else
-    k_pair_sum_culled<OP, D, 4, 64, 8><<<nblk, 64, 0, st>>>(a);
+void launch_cull_op(unsigned nblk, cudaStream_t st, const CullArgs &a) {
+  k_pair_sum_culled<OP, D><<<nblk, 32 * kCullWarps, 0, st>>>(a);
 }
 
 // Tile-16 lists shorter than this many tiles per SM are split: each tile's
@@ -1621,10 +1643,13 @@ int sep_parts(const bbkde_ctx *c, int tile, unsigned nblk) {
 // part stays below max(rel * S, abs_n) / 2, and *ratio is then the worst skipped
 // bound over that allowance; with abs_n = 0 it is the worst bound over S.
 // sep_tc: a tile-32 factored sum runs on the tensor cores (k_pair_sum_culled_sep_tc).
-int launch_culled(bbkde_ctx *c, const Resolved &r, int shape, unsigned nblk,
-                  const CullQueries &q, double rel, bool full, double *pairs, double *ratio,
+int launch_culled(bbkde_ctx *c, const Resolved &r, unsigned nblk, const CullQueries &q,
+                  double rel, bool full, double *pairs, double *ratio,
                   int sep_tile = 0, double abs_n = 0.0, bool sep_tc = false) {
   if (nblk == 0) return BBKDE_OK;
+  const int level = sep_tile > 0 ? 0 : 1;
+  TRY(ensure_culled(c, r, level));
+  const CullLevel &lv = c->cull.level[level];
   TRY(ensure(c, c->cb_bound, (size_t)nblk * sizeof(double)));
   TRY(ensure(c, c->cb_smin, (size_t)nblk * sizeof(double)));
   TRY(ensure(c, c->cb_tiles, (size_t)nblk * sizeof(int)));
@@ -1635,12 +1660,12 @@ int launch_culled(bbkde_ctx *c, const Resolved &r, int shape, unsigned nblk,
   CullArgs a;
   a.refs = c->cull.rec.as<float4>();
   a.extra = c->cull.ext.as<float>();
-  a.tiles = c->cull.tiles.as<RefTile>();
-  a.groups = c->cull.groups.as<RefTile>();
-  a.n_tiles = c->cull.n_tiles;
-  a.n_groups = c->cull.n_groups;
+  a.tiles = lv.tiles.as<RefTile>();
+  a.groups = lv.groups.as<RefTile>();
+  a.n_tiles = lv.n_tiles;
+  a.n_groups = lv.n_groups;
   a.n_ref = c->sets[BBKDE_REFERENCE].n;
-  a.cut = full ? INFINITY : kCullCut;
+  a.cut = full ? INFINITY : sep_tile > 0 ? kCullCut : kCullCutPair;
   a.rel = rel;
   a.abs_n = abs_n;
   a.q = q;
@@ -1679,19 +1704,19 @@ int launch_culled(bbkde_ctx *c, const Resolved &r, int shape, unsigned nblk,
     }
   } else switch (r.op) {
     case OP_GAUSS_ISO:
-      d2 ? launch_cull_op<OP_GAUSS_ISO, 2>(shape, nblk, c->stream, a)
-         : launch_cull_op<OP_GAUSS_ISO, 1>(shape, nblk, c->stream, a);
+      d2 ? launch_cull_op<OP_GAUSS_ISO, 2>(nblk, c->stream, a)
+         : launch_cull_op<OP_GAUSS_ISO, 1>(nblk, c->stream, a);
       break;
-    case OP_GAUSS_PROD: launch_cull_op<OP_GAUSS_PROD, 2>(shape, nblk, c->stream, a); break;
+    case OP_GAUSS_PROD: launch_cull_op<OP_GAUSS_PROD, 2>(nblk, c->stream, a); break;
     case OP_EPAN_ISO:
-      d2 ? launch_cull_op<OP_EPAN_ISO, 2>(shape, nblk, c->stream, a)
-         : launch_cull_op<OP_EPAN_ISO, 1>(shape, nblk, c->stream, a);
+      d2 ? launch_cull_op<OP_EPAN_ISO, 2>(nblk, c->stream, a)
+         : launch_cull_op<OP_EPAN_ISO, 1>(nblk, c->stream, a);
       break;
-    case OP_EPAN_PROD: launch_cull_op<OP_EPAN_PROD, 2>(shape, nblk, c->stream, a); break;
+    case OP_EPAN_PROD: launch_cull_op<OP_EPAN_PROD, 2>(nblk, c->stream, a); break;
     default: return fail(c, BBKDE_UNSUPPORTED, "culled sum: unsupported kernel");
   }
   COUNT_LAUNCH(c);
-  k_cull_stats<<<1, 256, 0, c->stream>>>(a.blk_bound, a.blk_smin, a.blk_tiles, (int)nblk,
+  k_cull_stats<<<1, 1024, 0, c->stream>>>(a.blk_bound, a.blk_smin, a.blk_tiles, (int)nblk,
                                          c->cb_stats.as<double>());
   COUNT_LAUNCH(c);
   CUDA_TRY(c, cudaGetLastError());
@@ -1706,7 +1731,9 @@ int launch_culled(bbkde_ctx *c, const Resolved &r, int shape, unsigned nblk,
       return fail(c, BBKDE_CUDA_ERROR,
                   "culled sum: a tensor-core wait expired (the results are not written)");
   }
-  if (pairs) *pairs += st[1] * kRefTile * kCullQpb[shape];
+  if (pairs)
+    *pairs += st[1] * (sep_tile > 0 ? (double)kRefTile * sep_tile * sep_tile
+                                    : (double)kCullUnit * kCullQpb);
   if (ratio) *ratio = std::max(*ratio, abs_n > 0.0 ? st[0] : st[0] * rel);
   return BBKDE_OK;
 }
@@ -1748,34 +1775,25 @@ int eval_culled_impl(bbkde_ctx *c, const bbkde_kernel_desc *k, int normalized, d
   if (rs.n == 0) {
     CUDA_TRY(c, cudaMemsetAsync(dst, 0, (size_t)nq * sizeof(double), c->stream));
   } else {
-    TRY(ensure_culled(c, r));
+    TRY(ensure_culled(c, r, 1));
     const void *qx = nullptr, *qy = nullptr;
     TRY(ensure_queries(c, BBKDE_QUERY, false, &qx, &qy));
     const float *fx = static_cast<const float *>(qx), *fy = static_cast<const float *>(qy);
-    const int *perm = nullptr;
-    TRY(morton_sort(c, fx, r.dim == 2 ? fy : nullptr, 1, nq, &perm));
-    TRY(ensure(c, c->cq_x, (size_t)nq * sizeof(float)));
-    TRY(ensure(c, c->cq_y, (size_t)nq * sizeof(float)));
-    TRY(ensure(c, c->cq_out, (size_t)nq * sizeof(double)));
-    k_gather_xy<<<grid1d(nq), 256, 0, c->stream>>>(fx, r.dim == 2 ? fy : nullptr, perm, nq,
-                                                   c->cq_x.as<float>(), c->cq_y.as<float>());
-    COUNT_LAUNCH(c);
+    TRY(curve_sort(c, fx, r.dim == 2 ? fy : nullptr, 1, nq, c->ms_perm2));
     CullQueries q = {};
     q.mode = 0;
-    q.qx = c->cq_x.as<float>();
-    q.qy = c->cq_y.as<float>();
+    q.qx = fx;
+    q.qy = fy;
+    q.stride = 1;
+    q.perm = c->ms_perm2.as<int>();
     q.count = nq;
-    q.out = c->cq_out.as<double>();
+    q.out = dst;
     q.scale = normalized ? r.norm : 1.0;
-    const unsigned nblk = (unsigned)((nq + kCullQpb[0] - 1) / kCullQpb[0]);
+    const unsigned nblk = (unsigned)((nq + kCullQpb - 1) / kCullQpb);
     CUDA_TRY(c, cudaEventRecord(c->ev0, c->stream));
-    TRY(launch_culled(c, r, 0, nblk, q, rel_tol, false, &st.pairs, &st.max_bound_ratio, 0,
-                      abs_n));
+    TRY(launch_culled(c, r, nblk, q, rel_tol, false, &st.pairs, &st.max_bound_ratio, 0, abs_n));
     CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
-    k_scatter<<<grid1d(nq), 256, 0, c->stream>>>(c->cq_out.as<double>(), perm, nq, dst);
-    COUNT_LAUNCH(c);
-    CUDA_TRY(c, cudaGetLastError());
-    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    CUDA_TRY(c, cudaEventSynchronize(c->ev1));
     float ms = 0.f;
     CUDA_TRY(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     st.kernel_ms = ms;
@@ -1820,39 +1838,27 @@ namespace {
 // self term included: out[i] (device, the set's order) within max(rel * f_i,
 // abs_err) / 2 of f_i = C sum_j m_j U(x_i, x_j) (abs_err in normalised density
 // units), FP32-compensated. Queries are the set's own FP32
-// coordinates in Morton order. *pairs gets the pairs at tile granularity and
+// coordinates in curve order. *pairs gets the pairs at tile granularity and
 // *ms the device time of the culled launch.
 int culled_self_sum(bbkde_ctx *c, const Resolved &r, double rel, double abs_err, double *out,
                     double *pairs, float *ms) {
   const int64_t n = c->sets[BBKDE_REFERENCE].n;
-  TRY(ensure_culled(c, r));
-  const void *qx = nullptr, *qy = nullptr;
-  TRY(ensure_queries(c, BBKDE_REFERENCE, false, &qx, &qy));
-  const float *fx = static_cast<const float *>(qx), *fy = static_cast<const float *>(qy);
-  const int *perm = nullptr;
-  TRY(morton_sort(c, fx, r.dim == 2 ? fy : nullptr, 1, n, &perm));
-  TRY(ensure(c, c->cq_x, (size_t)n * sizeof(float)));
-  TRY(ensure(c, c->cq_y, (size_t)n * sizeof(float)));
-  TRY(ensure(c, c->cq_out, (size_t)std::max<int64_t>(n, kWlogBlocks) * sizeof(double)));
-  k_gather_xy<<<grid1d(n), 256, 0, c->stream>>>(fx, r.dim == 2 ? fy : nullptr, perm, n,
-                                                c->cq_x.as<float>(), c->cq_y.as<float>());
-  COUNT_LAUNCH(c);
+  TRY(ensure_culled(c, r, 1));
   CullQueries q = {};
   q.mode = 0;
-  q.qx = c->cq_x.as<float>();
-  q.qy = c->cq_y.as<float>();
+  q.qx = c->pack32.rec.as<float>();   // the records' own coordinates, 4 floats apart
+  q.qy = q.qx + 1;
+  q.stride = 4;
+  q.perm = c->cull.perm.as<int>();
   q.count = n;
-  q.out = c->cq_out.as<double>();
+  q.out = out;
   q.scale = r.norm;
   double ratio = 0.0;
   *pairs = 0.0;
   CUDA_TRY(c, cudaEventRecord(c->ev0, c->stream));
-  TRY(launch_culled(c, r, 0, (unsigned)((n + kCullQpb[0] - 1) / kCullQpb[0]), q, rel, false,
-                    pairs, &ratio, 0, abs_err > 0.0 ? abs_err / r.norm : 0.0));
+  TRY(launch_culled(c, r, (unsigned)((n + kCullQpb - 1) / kCullQpb), q, rel, false, pairs,
+                    &ratio, 0, abs_err > 0.0 ? abs_err / r.norm : 0.0));
   CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
-  k_scatter<<<grid1d(n), 256, 0, c->stream>>>(c->cq_out.as<double>(), perm, n, out);
-  COUNT_LAUNCH(c);
-  CUDA_TRY(c, cudaGetLastError());
   CUDA_TRY(c, cudaEventSynchronize(c->ev1));
   CUDA_TRY(c, cudaEventElapsedTime(ms, c->ev0, c->ev1));
   return BBKDE_OK;
@@ -2058,11 +2064,13 @@ int grid_exact(bbkde_ctx *c, const Resolved &r, const GridDesc &g, const int *li
   q.gdy = g.dy;
   q.out = out;
   q.scale = r.norm;
-  const int shape = g.tile == 32 ? 0 : 1;
   const int sep = (!pair_form && r.dim == 2 && op_separable(r.op)) ? g.tile : 0;
   const bool tc = sep == 32 && (tensor_cores == 2 ||
                                 (tensor_cores == 0 && !full && rel >= kSepTcMinRel));
-  return launch_culled(c, r, shape, (unsigned)n, q, rel, full, pairs, ratio, sep, 0.0, tc);
+  const int64_t pieces = (int64_t)(g.tile / kCullPiece) * (g.tile / kCullPiece);
+  const int64_t nblk = sep > 0 ? n : n * pieces;
+  if (nblk > INT32_MAX) return fail(c, BBKDE_OUT_OF_RANGE, "grid: too many tiles");
+  return launch_culled(c, r, (unsigned)nblk, q, rel, full, pairs, ratio, sep, 0.0, tc);
 }
 
 }  // namespace
@@ -2152,7 +2160,6 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
     if (stats) *stats = st;
     return BBKDE_OK;
   }
-  TRY(ensure_culled(c, r));
   TRY(tile_order(c, g, c->gr_order));
   TRY(ensure(c, c->gr_flag, (size_t)ntiles * sizeof(int)));
   TRY(ensure(c, c->gr_flag_ord, (size_t)ntiles * sizeof(int)));

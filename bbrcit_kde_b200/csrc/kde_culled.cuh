@@ -1,13 +1,13 @@
 // Culled direct sum: the pair sum over the reference tiles that can contribute,
 // with a rigorous bound on the part that is skipped.
 //
-// References are sorted along a Morton curve (host code) and packed exactly as
-// for k_pair_sum_f32x2; every run of kRefTile consecutive sorted references is a
-// "reference tile" with a bounding box, its widest kernel scale and its mass.
-// The queries of a block fall into QPT "slots" (slot k = the k-th query of every
-// thread: a compact strip of a grid tile, or a contiguous run of Morton-sorted
-// queries), each with its own bounding box. For a reference tile and a box, the
-// largest value any pair can reach is, for the Gaussians, 2^e with
+// References are sorted along a Hilbert curve (host code) and packed exactly as
+// for k_pair_sum_f32x2; every run of consecutive sorted references (kCullUnit of
+// them here, kRefTile in the factored grid kernels) is a "reference tile" with a
+// bounding box, its widest kernel scale and its mass. The queries of a block
+// (kCullQpb neighbours: consecutive queries in curve order, or an 8 x 8 piece of a
+// grid tile) have a bounding box too. For a reference tile and a box, the largest
+// value any pair can reach is, for the Gaussians, 2^e with
 // e = log2(mass) + s_max * d_min^2 (d_min the distance between the boxes); for
 // the Epanechnikov kernels the question is whether any pair lies inside the
 // support.
@@ -21,11 +21,11 @@
 // Gaussian blocks run three scans over the tiles:
 //   1. M = the largest e over the block's box;
 //   2. sum every tile with e >= M - cut (the near field);
-//   3. with S_k = the smallest near-field sum in slot k, the allowance
-//      A_k = max(rel * S_k, abs) and T_k = log2(A_k / n_tiles) - 1, also sum
-//      every remaining tile that reaches e_k >= T_k for some slot k.
-// A tile left out has 2^e_k < A_k / (2 n_tiles) for every slot, so the skipped
-// part of every query q of slot k is below A_k / 2 <= max(rel * S_q, abs) / 2:
+//   3. with S = the smallest near-field sum of the block's queries, the allowance
+//      A = max(rel * S, abs) and T = log2(A / n_tiles) - 1, also sum every
+//      remaining tile that reaches e >= T.
+// A tile left out has 2^e < A / (2 n_tiles), so the skipped part of every query q
+// of the block is below A / 2 <= max(rel * S_q, abs) / 2:
 // every culled sum is within rel of the full sum, or within abs of it, whichever
 // is larger (plus the FP32 arithmetic error of the full sum). abs = 0 gives the
 // purely relative bound. This is the reference's combined criterion: its tree
@@ -33,13 +33,14 @@
 // abs_err absolute (KernelDensityImpl.h:1071-1095). Tiles whose largest pair exponent s_max d_min^2 is below -128
 // are skipped without a bound: ex2.approx.ftz flushes every such kernel value
 // to zero, so they add exactly nothing to the FP32 sum either. The per-block
-// worst ratio (skipped bound / S_k) is written for the host to verify.
-// Epanechnikov blocks sum every tile that intersects the support of some slot;
+// worst ratio (skipped bound / A) is written for the host to verify.
+// Epanechnikov blocks sum every tile that intersects the support of the box;
 // the skipped part is exactly zero.
 //
-// Summation is the direct kernel's: FP32 partial sums of kChunk pairs folded
-// into per-query Kahan accumulators, tiles in ascending sorted order, near field
-// before far field, so results are deterministic.
+// Summation: the warps of a block share its queries and take the listed tiles in
+// turn (warp w the entries w, w + warps, ...); FP32 partial sums of kChunk pairs
+// are folded into per-query Kahan accumulators of the warp, and the warps' sums
+// are added in FP64 in warp order, so results are deterministic.
 #pragma once
 
 #include <cstdint>
@@ -49,9 +50,24 @@
 
 namespace bbkde {
 
-constexpr int kRefTile = 256;      // references per culling tile
+constexpr int kRefTile = 256;      // references per culling tile of the factored grid kernels
 constexpr int kCullChunk = 1024;   // capacity of the per-batch list of needed tiles
 constexpr int kGroupTiles = 16;    // tiles per tile group (two-level scan)
+
+// Shape of the pair-form kernel: queries and warps per block, references per tile.
+// The bound is MUFU (16 ex2 per clock per SM) on the listed pairs; what a shape
+// decides is how many pairs are listed beyond the needed ones and whether a call of
+// 10^4 queries fills the chip. Measured, 60,001 queries x 100,003 adaptive
+// references at rel 1e-6, device ms (pairs listed): 64 queries x 64 references, 8
+// warps 0.19 (3.3e8); 32 references 0.23 (2.7e8: staging per pair); 128
+// references 0.22 (4.1e8); 128 queries 0.29 (3.7e8); 4 warps 0.23. The former
+// shape, 1,024 queries in eight strips x 256 references, 128 threads: 2.86
+// (1.35e9), on 59 blocks. 300,000 x 300,000 (h = 0.2): 4.3 ms, 3.6e12 pairs/s (77%
+// of the bound); 17.7 ms before.
+constexpr int kCullQpb = 64;
+constexpr int kCullWarps = 8;
+constexpr int kCullUnit = 64;
+constexpr int kCullPiece = 8;      // a block's piece of a grid tile: 8 x 8 points
 
 struct RefTile {
   float x0, x1, y0, y1;   // bounding box (y unused in 1-D)
@@ -61,14 +77,19 @@ struct RefTile {
 };
 
 // Where the queries of a block come from and where its results go.
-//   mode 0: explicit FP32 coordinates qx/qy[0, count), block b owns queries
-//           [b * QPB, (b + 1) * QPB); result i -> out[i].
-//   mode 1: tiles of a regular grid: block b owns grid tile tile_list[b] of
-//           tile x tile points (tiles numbered ty * ntx + tx); point (i, j) is at
-//           (gx0 + i gdx, gy0 + j gdy) and its result goes to out[j * gnx + i].
+//   mode 0: explicit FP32 coordinates: block b owns the queries perm[i], i in
+//           [b * kCullQpb, (b + 1) * kCullQpb), of the count at qx/qy[p * stride];
+//           the result of query p -> out[p].
+//   mode 1: tiles of a regular grid: tile_list holds tiles of tile x tile points
+//           (tiles numbered ty * ntx + tx); point (i, j) is at (gx0 + i gdx,
+//           gy0 + j gdy) and its result goes to out[j * gnx + i]. A pair-form
+//           block owns an 8 x 8 piece of a tile (block b: piece b % (tile / 8)^2 of
+//           tile tile_list[b / (tile / 8)^2]), a factored block a whole tile.
 struct CullQueries {
   int mode;
   const float *qx, *qy;
+  int stride;
+  const int *perm;
   int64_t count;
   const int *tile_list;
   int tile, ntx;
@@ -79,7 +100,7 @@ struct CullQueries {
 };
 
 struct CullArgs {
-  const float4 *refs;     // Morton-sorted packed records
+  const float4 *refs;     // curve-sorted packed records
   const float *extra;     // second scale column of the product kernels (or null)
   const RefTile *tiles;
   const RefTile *groups;  // one per kGroupTiles consecutive tiles (bounds of the union)
@@ -90,7 +111,7 @@ struct CullArgs {
   double rel;             // bound of the skipped part relative to the block minimum
   double abs_n;           // absolute allowance of the skipped part (unnormalised units)
   CullQueries q;
-  double *blk_bound;      // per block: worst (skipped bound / slot allowance A_k)
+  double *blk_bound;      // per block: worst (skipped bound / allowance)
   double *blk_smin;       // per block: smallest unnormalised sum of its queries
   int *blk_tiles;         // per block: reference tiles summed
   int *status;            // tensor-core form: set to 1 if a wait expired (or null)
@@ -117,23 +138,23 @@ __host__ __device__ constexpr bool op_gauss(int op) {
   return op == OP_GAUSS_ISO || op == OP_GAUSS_PROD;
 }
 
-// Query (slot k of this thread) -> coordinates and output index; false if the
-// slot is empty.
-template <int D, int QPB>
-__device__ __forceinline__ bool cull_query(const CullQueries &q, int64_t lq, float &x, float &y,
+// Query lq of a pair-form block -> coordinates and output index; false if empty.
+template <int D>
+__device__ __forceinline__ bool cull_query(const CullQueries &q, int lq, float &x, float &y,
                                            int64_t &o) {
   if (q.mode == 0) {
-    const int64_t i = (int64_t)blockIdx.x * QPB + lq;
+    const int64_t i = (int64_t)blockIdx.x * kCullQpb + lq;
     if (i >= q.count) return false;
-    x = q.qx[i];
-    y = D == 2 ? q.qy[i] : 0.f;
-    o = i;
+    o = q.perm[i];
+    x = q.qx[o * q.stride];
+    y = D == 2 ? q.qy[o * q.stride] : 0.f;
     return true;
   }
-  const int t = q.tile_list[blockIdx.x];
-  const int64_t tx = t % q.ntx, ty = t / q.ntx;
-  const int64_t i = tx * q.tile + lq % q.tile, j = ty * q.tile + lq / q.tile;
-  if (lq >= (int64_t)q.tile * q.tile || i >= q.gnx || j >= q.gny) return false;
+  const int pe = q.tile / kCullPiece, pieces = pe * pe;   // pieces per tile edge, per tile
+  const int t = q.tile_list[blockIdx.x / pieces], p = blockIdx.x % pieces;
+  const int64_t i = (int64_t)(t % q.ntx) * q.tile + (p % pe) * kCullPiece + lq % kCullPiece;
+  const int64_t j = (int64_t)(t / q.ntx) * q.tile + (p / pe) * kCullPiece + lq / kCullPiece;
+  if (i >= q.gnx || j >= q.gny) return false;
   x = grid_coord(q.gx0, q.gdx, i);
   y = grid_coord(q.gy0, q.gdy, j);
   o = j * q.gnx + i;
@@ -238,171 +259,149 @@ __device__ __forceinline__ int cull_pass(const CullArgs &a, int *s_list, int *s_
   return summed;
 }
 
-template <int OP, int D, int QPT, int BLOCK, int MINB>
-__global__ void __launch_bounds__(BLOCK, MINB) k_pair_sum_culled(CullArgs a) {
-  static_assert(QPT % 2 == 0 && kRefTile % BLOCK == 0 && kCullChunk % BLOCK == 0, "shape");
-  constexpr int NP = QPT / 2;
-  constexpr int QPB = QPT * BLOCK;
-  constexpr int NW = BLOCK / 32;
+template <int OP, int D>
+__global__ void __launch_bounds__(32 * kCullWarps, 4) k_pair_sum_culled(CullArgs a) {
+  constexpr int BLOCK = 32 * kCullWarps;
+  constexpr int NW = kCullWarps;
+  constexpr int QPT = kCullQpb / 32;       // queries per thread: 32 k + lane
+  constexpr int U = kCullUnit;
+  constexpr int PER = U / 32;              // references a lane stages per tile
   constexpr bool kExt = op_has_extra(OP) && D == 2;
   constexpr bool kGauss = op_gauss(OP);
-  __shared__ float4 s_r0[kRefTile];
-  __shared__ float4 s_r1[kRefTile];
-  __shared__ float4 s_r2[kExt ? kRefTile : 1];
+  constexpr int COLS = (D == 2 ? 4 : 3) + (kExt ? 1 : 0);   // -x, m, s (, -y (, second s))
+  static_assert(U % kChunk == 0 && kCullQpb == kCullPiece * kCullPiece, "shape");
+  __shared__ __align__(16) float s_ref[NW][COLS][U];
   __shared__ int s_list[cull_list_len(BLOCK)];
   __shared__ int s_glist[cull_groups_per_batch(BLOCK)];
   __shared__ int s_wc[NW];
-  __shared__ float s_box[QPT][4];     // slot boxes
-  __shared__ float s_th[QPT];         // slot thresholds T_k
-  __shared__ float s_f[QPT][4][NW];
-  __shared__ double s_d[QPT][NW];
+  __shared__ float s_red[NW];
+  __shared__ double s_sum[NW][kCullQpb];
+  __shared__ double s_min[kCullQpb / 32];
+  __shared__ double s_skip[NW];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  float2 qx[NP], qy[NP];
+  float2 qx[QPT], qy[QPT];   // (x, x), (y, y): two references per packed operation
   float sum[QPT], comp[QPT];
-  bool valid[QPT];
+  float qx0 = 3e38f, qx1 = -3e38f, qy0 = 3e38f, qy1 = -3e38f;
 #pragma unroll
   for (int k = 0; k < QPT; ++k) {
     float x = 0.f, y = 0.f;
     int64_t o = 0;
-    valid[k] = cull_query<D, QPB>(a.q, (int64_t)k * BLOCK + tid, x, y, o);
-    if (!valid[k]) { x = 0.f; y = 0.f; }
-    float bx0 = valid[k] ? x : 3e38f, bx1 = valid[k] ? x : -3e38f;
-    float by0 = valid[k] ? y : 3e38f, by1 = valid[k] ? y : -3e38f;
-#pragma unroll
-    for (int o2 = 16; o2 > 0; o2 >>= 1) {
-      bx0 = fminf(bx0, __shfl_xor_sync(0xffffffffu, bx0, o2));
-      bx1 = fmaxf(bx1, __shfl_xor_sync(0xffffffffu, bx1, o2));
-      by0 = fminf(by0, __shfl_xor_sync(0xffffffffu, by0, o2));
-      by1 = fmaxf(by1, __shfl_xor_sync(0xffffffffu, by1, o2));
+    if (cull_query<D>(a.q, 32 * k + lane, x, y, o)) {
+      qx0 = fminf(qx0, x); qx1 = fmaxf(qx1, x);
+      qy0 = fminf(qy0, y); qy1 = fmaxf(qy1, y);
     }
-    if (lane == 0) {
-      s_f[k][0][warp] = bx0; s_f[k][1][warp] = bx1; s_f[k][2][warp] = by0; s_f[k][3][warp] = by1;
-    }
-    if (k & 1) { qx[k >> 1].y = x; qy[k >> 1].y = y; }
-    else { qx[k >> 1].x = x; qy[k >> 1].x = y; }
+    qx[k] = f2(x);
+    qy[k] = f2(y);
     sum[k] = 0.f;
     comp[k] = 0.f;
   }
-  __syncthreads();
-  if (tid < QPT) {
-    float v0 = 3e38f, v1 = -3e38f, v2 = 3e38f, v3 = -3e38f;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      v0 = fminf(v0, s_f[tid][0][w]); v1 = fmaxf(v1, s_f[tid][1][w]);
-      v2 = fminf(v2, s_f[tid][2][w]); v3 = fmaxf(v3, s_f[tid][3][w]);
-    }
-    s_box[tid][0] = v0; s_box[tid][1] = v1; s_box[tid][2] = v2; s_box[tid][3] = v3;
+  for (int o = 16; o > 0; o >>= 1) {
+    qx0 = fminf(qx0, __shfl_xor_sync(0xffffffffu, qx0, o));
+    qx1 = fmaxf(qx1, __shfl_xor_sync(0xffffffffu, qx1, o));
+    qy0 = fminf(qy0, __shfl_xor_sync(0xffffffffu, qy0, o));
+    qy1 = fmaxf(qy1, __shfl_xor_sync(0xffffffffu, qy1, o));
   }
-  __syncthreads();
-  // Block box = union of the slot boxes.
-  float qx0 = 3e38f, qx1 = -3e38f, qy0 = 3e38f, qy1 = -3e38f;
-#pragma unroll
-  for (int k = 0; k < QPT; ++k) {
-    qx0 = fminf(qx0, s_box[k][0]); qx1 = fmaxf(qx1, s_box[k][1]);
-    qy0 = fminf(qy0, s_box[k][2]); qy1 = fmaxf(qy1, s_box[k][3]);
-  }
+
+  // No box: a piece outside the grid, or no query is a number. Nothing is summed.
+  const bool boxed = qx0 <= qx1 && qy0 <= qy1;
 
   // Scan 1 (Gaussians): largest tile bound over the block's box.
   float e_max = -INFINITY;
-  if (kGauss)
-    e_max = cull_max<BLOCK>(a, &s_f[0][0][0], [&](const RefTile &t) {
+  if (kGauss && boxed)
+    e_max = cull_max<BLOCK>(a, s_red, [&](const RefTile &t) {
       return t.lm + tile_peak<OP, D>(t, qx0, qx1, qy0, qy1);
     });
   const float t_a = e_max - a.cut;
 
-  // Skipped bound of slot k relative to its threshold: sum of 2^(e_k - T_k) < 1
-  // per skipped unit (terms below 2^-126 of the threshold flush; they are
-  // negligible). ex2.approx errs by ~2^-22 relative, inside the 1% mass slack.
-  float skipped[QPT];
-#pragma unroll
-  for (int k = 0; k < QPT; ++k) skipped[k] = 0.f;
+  // Skipped bound relative to the threshold: sum of 2^(e - T) < 1 per skipped
+  // unit (terms below 2^-126 of the threshold flush; they are negligible).
+  // ex2.approx errs by ~2^-22 relative, inside the 1% mass slack.
+  float skipped = 0.f, th = 0.f;
   int summed = 0;
 
-  // Is tile (or group) t needed? phase 0: Epanechnikov (support of some slot);
-  // phase 1: Gaussian near field; phase 2: Gaussian far field (per-slot
-  // thresholds; a unit that is not needed books its per-slot bound). For a group
-  // the near-field test of phase 2 is left out: a skipped group may hold tiles
-  // summed in phase 1, whose bound is then booked as well (an over-estimate).
+  // Is tile (or group) t needed? phase 0: Epanechnikov (support of the box);
+  // phase 1: Gaussian near field; phase 2: Gaussian far field (a unit that is not
+  // needed books its bound). For a group the near-field test of phase 2 is left
+  // out: a skipped group may hold tiles summed in phase 1, whose bound is then
+  // booked as well (an over-estimate).
   auto needed = [&](const RefTile &t, int phase, bool group) -> bool {
-    if (!kGauss) {
-      bool need = false;
-#pragma unroll
-      for (int k = 0; k < QPT; ++k)
-        need |= tile_peak<OP, D>(t, s_box[k][0], s_box[k][1], s_box[k][2], s_box[k][3]) > 0.f;
-      return need;
-    }
     const float pb = tile_peak<OP, D>(t, qx0, qx1, qy0, qy1);
+    if (!kGauss) return pb > 0.f;
     if (pb < kFlushExp) return false;   // every pair flushes to zero
-    const bool near = t.lm + pb >= t_a;
+    const float e = t.lm + pb;
+    const bool near = e >= t_a;
     if (phase == 1) return near;
     if (near && !group) return false;   // already summed
-    bool need = false;
-#pragma unroll
-    for (int k = 0; k < QPT; ++k) {
-      const float pk = tile_peak<OP, D>(t, s_box[k][0], s_box[k][1], s_box[k][2], s_box[k][3]);
-      need |= pk >= kFlushExp && t.lm + pk >= s_th[k];
-    }
-    if (!need) {
-#pragma unroll
-      for (int k = 0; k < QPT; ++k) {
-        const float pk = tile_peak<OP, D>(t, s_box[k][0], s_box[k][1], s_box[k][2], s_box[k][3]);
-        if (pk >= kFlushExp) skipped[k] += ex2_approx(t.lm + pk - s_th[k]);
-      }
-    }
-    return need;
+    if (e >= th) return true;
+    skipped += ex2_approx(e - th);
+    return false;
   };
 
-  // Sum the listed tiles (ascending order).
-  auto sum_list = [&](int running) {
-    for (int li = 0; li < running; ++li) {
-      const int64_t t0 = (int64_t)s_list[li] * kRefTile;
-      const int64_t t1 = min(t0 + kRefTile, a.n_ref);
+  // Sum the listed tiles: each warp stages its next tile's records while it sums
+  // the current one.
+  float (&st)[COLS][U] = s_ref[warp];
+  float4 rec[PER];
+  float ext[PER];
+  auto fetch = [&](int unit) {
 #pragma unroll
-      for (int i = tid; i < kRefTile; i += BLOCK) {
-        const int64_t rr = t0 + i;
-        const float4 v = rr < t1 ? a.refs[rr] : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (D == 2) {
-          s_r0[i] = make_float4(-v.x, -v.x, -v.y, -v.y);
-          s_r1[i] = make_float4(v.z, v.z, v.w, v.w);
-          if (kExt) {
-            const float e = rr < t1 ? a.extra[rr] : 0.f;
-            s_r2[i] = make_float4(e, e, 0.f, 0.f);
-          }
-        } else {
-          s_r0[i] = make_float4(-v.x, -v.x, 0.f, 0.f);
-          s_r1[i] = make_float4(v.y, v.y, v.z, v.z);
-        }
+    for (int u = 0; u < PER; ++u) {
+      const int64_t rr = (int64_t)unit * U + 32 * u + lane;
+      const bool in = rr < a.n_ref;
+      rec[u] = in ? __ldg(a.refs + rr) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (kExt) ext[u] = in ? __ldg(a.extra + rr) : 0.f;
+    }
+  };
+  auto sum_list = [&](int total) {
+    if (warp < total) fetch(s_list[warp]);
+    for (int li = warp; li < total; li += NW) {
+#pragma unroll
+      for (int u = 0; u < PER; ++u) {
+        const int i = 32 * u + lane;
+        st[0][i] = -rec[u].x;
+        st[1][i] = D == 2 ? rec[u].z : rec[u].y;
+        st[2][i] = D == 2 ? rec[u].w : rec[u].z;
+        if (D == 2) st[3][i] = -rec[u].y;
+        if (kExt) st[COLS - 1][i] = ext[u];
       }
-      __syncthreads();
-      for (int j0 = 0; j0 < kRefTile; j0 += kChunk) {
-        float2 acc[NP];
+      __syncwarp();
+      if (li + NW < total) fetch(s_list[li + NW]);
+#pragma unroll 1
+      for (int j0 = 0; j0 < U; j0 += kChunk) {
+        float2 acc[QPT];
 #pragma unroll
-        for (int p = 0; p < NP; ++p) acc[p] = f2(0.0f);
+        for (int k = 0; k < QPT; ++k) acc[k] = f2(0.0f);
 #pragma unroll 4
-        for (int j = 0; j < kChunk; ++j) {
-          const float4 r0 = s_r0[j0 + j];
-          const float4 r1 = s_r1[j0 + j];
-          const float4 r2 = kExt ? s_r2[j0 + j] : r1;
-          const float2 m = make_float2(r1.x, r1.y);
-#pragma unroll
-          for (int p = 0; p < NP; ++p)
-            acc[p] = __ffma2_rn(m, pair_u2<OP, D>(qx[p], qy[p], r0, r1, r2), acc[p]);
-        }
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
+        for (int j = 0; j < kChunk; j += 4) {
+          auto col = [&](int cidx) {
+            return *reinterpret_cast<const float4 *>(&st[cidx][j0 + j]);
+          };
+          const float4 x4 = col(0), m4 = col(1), s4 = col(2);
+          const float4 y4 = D == 2 ? col(D == 2 ? 3 : 0) : x4, e4 = kExt ? col(COLS - 1) : s4;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const int k = 2 * p + h;
-            const float v = h ? acc[p].y : acc[p].x;
-            const float y = v - comp[k];
-            const float t = sum[k] + y;
-            comp[k] = (t - sum[k]) - y;
-            sum[k] = t;
+            auto half = [&](const float4 &v) {
+              return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
+            };
+            const float2 m = half(m4);
+#pragma unroll
+            for (int k = 0; k < QPT; ++k)
+              acc[k] = __ffma2_rn(
+                  m, pair_u2r<OP, D>(qx[k], qy[k], half(x4), half(y4), half(s4), half(e4)),
+                  acc[k]);
           }
         }
+        // Kahan fold of the chunk partial (even + odd references).
+#pragma unroll
+        for (int k = 0; k < QPT; ++k) {
+          const float y = (acc[k].x + acc[k].y) - comp[k];
+          const float t = sum[k] + y;
+          comp[k] = (t - sum[k]) - y;
+          sum[k] = t;
+        }
       }
-      __syncthreads();
+      __syncwarp();
     }
   };
 
@@ -411,74 +410,63 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pair_sum_culled(CullArgs a) {
         a, s_list, s_glist, s_wc, [&](const RefTile &g) { return needed(g, phase, true); },
         [&](const RefTile &t) { return needed(t, phase, false); }, sum_list);
   };
-
-  double smin_all = 0.0, ratio = 0.0;
-  if (kGauss) {
-    pass(1);   // scan 2: near field
-    // Smallest near-field sum of every slot -> slot thresholds.
+  // The warps' sums of query tid (tid < kCullQpb) added in warp order.
+  auto total_of = [&]() {
 #pragma unroll
-    for (int k = 0; k < QPT; ++k) {
-      double m = valid[k] ? (double)sum[k] - (double)comp[k] : INFINITY;
+    for (int k = 0; k < QPT; ++k)
+      s_sum[warp][32 * k + lane] = (double)sum[k] - (double)comp[k];
+    __syncthreads();
+    double v = 0.0;
+    if (tid < kCullQpb) {
+#pragma unroll
+      for (int w = 0; w < NW; ++w) v += s_sum[w][tid];
+    }
+    return v;
+  };
+
+  float fx = 0.f, fy = 0.f;   // query tid, its output
+  int64_t fo = 0;
+  const bool mine = tid < kCullQpb && cull_query<D>(a.q, tid, fx, fy, fo);
+  double smin = 0.0, ratio = 0.0;
+  if (kGauss && boxed) {
+    pass(1);   // scan 2: near field
+    double m = total_of();
+    if (tid < kCullQpb) {   // whole warps
+      if (!mine) m = INFINITY;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, o));
-      if (lane == 0) s_d[k][warp] = m;
+      if (lane == 0) s_min[warp] = m;
     }
     __syncthreads();
-    if (tid < QPT) {
-      double m = INFINITY;
+    smin = INFINITY;
 #pragma unroll
-      for (int w = 0; w < NW; ++w) m = fmin(m, s_d[tid][w]);
-      // m = +inf: an empty slot needs nothing; allowance 0 (m <= 0 and no abs):
-      // the slot needs every tile that does not flush to zero.
-      const double allow = fmax(a.rel * m, a.abs_n);
-      s_th[tid] = allow > 0.0 ? (float)(log2(allow) - log2((double)a.n_tiles)) - 1.0f
-                              : -INFINITY;
-      s_d[tid][0] = m;
-      s_d[tid][1] = allow;
-    }
-    __syncthreads();
-    double smk[QPT], alk[QPT];
-#pragma unroll
-    for (int k = 0; k < QPT; ++k) {
-      smk[k] = s_d[k][0];
-      alk[k] = s_d[k][1];
-    }
-    __syncthreads();
+    for (int w = 0; w < kCullQpb / 32; ++w) smin = fmin(smin, s_min[w]);
+    // allowance 0 (smin <= 0 and no abs): every tile that does not flush to zero
+    const double allow = fmax(a.rel * smin, a.abs_n);
+    th = allow > 0.0 ? (float)(log2(allow) - log2((double)a.n_tiles)) - 1.0f : -INFINITY;
     pass(2);   // scan 3: far field, bound of the rest
-    // Per-slot bound of the skipped part (fixed-order reduction), worst ratio to
-    // the allowance: bound_k = skipped_k 2^T_k and 2^T_k = A_k / (2 n_tiles).
+    // Bound of the skipped part (fixed-order reduction) over the allowance:
+    // skipped 2^T with 2^T = A / (2 n_tiles).
+    double sk = skipped;
 #pragma unroll
-    for (int k = 0; k < QPT; ++k) {
-      double sk = skipped[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sk += __shfl_xor_sync(0xffffffffu, sk, o);
-      if (lane == 0) s_d[k][warp] = sk;
-    }
+    for (int o = 16; o > 0; o >>= 1) sk += __shfl_xor_sync(0xffffffffu, sk, o);
+    if (lane == 0) s_skip[warp] = sk;
     __syncthreads();
-    smin_all = INFINITY;
+    double b = 0.0;
 #pragma unroll
-    for (int k = 0; k < QPT; ++k) {
-      double b = 0.0;
-#pragma unroll
-      for (int w = 0; w < NW; ++w) b += s_d[k][w];
-      smin_all = fmin(smin_all, smk[k]);
-      if (b > 0.0) ratio = fmax(ratio, b * exp2((double)s_th[k]) / alk[k]);
-    }
-  } else {
+    for (int w = 0; w < NW; ++w) b += s_skip[w];
+    if (b > 0.0) ratio = b * exp2((double)th) / allow;
+  } else if (boxed) {
     pass(0);
   }
+  const double v = total_of();
   if (tid == 0) {
     a.blk_bound[blockIdx.x] = ratio;
-    a.blk_smin[blockIdx.x] = smin_all;
+    a.blk_smin[blockIdx.x] = smin;
     a.blk_tiles[blockIdx.x] = summed;
   }
-#pragma unroll
-  for (int k = 0; k < QPT; ++k) {
-    float x, y;
-    int64_t o;
-    if (cull_query<D, QPB>(a.q, (int64_t)k * BLOCK + tid, x, y, o))
-      a.q.out[o] = a.q.scale * ((double)sum[k] - (double)comp[k]);
-  }
+  // A query that is not a number reaches no tile; its Gaussian sum is not a number.
+  if (mine) a.q.out[fo] = kGauss && (fx != fx || fy != fy) ? (double)NAN : a.q.scale * v;
 }
 
 // ---------------------------------------------------------------------------
@@ -519,14 +507,24 @@ __global__ void k_bbox(const float *x, const float *y, int stride, int64_t n, un
   }
 }
 
-// Spread the low 16 bits of v to the even bit positions.
-__device__ __forceinline__ unsigned spread16(unsigned v) {
-  v &= 0xffffu;
-  v = (v | (v << 8)) & 0x00ff00ffu;
-  v = (v | (v << 4)) & 0x0f0f0f0fu;
-  v = (v | (v << 2)) & 0x33333333u;
-  v = (v | (v << 1)) & 0x55555555u;
-  return v;
+// Position of (x, y), 16 bits each, along a Hilbert curve: per level the quadrant
+// (rx, ry) is digit (3 rx) ^ ry, and the lower levels are reflected / transposed
+// into the quadrant's own orientation. Unlike Morton order it has no jumps, so a
+// run of consecutive points never spans two distant quadrants.
+__device__ __forceinline__ unsigned hilbert16(unsigned x, unsigned y) {
+  unsigned key = 0;
+#pragma unroll
+  for (int b = 15; b >= 0; --b) {
+    const unsigned rx = (x >> b) & 1u, ry = (y >> b) & 1u;
+    key = (key << 2) | ((3u * rx) ^ ry);
+    if (ry == 0u) {
+      if (rx) { x = ~x; y = ~y; }   // only the bits below b are read from here on
+      const unsigned t = x;
+      x = y;
+      y = t;
+    }
+  }
+  return key;
 }
 
 __device__ __forceinline__ unsigned quantize(float v, float lo, float hi, float levels) {
@@ -535,9 +533,9 @@ __device__ __forceinline__ unsigned quantize(float v, float lo, float hi, float 
   return (unsigned)fminf(fmaxf(u * levels, 0.f), levels - 1.f);
 }
 
-// Morton key (2-D: 16 bits per axis interleaved; 1-D: 32-bit quantised x) and
+// Curve key (2-D: Hilbert order of 16 bits per axis; 1-D: 32-bit quantised x) and
 // the identity permutation.
-__global__ void k_morton(const float *x, const float *y, int stride, int64_t n,
+__global__ void k_curve_keys(const float *x, const float *y, int stride, int64_t n,
                          const unsigned *box, unsigned *keys, int *idx) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -545,8 +543,8 @@ __global__ void k_morton(const float *x, const float *y, int stride, int64_t n,
   const float xhi = from_ordered(box[2]), yhi = from_ordered(box[3]);
   unsigned key;
   if (y) {
-    key = spread16(quantize(x[i * stride], xlo, xhi, 65536.f)) |
-          (spread16(quantize(y[i * stride], ylo, yhi, 65536.f)) << 1);
+    key = hilbert16(quantize(x[i * stride], xlo, xhi, 65536.f),
+                    quantize(y[i * stride], ylo, yhi, 65536.f));
   } else {
     const float span = xhi - xlo;
     const double u = span > 0.f ? ((double)x[i * stride] - xlo) / span : 0.0;
@@ -565,31 +563,17 @@ __global__ void k_gather_rec(const float4 *rec, const float *ext, const int *per
   if (ext) ext_out[i] = ext[p];
 }
 
-__global__ void k_gather_xy(const float *x, const float *y, const int *perm, int64_t n,
-                            float *x_out, float *y_out) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int p = perm[i];
-  x_out[i] = x[p];
-  if (y) y_out[i] = y[p];
-}
-
-__global__ void k_scatter(const double *src, const int *perm, int64_t n, double *dst) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[perm[i]] = src[i];
-}
-
-// One warp per tile of kRefTile sorted records.
+// One warp per tile of `size` sorted records.
 template <int D>
-__global__ void k_ref_tiles(const float4 *rec, const float *ext, int64_t n, int n_tiles,
-                            RefTile *tiles) {
+__global__ void k_ref_tiles(const float4 *rec, const float *ext, int64_t n, int size,
+                            int n_tiles, RefTile *tiles) {
   const int t = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= n_tiles) return;
   float x0 = 3e38f, x1 = -3e38f, y0 = 3e38f, y1 = -3e38f, sx = -3e38f, sy = -3e38f;
   double m = 0.0;
-  for (int i = lane; i < kRefTile; i += 32) {
-    const int64_t r = (int64_t)t * kRefTile + i;
+  for (int i = lane; i < size; i += 32) {
+    const int64_t r = (int64_t)t * size + i;
     if (r >= n) break;
     const float4 v = rec[r];
     const float px = v.x, py = D == 2 ? v.y : 0.f;
@@ -620,33 +604,41 @@ __global__ void k_ref_tiles(const float4 *rec, const float *ext, int64_t n, int 
   }
 }
 
-// One thread per group of kGroupTiles consecutive tiles: union of the boxes,
+// kGroupTiles lanes per group of as many consecutive tiles: union of the boxes,
 // widest scales, log2 of the summed (already 1%-padded) masses, rounded up.
 __global__ void k_ref_groups(const RefTile *tiles, int n_tiles, int n_groups,
                              RefTile *groups) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= n_groups) return;
+  static_assert(kGroupTiles == 16, "half a warp per group");
+  const int ti = blockIdx.x * blockDim.x + threadIdx.x;   // group ti / 16
   RefTile u;
   u.x0 = 3e38f; u.x1 = -3e38f; u.y0 = 3e38f; u.y1 = -3e38f;
   u.sx = -3e38f; u.sy = -3e38f;
   double m = 0.0;
-  const int t1 = min((g + 1) * kGroupTiles, n_tiles);
-  for (int ti = g * kGroupTiles; ti < t1; ++ti) {
-    const RefTile t = tiles[ti];
-    u.x0 = fminf(u.x0, t.x0); u.x1 = fmaxf(u.x1, t.x1);
-    u.y0 = fminf(u.y0, t.y0); u.y1 = fmaxf(u.y1, t.y1);
-    u.sx = fmaxf(u.sx, t.sx); u.sy = fmaxf(u.sy, t.sy);
-    if (t.lm > -INFINITY) m += exp2((double)t.lm);
+  if (ti < n_tiles) {
+    u = tiles[ti];
+    if (u.lm > -INFINITY) m = exp2((double)u.lm);
   }
-  u.lm = m > 0.0 ? nextafterf((float)log2(m), INFINITY) : -INFINITY;
-  u.pad = 0.f;
-  groups[g] = u;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
+    u.x0 = fminf(u.x0, __shfl_xor_sync(0xffffffffu, u.x0, o));
+    u.x1 = fmaxf(u.x1, __shfl_xor_sync(0xffffffffu, u.x1, o));
+    u.y0 = fminf(u.y0, __shfl_xor_sync(0xffffffffu, u.y0, o));
+    u.y1 = fmaxf(u.y1, __shfl_xor_sync(0xffffffffu, u.y1, o));
+    u.sx = fmaxf(u.sx, __shfl_xor_sync(0xffffffffu, u.sx, o));
+    u.sy = fmaxf(u.sy, __shfl_xor_sync(0xffffffffu, u.sy, o));
+    m += __shfl_xor_sync(0xffffffffu, m, o);
+  }
+  if (ti % kGroupTiles == 0 && ti / kGroupTiles < n_groups) {
+    u.lm = m > 0.0 ? nextafterf((float)log2(m), INFINITY) : -INFINITY;
+    u.pad = 0.f;
+    groups[ti / kGroupTiles] = u;
+  }
 }
 
 // Largest skipped-bound ratio over the blocks, summed tiles.
 __global__ void k_cull_stats(const double *bound, const double *smin, const int *tiles,
                              int nblk, double *out2) {
-  __shared__ double s_r[256], s_t[256];
+  __shared__ double s_r[1024], s_t[1024];   // blockDim.x <= 1024, a power of two
   double r = 0.0, tsum = 0.0;
   for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
     r = fmax(r, bound[b]);

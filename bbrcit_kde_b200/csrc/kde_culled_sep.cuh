@@ -9,7 +9,7 @@
 // bound (16 pairs per clock per SM): 2T exponentials and T^2 multiply-adds per
 // reference, ~T^2/2T = T/2 times fewer exponentials than pairs.
 //
-// Culling is k_pair_sum_culled's (kde_culled.cuh): Morton-sorted 256-reference
+// Culling is k_pair_sum_culled's (kde_culled.cuh): curve-sorted 256-reference
 // tiles scanned two levels deep (tile groups first), near field within 2^-cut of
 // the largest tile bound, far field against per-slot thresholds (slot k = the
 // k-th strip of T/8 rows), every skipped unit booked in the per-slot bound

@@ -293,21 +293,19 @@ __device__ __forceinline__ float2 exp2_poly2(float2 x) {
                      __uint_as_float(__float_as_uint(p.y) + (__float_as_uint(t.y) << 23)));
 }
 
+// U of two pairs, one per packed lane: coordinate differences from q + (-r), the
+// reference's scales s (and sy for the product kernels).
 template <int OP, int D, bool POLY = false>
-__device__ __forceinline__ float2 pair_u2(const float2 qx, const float2 qy, const float4 &r0,
-                                          const float4 &r1, const float4 &r2) {
-  const float2 nrx = make_float2(r0.x, r0.y);
-  const float2 s = make_float2(r1.z, r1.w);
+__device__ __forceinline__ float2 pair_u2r(const float2 qx, const float2 qy, const float2 nrx,
+                                           const float2 nry, const float2 s, const float2 sy) {
   float2 dx = __fadd2_rn(qx, nrx);
   if (D == 2) {
-    const float2 nry = make_float2(r0.z, r0.w);
     float2 dy = __fadd2_rn(qy, nry);
     if (OP == OP_GAUSS_ISO) {
       float2 d2 = __ffma2_rn(dy, dy, __fmul2_rn(dx, dx));
       float2 e = __fmul2_rn(d2, s);
       return POLY ? exp2_poly2(e) : make_float2(ex2_approx(e.x), ex2_approx(e.y));
     } else if (OP == OP_GAUSS_PROD) {
-      const float2 sy = make_float2(r2.x, r2.y);
       float2 e = __ffma2_rn(__fmul2_rn(dy, dy), sy, __fmul2_rn(__fmul2_rn(dx, dx), s));
       return POLY ? exp2_poly2(e) : make_float2(ex2_approx(e.x), ex2_approx(e.y));
     } else if (OP == OP_EPAN_ISO) {
@@ -315,7 +313,6 @@ __device__ __forceinline__ float2 pair_u2(const float2 qx, const float2 qy, cons
       float2 u = __ffma2_rn(d2, s, f2(1.0f));
       return make_float2(fmaxf(u.x, 0.0f), fmaxf(u.y, 0.0f));
     } else {  // OP_EPAN_PROD
-      const float2 sy = make_float2(r2.x, r2.y);
       float2 ux = __ffma2_rn(__fmul2_rn(dx, dx), s, f2(1.0f));
       float2 uy = __ffma2_rn(__fmul2_rn(dy, dy), sy, f2(1.0f));
       return __fmul2_rn(make_float2(fmaxf(ux.x, 0.0f), fmaxf(ux.y, 0.0f)),
@@ -330,6 +327,14 @@ __device__ __forceinline__ float2 pair_u2(const float2 qx, const float2 qy, cons
       return make_float2(fmaxf(u.x, 0.0f), fmaxf(u.y, 0.0f));
     }
   }
+}
+
+// The same from a pre-duplicated shared-memory record (two queries, one reference).
+template <int OP, int D, bool POLY = false>
+__device__ __forceinline__ float2 pair_u2(const float2 qx, const float2 qy, const float4 &r0,
+                                          const float4 &r1, const float4 &r2) {
+  return pair_u2r<OP, D, POLY>(qx, qy, make_float2(r0.x, r0.y), make_float2(r0.z, r0.w),
+                               make_float2(r1.z, r1.w), make_float2(r2.x, r2.y));
 }
 
 __host__ __device__ constexpr bool op_packed(int op) {
