@@ -999,22 +999,23 @@ int bbkde_device_info(const bbkde_ctx *c, int *sm_count, int *device) {
 // ===========================================================================
 namespace {
 
-constexpr int kCvBlock = 1024;
-
-// Work-item plans of the batched CV launch: likelihood items of `chunk` queries
-// of one set, convolution items of at most `qblock` (<= kCvQBlock) queries of one
-// grid cell. Smaller items balance the 148 persistent blocks better at the end of
-// the launch; larger ones pay the per-item histogram set-up and flush less often.
+// Work-item plans of the batched CV launch: likelihood items of at most `chunk`
+// queries of one set, convolution items of at most `qblock` (<= kCvQBlock) queries of
+// a run of grid cells. Smaller items balance the 148 persistent blocks better at the
+// end of the launch; larger ones pay the per-item histogram set-up and flush less
+// often. A call with few points takes smaller items whatever the plan: about
+// kCvItemsPerSm of each kind per SM (500 points at 64 x 48: 5.2 ms in
+// one item of 500 queries, 0.09 ms in items of two).
+constexpr int kCvItemsPerSm = 8;
+constexpr int kCvMinQueries = 16;   // least queries of a convolution item
+// A likelihood query's histogram and scores cost as much as this many candidates.
+constexpr double kCvQueryCost = 5000.0;
+constexpr int kCvSpan = 8;          // most cells of one: half its candidate width to a side
 struct CvPlan {
   int chunk, qblock;
 };
 constexpr CvPlan kCvPlans[] = {{4096, 256}, {1024, 256}, {2048, 128}};
 constexpr int kCvNumPlans = 3;
-
-size_t cv_smem_bytes() {
-  return sizeof(double) * (4 * kCvHist + 6 * kCvMaxH + 3 * kCvQBlock) +
-         sizeof(int64_t) * (2 * kCvMaxRanges + 1) + 4 * sizeof(int) + 2 * kCvLut;
-}
 
 // Lower-bound table for cv_cell: bin i holds #{h[a] <= the smallest double whose
 // key (bits >> shift) is base + i}. The shift keeps as many mantissa bits as fit
@@ -1100,6 +1101,8 @@ extern "C" int bbkde_cv_batch(bbkde_ctx *c, int kind, int n_sets, const bbkde_da
   for (int sidx = 0; sidx < n_sets; ++sidx) {
     if (sets[sidx].n < 2 || !sets[sidx].coords)
       return fail(c, BBKDE_INVALID_ARGUMENT, "cv_batch: every dataset needs at least 2 points");
+    if (sets[sidx].n > INT32_MAX)
+      return fail(c, BBKDE_OUT_OF_RANGE, "cv_batch: more than 2^31 - 1 points in a dataset");
   }
   if (kind == BBKDE_GAUSSIAN_PRODUCT_2D)
     return cv_batch_loop(c, kind, n_sets, sets, n_hx, hx, n_hy, hy, precision, lik_out,
@@ -1178,15 +1181,18 @@ extern "C" int bbkde_cv_batch(bbkde_ctx *c, int kind, int n_sets, const bbkde_da
     });
     X.resize(s.begin + n); Y.resize(s.begin + n); Wt.resize(s.begin + n);
     double diag = 0;
+    bool uniform = hmax < 1e60 && std::min(hx[0], hy[0]) > 1e-60;
     for (int64_t r = 0; r < n; ++r) {
       const int64_t i = order[r], at = s.begin + r;
       const double w = (d.weights ? d.weights[i] : 1.0) / wt;
       X[at] = d.coords[2 * i];
       Y[at] = d.coords[2 * i + 1];
       Wt[at] = w;
+      uniform = uniform && w == Wt[s.begin];
       diag += w * w;
     }
     s.diag_wm = diag;
+    s.uniform = uniform ? 1 : 0;
     sum_pairs += (double)n * (double)n;
   }
   // Work-item plan: forced, or tuned per problem class on the real calls -- the
@@ -1214,7 +1220,13 @@ extern "C" int bbkde_cv_batch(bbkde_ctx *c, int kind, int n_sets, const bbkde_da
       trials = nullptr;   // tuned: nothing more to record
     }
   }
-  const CvPlan plan = kCvPlans[plan_id];
+  CvPlan plan = kCvPlans[plan_id];
+  {
+    const int64_t items = (int64_t)c->sm_count * kCvItemsPerSm;
+    plan.chunk = (int)std::min<int64_t>(plan.chunk, std::max<int64_t>(2, (total + items - 1) / items));
+    plan.qblock = (int)std::min<int64_t>(
+        plan.qblock, std::max<int64_t>(kCvMinQueries, (4 * total + items - 1) / items));
+  }
   // Work items: likelihood items (set, chunk of queries) and convolution items
   // (set, grid cell, block of <= plan.qblock queries, x-power group), ordered by
   // estimated cost so the largest start first.
@@ -1230,21 +1242,28 @@ extern "C" int bbkde_cv_batch(bbkde_ctx *c, int kind, int n_sets, const bbkde_da
       const int64_t q0 = (int64_t)ch * plan.chunk;
       const int64_t q1 = std::min<int64_t>(st.n, q0 + plan.chunk);
       items.push_back({sidx, 0, parts + ch, 0, 0, 0, q0, q1});
-      cost.push_back((double)(q1 - q0) * st.n);
+      cost.push_back((double)(q1 - q0) * (st.n + kCvQueryCost));
     }
     parts += part_count[sidx];
     const int64_t *cst = cells.data() + st.cell_begin;
-    for (int cy = 0; cy < st.gy; ++cy)
-      for (int cx = 0; cx < st.gx; ++cx) {
-        const int64_t cb = cst[(int64_t)cy * st.gx + cx], ce = cst[(int64_t)cy * st.gx + cx + 1];
-        for (int64_t q0 = cb; q0 < ce; q0 += plan.qblock) {
-          const int64_t q1 = std::min<int64_t>(ce, q0 + plan.qblock);
+    for (int cy = 0; cy < st.gy; ++cy) {
+      const int64_t *row = cst + (int64_t)cy * st.gx;
+      for (int cx = 0; cx < st.gx;) {
+        // cells cx .. cx1 of this row: at most plan.qblock queries and kCvSpan cells
+        // (one cell of more queries is cut into blocks)
+        int cx1 = cx;
+        while (cx1 + 1 < st.gx && cx1 + 1 - cx < kCvSpan && row[cx1 + 2] - row[cx] <= plan.qblock)
+          ++cx1;
+        for (int64_t q0 = row[cx]; q0 < row[cx1 + 1]; q0 += plan.qblock) {
+          const int64_t q1 = std::min<int64_t>(row[cx1 + 1], q0 + plan.qblock);
           for (int g = 0; g < 4; ++g) {
-            items.push_back({sidx, 1 + g, 0, cx, cy, 0, q0, q1});
+            items.push_back({sidx, 1 + g, 0, cx, cy, cx1, q0, q1});
             cost.push_back(0.5 * (double)(q1 - q0) * st.n);
           }
         }
+        cx = cx1 + 1;
       }
+    }
   }
   {
     std::vector<size_t> idx(items.size());
@@ -1339,8 +1358,9 @@ extern "C" int bbkde_cv_batch(bbkde_ctx *c, int kind, int n_sets, const bbkde_da
     e = cudaMemsetAsync(a.conv_hist, 0, (size_t)n_sets * 16 * kCvCells * sizeof(double),
                         c->stream);
     if (e != cudaSuccess) return e;
-    k_cv_batch<<<c->sm_count, kCvBlock, smem, c->stream>>>(a);
-    k_cv_finalize<<<n_sets, kCvBlock, 0, c->stream>>>(a, pbeg, pcnt, lik_dev, lsq_dev);
+    k_cv_batch<<<c->sm_count, kCvThreads, smem, c->stream>>>(a);
+    k_cv_prefix<<<dim3(n_sets, 16), kCvThreads, 0, c->stream>>>(a);
+    k_cv_scores<<<dim3(n_sets, n_hx), kCvThreads, 0, c->stream>>>(a, pbeg, pcnt, lik_dev, lsq_dev);
     return cudaGetLastError();
   };
   const bool capturable = c->stream != nullptr && c->stream != cudaStreamLegacy;
@@ -1372,7 +1392,7 @@ extern "C" int bbkde_cv_batch(bbkde_ctx *c, int kind, int n_sets, const bbkde_da
     CUDA_TRY(c, enqueue());
   }
   CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
-  c->launch_total += 2;
+  c->launch_total += 3;
   CUDA_TRY(c, cudaMemcpyAsync(lik_out, lik_dev, nout * sizeof(double), cudaMemcpyDeviceToHost,
                               c->stream));
   CUDA_TRY(c, cudaMemcpyAsync(lsq_out, lsq_dev, nout * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1385,7 +1405,7 @@ extern "C" int bbkde_cv_batch(bbkde_ctx *c, int kind, int n_sets, const bbkde_da
   CUDA_TRY(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   c->last_ms = ms;
   c->last_pairs = sum_pairs;
-  c->last_launches = 2;
+  c->last_launches = 3;
   c->cv_counts[0] = (int64_t)counts[0];
   c->cv_counts[1] = (int64_t)(counts[1] / 4);   // each x-power group counts every pair
   c->cv_last_plan = plan_id;

@@ -47,14 +47,18 @@ struct CvSet {
   double x0, y0, inv_cell;   // grid origin and 1 / cell size
   int gx, gy;
   double diag_wm;            // sum_i w_i m_i (the i == j convolution terms)
+  int uniform;               // every point has the same weight, and the bandwidths are
+                             // within 1e-60 .. 1e60, so that a density is 0 or normal
+                             // (nonzero sums are above 2^-120)
+  int pad;
 };
 
 // Work item: queries [q0, q1) of one set; kind 0 = likelihood / leave-one-out
 // pass (part = its row in the partial buffer), kind 1..4 = convolution pass for
-// x-power group kind - 1 over the queries of one grid cell (cx, cy).
+// x-power group kind - 1 over queries of the grid cells (cx .. cx1, cy).
 struct CvItem {
   int set, kind, part, cx;
-  int cy, pad;
+  int cy, cx1;
   int64_t q0, q1;
 };
 
@@ -98,30 +102,30 @@ __device__ __forceinline__ void cv_cell_of(const CvSet &s, double x, double y, i
 }
 
 // Candidate ranges (set-relative point indices) of the grid rows within `r`
-// cells of cell (cx, cy), one row per lane of warp 0, keeping only indices
-// >= min_j. Empty rows stay as empty ranges. Returns through shared memory.
-__device__ __forceinline__ void cv_ranges(const CvSet &s, const int64_t *cs, int cx, int cy,
-                                          int r, int64_t min_j, int64_t *rb, int64_t *pre,
+// cells of the cells (cx .. cx1, cy), one row per lane of warp 0, keeping only
+// indices >= min_j. Empty rows stay as empty ranges. Returns through shared memory.
+__device__ __forceinline__ void cv_ranges(const CvSet &s, const int64_t *cs, int cx, int cx1,
+                                          int cy, int r, int64_t min_j, int *rb, int *pre,
                                           int *nr) {
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     const int clo = cx - r < 0 ? 0 : cx - r;
-    const int chi = cx + r >= s.gx ? s.gx - 1 : cx + r;
+    const int chi = cx1 + r >= s.gx ? s.gx - 1 : cx1 + r;
     const int rlo = cy - r < 0 ? 0 : cy - r;
     const int rhi = cy + r >= s.gy ? s.gy - 1 : cy + r;
     const int rows = rhi - rlo + 1;   // <= 2 r + 1 <= kCvMaxRanges <= 32
-    int64_t b = 0, len = 0;
+    int b = 0, len = 0;   // a set has fewer than 2^31 points
     if (lane < rows) {
       const int row = rlo + lane;
-      b = cs[(int64_t)row * s.gx + clo];
-      int64_t e = cs[(int64_t)row * s.gx + chi + 1];
-      if (b < min_j) b = min_j;
+      b = (int)cs[(int64_t)row * s.gx + clo];
+      const int e = (int)cs[(int64_t)row * s.gx + chi + 1];
+      if (b < min_j) b = (int)min_j;
       len = e > b ? e - b : 0;
     }
-    int64_t incl = len;   // inclusive warp scan of the lengths
+    int incl = len;   // inclusive warp scan of the lengths
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      int64_t v = __shfl_up_sync(0xffffffffu, incl, o);
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += v;
     }
     if (lane < rows) {
@@ -190,25 +194,50 @@ __device__ __forceinline__ void cv_run_add(unsigned long long *H, CvRun &r, int 
 
 constexpr int kCvQBlock = 256;   // queries of one convolution item (staged in smem)
 constexpr int kCvUnroll = 2;     // consecutive candidates per thread and step
+constexpr int kCvThreads = 1024;
+constexpr int kCvSegs1 = 8;      // segments of a row in the likelihood's first prefix ...
+constexpr int kCvSegs2 = 16;     // ... and of a column in its second
 
-// Shared memory: H[4][kCvHist] (fixed point, then FP64 in place) | hx | hy |
-// 1/hx | 1/hy | 1/hx^2 | 1/hy^2 | query block x, y, 2 w | ranges | misc | LUTs.
-__global__ void __launch_bounds__(1024, 1) k_cv_batch(CvArgs a) {
+// Shared memory: H[4][kCvHist] (fixed point) | likelihood prefix rows [2][kCvHist]
+// (the convolution's query block x, y, 2 w) | segment totals | hx | hy | 1/hx | 1/hy
+// | 1/hx^2 | 1/hy^2 | ranges | misc | LUTs.
+constexpr size_t kCvTotals = 4 * kCvSegs1 * kCvMaxH;
+static_assert(kCvTotals >= 2 * kCvSegs2 * kCvMaxH && 2 * kCvHist >= 3 * kCvQBlock, "shared areas");
+static_assert(kCvMaxH * kCvSegs1 * 2 == kCvThreads && kCvMaxH * kCvSegs2 == kCvThreads,
+              "one thread per (row, segment, moment pair) and per (column, segment)");
+
+__host__ __device__ constexpr size_t cv_smem_bytes() {
+  return sizeof(double) * (6 * kCvHist + kCvTotals + 6 * kCvMaxH) +
+         sizeof(int) * (2 * kCvMaxRanges + 1 + 4) + 2 * kCvLut;
+}
+
+// What bounds the likelihood items: per query the 4 x 64 x 64 fixed-point moments
+// are read and cleared once (2 x 133 KB of shared memory, ~2,100 clocks) and one
+// logarithm per bandwidth pair runs on the FP64 pipe (~2,600 clocks at 64 x 64);
+// both prefix directions are therefore split over all 1,024 threads (8 or 4 cells
+// in registers, segment totals exchanged once), and the next query's pairs are
+// counted in the same interval as this query's logarithms. Measured,
+// four sets of 1,500-9,000 points at 64 x 48 bandwidths: 4.0 ms (17.2 ms with one
+// serial 64-step prefix per row and column and items of 1,024 queries); 16 sets of
+// 20,000 points at 64 x 64: 167 ms (176 ms), where the pairs are the bound.
+__global__ void __launch_bounds__(kCvThreads, 1) k_cv_batch(CvArgs a) {
   extern __shared__ __align__(16) double sh[];
   unsigned long long *H = reinterpret_cast<unsigned long long *>(sh);   // 4 * kCvHist
-  double *Hd = sh;
-  double *shx = sh + 4 * kCvHist;
+  double *PA = sh + 4 * kCvHist;       // row prefixes of {1, y^2} and ...
+  double *PB = PA + kCvHist;           // ... {x^2, x^2 y^2}, combined per bandwidth b
+  double *bqx = PA;                    // kCvQBlock each
+  double *bqy = bqx + kCvQBlock;
+  double *bqw = bqy + kCvQBlock;
+  double *tot = PA + 2 * kCvHist;      // kCvTotals
+  double *shx = tot + kCvTotals;
   double *shy = shx + kCvMaxH;
   double *ihx = shy + kCvMaxH;
   double *ihy = ihx + kCvMaxH;
   double *ihx2 = ihy + kCvMaxH;
   double *ihy2 = ihx2 + kCvMaxH;
-  double *bqx = ihy2 + kCvMaxH;        // kCvQBlock
-  double *bqy = bqx + kCvQBlock;
-  double *bqw = bqy + kCvQBlock;
-  int64_t *rb = reinterpret_cast<int64_t *>(bqw + kCvQBlock);   // kCvMaxRanges
-  int64_t *pre = rb + kCvMaxRanges;                            // kCvMaxRanges + 1
-  int *misc = reinterpret_cast<int *>(pre + kCvMaxRanges + 1); // [0] item, [1] nr
+  int *rb = reinterpret_cast<int *>(ihy2 + kCvMaxH);   // kCvMaxRanges
+  int *pre = rb + kCvMaxRanges;                        // kCvMaxRanges + 1
+  int *misc = pre + kCvMaxRanges + 1;                  // [0] item, [1] nr
   unsigned char *slutx = reinterpret_cast<unsigned char *>(misc + 4);
   unsigned char *sluty = slutx + kCvLut;
 
@@ -247,26 +276,42 @@ __global__ void __launch_bounds__(1024, 1) k_cv_batch(CvArgs a) {
 
     if (item.kind == 0) {
       // ---- likelihood / leave-one-out pass, one query at a time ----------
-      // Each thread owns the cells c = tid + k * nt (k < 4) of the accumulators.
-      double lik[4] = {0.0, 0.0, 0.0, 0.0}, llo[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int c = tid; c < 4 * kCvHist; c += nt) H[c] = 0ull;
+      // First prefix (along q): thread (row p1, segment s1 of 8 columns, moment pair
+      // mp). Second (along p) and scores: thread (column b2, segment s2 of 4 rows),
+      // whose four scores stay in registers for all queries of the item.
+      constexpr int C1 = kCvMaxH / kCvSegs1, C2 = kCvMaxH / kCvSegs2;
+      const int p1 = tid % kCvMaxH, s1 = (tid / kCvMaxH) % kCvSegs1, mp = tid / (kCvMaxH * kCvSegs1);
+      const int b2 = tid % kCvMaxH, s2 = tid / kCvMaxH;
+      // With equal weights sum w log f = w log prod f: lik holds the product's
+      // mantissa in [1, 2) (0 once a factor is 0), lexp its exponent.
+      double lik[C2], llo[C2];
+      int lexp[C2];
+      const bool uniform = s.uniform != 0;
+#pragma unroll
+      for (int k = 0; k < C2; ++k) { lik[k] = uniform ? 1.0 : 0.0; llo[k] = 0.0; lexp[k] = 0; }
+      int pcx = -1, pcy = -1;
       for (int64_t i = item.q0; i < item.q1; ++i) {
-        for (int c = tid; c < 4 * kCvHist; c += nt) H[c] = 0ull;
         const double qx = X[i], qy = Y[i];
         int cx, cy;
         cv_cell_of(s, qx, qy, cx, cy);
-        cv_ranges(s, cs, cx, cy, a.r_epan, 0, rb, pre, misc + 1);
-        __syncthreads();
+        if (cx != pcx || cy != pcy) {   // the same for every thread
+          __syncthreads();              // the former ranges are no longer read
+          cv_ranges(s, cs, cx, cx, cy, a.r_epan, 0, rb, pre, misc + 1);
+          __syncthreads();
+          pcx = cx;
+          pcy = cy;
+        }
         const int nr = misc[1];
-        const int64_t total = pre[nr];
+        const int total = pre[nr], self = (int)i;
         int r = 0;
         CvRun run;
-        for (int64_t base = (int64_t)tid * kCvUnroll; base < total;
-             base += (int64_t)nt * kCvUnroll) {
-          int64_t js[kCvUnroll];
+        for (int base = tid * kCvUnroll; base < total; base += nt * kCvUnroll) {
+          int js[kCvUnroll];
           double xs[kCvUnroll], ys[kCvUnroll], ws[kCvUnroll];
 #pragma unroll
           for (int u = 0; u < kCvUnroll; ++u) {
-            const int64_t k = base + u;
+            const int k = base + u;
             js[u] = -1;
             if (k < total) {
               while (k >= pre[r + 1]) ++r;
@@ -286,7 +331,7 @@ __global__ void __launch_bounds__(1024, 1) k_cv_batch(CvArgs a) {
             if (js[u] < 0) continue;
             const double dx = qx - xs[u], dy = qy - ys[u];
             const double ax = fabs(dx), ay = fabs(dy);
-            if (ax >= hxmax || ay >= hymax || js[u] == i) continue;
+            if (ax >= hxmax || ay >= hymax || js[u] == self) continue;
             ++n_lik;
             const int p = cv_cell(ax, shx, a.nhx, slutx, a.lut_basex, a.lut_shift);
             const int q = cv_cell(ay, shy, a.nhy, sluty, a.lut_basey, a.lut_shift);
@@ -299,64 +344,106 @@ __global__ void __launch_bounds__(1024, 1) k_cv_batch(CvArgs a) {
         }
         cv_run_flush(H, run);
         __syncthreads();
-        // Fixed point -> FP64 moments sum m dx^k dy^l (k, l in {0, 2}).
-        for (int c = tid; c < kCvCells; c += nt) {
-          const int p = c / kCvMaxH, q = c % kCvMaxH;
-          const int hcell = p * kCvRow + q;
-          const double hp2 = p < a.nhx ? shx[p] * shx[p] : 0.0;
-          const double hq2 = q < a.nhy ? shy[q] * shy[q] : 0.0;
-          const double u0 = (double)(long long)H[hcell] / kCvFixLik;
-          const double u1 = (double)(long long)H[kCvHist + hcell] / kCvFixLik;
-          const double u2 = (double)(long long)H[2 * kCvHist + hcell] / kCvFixLik;
-          const double u3 = (double)(long long)H[3 * kCvHist + hcell] / kCvFixLik;
-          Hd[hcell] = u0;
-          Hd[kCvHist + hcell] = u1 * hp2;
-          Hd[2 * kCvHist + hcell] = u2 * hq2;
-          Hd[3 * kCvHist + hcell] = u3 * hp2 * hq2;
-        }
-        __syncthreads();
-        // 2-D inclusive prefix: along q (rows), then along p (columns).
-        for (int row = tid; row < 4 * kCvMaxH; row += nt) {
-          double *hr = Hd + (row / kCvMaxH) * kCvHist + (row % kCvMaxH) * kCvRow;
-          double run = 0.0;
-          for (int q = 0; q < kCvMaxH; ++q) { run += hr[q]; hr[q] = run; }
-        }
-        __syncthreads();
-        for (int col = tid; col < 4 * kCvMaxH; col += nt) {
-          double *hc = Hd + (col / kCvMaxH) * kCvHist + (col % kCvMaxH);
-          double run = 0.0;
-          for (int p = 0; p < kCvMaxH; ++p) { run += hc[p * kCvRow]; hc[p * kCvRow] = run; }
-        }
-        __syncthreads();
-        const double wi = Wt[i];
+        // Fixed point -> FP64 moments sum m dx^k dy^l (k, l in {0, 2}); the histogram
+        // is left cleared for the next query. mp = 0: {1, y^2}, 1: {x^2, x^2 y^2}.
+        double u0[C1], u1[C1];
+        {
+          unsigned long long *h0 = H + mp * kCvHist + p1 * kCvRow + s1 * C1, *h1 = h0 + 2 * kCvHist;
+          const bool on = p1 < a.nhx && s1 * C1 < a.nhy;
+          const double hp2 = mp == 0 ? 1.0 : shx[p1] * shx[p1];
+          double r0 = 0.0, r1 = 0.0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int c = tid + k * nt;
-          if (c >= kCvCells) break;
-          const int ia = c / kCvMaxH, ib = c % kCvMaxH;
-          if (ia >= a.nhx || ib >= a.nhy) continue;
-          const int hc = ia * kCvRow + ib;
-          double S = Hd[hc] - Hd[kCvHist + hc] * ihx2[ia] - Hd[2 * kCvHist + hc] * ihy2[ib] +
-                     Hd[3 * kCvHist + hc] * ihx2[ia] * ihy2[ib];
-          S = S > 0.0 ? S : 0.0;
-          const double f = 0.5625 / (shx[ia] * shy[ib]) * S;   // KernelTraits.h:250-252
-          lik[k] += wi * log(f);
-          llo[k] += wi * f;
+          for (int k = 0; k < C1; ++k) {
+            if (on) {
+              const double hq = shy[s1 * C1 + k];
+              r0 += (double)(long long)h0[k] * (1.0 / kCvFixLik) * hp2;
+              r1 += s1 * C1 + k < a.nhy
+                        ? (double)(long long)h1[k] * (1.0 / kCvFixLik) * hp2 * (hq * hq)
+                        : 0.0;
+              h0[k] = 0ull;
+              h1[k] = 0ull;
+            }
+            u0[k] = r0;
+            u1[k] = r1;
+          }
+          double *t = tot + (2 * mp * kCvSegs1 + s1) * kCvMaxH + p1;
+          t[0] = r0;
+          t[kCvSegs1 * kCvMaxH] = r1;
         }
         __syncthreads();
+        {
+          const double *t = tot + 2 * mp * kCvSegs1 * kCvMaxH + p1;
+          double o0 = 0.0, o1 = 0.0;
+          for (int sg = 0; sg < s1; ++sg) {
+            o0 += t[sg * kCvMaxH];
+            o1 += t[(kCvSegs1 + sg) * kCvMaxH];
+          }
+          double *dst = (mp == 0 ? PA : PB) + p1 * kCvRow + s1 * C1;
+#pragma unroll
+          for (int k = 0; k < C1; ++k)
+            dst[k] = (o0 + u0[k]) - (o1 + u1[k]) * ihy2[s1 * C1 + k];
+        }
+        __syncthreads();
+        double va[C2], vb[C2];
+        {
+          const double *ra = PA + s2 * C2 * kCvRow + b2, *rb2 = PB + s2 * C2 * kCvRow + b2;
+          double r0 = 0.0, r1 = 0.0;
+#pragma unroll
+          for (int k = 0; k < C2; ++k) {
+            r0 += ra[k * kCvRow];
+            r1 += rb2[k * kCvRow];
+            va[k] = r0;
+            vb[k] = r1;
+          }
+          tot[s2 * kCvMaxH + b2] = r0;
+          tot[(kCvSegs2 + s2) * kCvMaxH + b2] = r1;
+        }
+        __syncthreads();
+        if (s2 * C2 < a.nhx && b2 < a.nhy) {
+          double o0 = 0.0, o1 = 0.0;
+          for (int sg = 0; sg < s2; ++sg) {
+            o0 += tot[sg * kCvMaxH + b2];
+            o1 += tot[(kCvSegs2 + sg) * kCvMaxH + b2];
+          }
+          const double wi = Wt[i];
+          const double cb = 0.5625 * ihy[b2];   // KernelTraits.h:250-252
+#pragma unroll
+          for (int k = 0; k < C2; ++k) {
+            const int ia = s2 * C2 + k;
+            if (ia >= a.nhx) break;
+            double S = (o0 + va[k]) - (o1 + vb[k]) * ihx2[ia];
+            S = S > 0.0 ? S : 0.0;
+            const double f = cb * ihx[ia] * S;
+            llo[k] += wi * f;
+            if (uniform) {
+              const double t = lik[k] * f;   // normal or 0: see CvSet::uniform
+              const int hi = __double2hiint(t);
+              lexp[k] += (hi >> 20) - 1023;
+              lik[k] = t > 0.0 ? __hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(t))
+                               : 0.0;
+            } else {
+              lik[k] += wi * log(f);
+            }
+          }
+        }
+      }
+      if (uniform) {
+        const double w = Wt[item.q0];
+#pragma unroll
+        for (int k = 0; k < C2; ++k)
+          lik[k] = w * (log(lik[k]) + (double)lexp[k] * 0.69314718055994530942);
       }
       double *dst = a.epan_part + (int64_t)item.part * 2 * kCvCells;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int c = tid + k * nt;
-        if (c < kCvCells) {
-          dst[c] = lik[k];
-          dst[kCvCells + c] = llo[k];
-        }
+      for (int k = 0; k < C2; ++k) {
+        const int c = (s2 * C2 + k) * kCvMaxH + b2;
+        dst[c] = lik[k];
+        dst[kCvCells + c] = llo[k];
       }
+      __syncthreads();
     } else {
-      // ---- convolution pass, x-power group g, one block of queries of one
-      // grid cell against every candidate j > i within 2 h_max (pairs are
+      // ---- convolution pass, x-power group g, one block of queries of a run of
+      // grid cells against every candidate j > i within 2 h_max (pairs are
       // symmetric, so each unordered pair is counted once and doubled) ------
       const int g = item.kind - 1;
       const int nq = (int)(item.q1 - item.q0);
@@ -366,19 +453,18 @@ __global__ void __launch_bounds__(1024, 1) k_cv_batch(CvArgs a) {
         bqy[t] = Y[item.q0 + t];
         bqw[t] = 2.0 * Wt[item.q0 + t] * kCvFixConv;
       }
-      cv_ranges(s, cs, item.cx, item.cy, a.r_conv, item.q0 + 1, rb, pre, misc + 1);
+      cv_ranges(s, cs, item.cx, item.cx1, item.cy, a.r_conv, item.q0 + 1, rb, pre, misc + 1);
       __syncthreads();
       const int nr = misc[1];
-      const int64_t total = pre[nr];
+      const int total = pre[nr], q0 = (int)item.q0;
       const double hx2 = 2.0 * hxmax, hy2 = 2.0 * hymax;
       int r = 0;
       CvRun run;
-      for (int64_t k = tid; k < total; k += nt) {
+      for (int k = tid; k < total; k += nt) {
         while (k >= pre[r + 1]) ++r;
-        const int64_t j = rb[r] + (k - pre[r]);
+        const int j = rb[r] + (k - pre[r]);
         const double xj = X[j], yj = Y[j], mj = M[j];
-        const int64_t below = j - item.q0;                      // queries i < j
-        const int lim = below < nq ? (int)below : nq;
+        const int lim = min(j - q0, nq);                        // queries i < j
         int t = lane % (lim > 0 ? lim : 1);                    // decorrelate lanes
         for (int s2 = 0; s2 < lim; ++s2) {
           const double ax = fabs(bqx[t] - xj), ay = fabs(bqy[t] - yj);
@@ -426,66 +512,87 @@ __global__ void __launch_bounds__(1024, 1) k_cv_batch(CvArgs a) {
   }
 }
 
-// Finalisation, one block per set: the 16 fixed-point convolution moments ->
-// FP64 sum 2 w_i m_j |dx|^e_k |dy|^e_l (times (2 h_p)^e_k (2 h_q)^e_l), 2-D prefix
-// in place, then per (a, b): sq = C'_ab (T_ab + sum w m), llo = sum over the
-// set's likelihood items (fixed order), lsq = sq - 2 llo, lik likewise.
-__global__ void __launch_bounds__(1024) k_cv_finalize(CvArgs a, const int *part_begin,
-                                                      const int *part_count, double *lik_out,
-                                                      double *lsq_out) {
-  const int set = blockIdx.x;
-  const int tid = threadIdx.x;
-  const int nt = blockDim.x;
-  const int ek[4] = {0, 2, 3, 5};
-  double *hist = a.conv_hist + (int64_t)set * 16 * kCvCells;
+// Finalisation, first step, one block per (moment, set): the fixed-point
+// convolution moment -> FP64 sum 2 w_i m_j |dx|^e_k |dy|^e_l (times (2 h_p)^e_k
+// (2 h_q)^e_l), 2-D inclusive prefix, in place.
+__device__ __forceinline__ double cv_power(double v, int group) {   // v^{0, 2, 3, 5}
+  const double v2 = v * v;
+  return group == 0 ? 1.0 : group == 1 ? v2 : group == 2 ? v2 * v : v2 * v2 * v;
+}
+
+__global__ void __launch_bounds__(kCvThreads) k_cv_prefix(CvArgs a) {
+  __shared__ double m[kCvHist];
+  const int kx = blockIdx.y / 4, ky = blockIdx.y % 4, tid = threadIdx.x;
+  double *hist = a.conv_hist + ((int64_t)blockIdx.x * 16 + blockIdx.y) * kCvCells;
   const unsigned long long *ihist = reinterpret_cast<const unsigned long long *>(hist);
-  for (int e = tid; e < 16 * kCvCells; e += nt) {
-    const int kx = e / (4 * kCvCells), ky = (e / kCvCells) % 4, c = e % kCvCells;
+  for (int c = tid; c < kCvCells; c += kCvThreads) {
     const int p = c / kCvMaxH, q = c % kCvMaxH;
-    const double sx = p < a.nhx ? pow(2.0 * a.hx[p], (double)ek[kx]) : 0.0;
-    const double sy = q < a.nhy ? pow(2.0 * a.hy[q], (double)ek[ky]) : 0.0;
-    hist[e] = (double)(long long)ihist[e] / kCvFixConv * sx * sy;
+    const double sx = p < a.nhx ? cv_power(2.0 * a.hx[p], kx) : 0.0;
+    const double sy = q < a.nhy ? cv_power(2.0 * a.hy[q], ky) : 0.0;
+    m[p * kCvRow + q] = (double)(long long)ihist[c] / kCvFixConv * sx * sy;
   }
   __syncthreads();
-  for (int row = tid; row < 16 * kCvMaxH; row += nt) {
-    double *hr = hist + (row / kCvMaxH) * kCvCells + (row % kCvMaxH) * kCvMaxH;
+  if (tid < kCvMaxH) {
     double run = 0.0;
-    for (int q = 0; q < kCvMaxH; ++q) { run += hr[q]; hr[q] = run; }
+#pragma unroll 8
+    for (int q = 0; q < kCvMaxH; ++q) { run += m[tid * kCvRow + q]; m[tid * kCvRow + q] = run; }
   }
   __syncthreads();
-  for (int col = tid; col < 16 * kCvMaxH; col += nt) {
-    double *hc = hist + (col / kCvMaxH) * kCvCells + (col % kCvMaxH);
+  if (tid < kCvMaxH) {
     double run = 0.0;
-    for (int p = 0; p < kCvMaxH; ++p) { run += hc[p * kCvMaxH]; hc[p * kCvMaxH] = run; }
+#pragma unroll 8
+    for (int p = 0; p < kCvMaxH; ++p) { run += m[p * kCvRow + tid]; m[p * kCvRow + tid] = run; }
   }
   __syncthreads();
+  for (int c = tid; c < kCvCells; c += kCvThreads)
+    hist[c] = m[(c / kCvMaxH) * kCvRow + c % kCvMaxH];
+}
+
+// Second step, one block per (row a of the grid, set): sq = C'_ab (T_ab + sum w m),
+// lik and llo = sums over the set's likelihood items in a fixed order (kCvPartSplit
+// runs of items per cell, then the runs), lsq = sq - 2 llo.
+constexpr int kCvPartSplit = 16;
+__global__ void __launch_bounds__(kCvThreads) k_cv_scores(CvArgs a, const int *part_begin,
+                                                          const int *part_count, double *lik_out,
+                                                          double *lsq_out) {
+  __shared__ double s_lik[kCvPartSplit][kCvMaxH], s_llo[kCvPartSplit][kCvMaxH];
+  static_assert(kCvPartSplit * kCvMaxH == kCvThreads, "one thread per (run, cell)");
+  const int set = blockIdx.x, ia = blockIdx.y;
+  const int ib = threadIdx.x % kCvMaxH, run = threadIdx.x / kCvMaxH;
+  const int pb = part_begin[set], pc = part_count[set];
+  const int per = (pc + kCvPartSplit - 1) / kCvPartSplit;
+  const int c = ia * kCvMaxH + ib;
+  double lik = 0.0, llo = 0.0;
+#pragma unroll 4
+  for (int k = run * per; k < min((run + 1) * per, pc); ++k) {
+    const double *pp = a.epan_part + (int64_t)(pb + k) * 2 * kCvCells;
+    lik += pp[c];
+    llo += pp[kCvCells + c];
+  }
+  s_lik[run][ib] = lik;
+  s_llo[run][ib] = llo;
+  __syncthreads();
+  if (run != 0 || ib >= a.nhy) return;
+  for (int k = 1; k < kCvPartSplit; ++k) {
+    lik += s_lik[k][ib];
+    llo += s_llo[k][ib];
+  }
   // P(u) = sum_k c_k u^{e_k}: (c, e) = (1, 0), (-5/4, 2), (5/8, 3), (-1/32, 5).
   const double ck[4] = {1.0, -1.25, 0.625, -0.03125};
-  const double diag = a.sets[set].diag_wm;
-  const int pb = part_begin[set], pc = part_count[set];
-  for (int c = tid; c < kCvCells; c += nt) {
-    const int ia = c / kCvMaxH, ib = c % kCvMaxH;
-    if (ia >= a.nhx || ib >= a.nhy) continue;
-    const double hxa = a.hx[ia], hyb = a.hy[ib];
-    double T = 0.0;
-    for (int kx = 0; kx < 4; ++kx) {
-      const double fx = ck[kx] / pow(hxa, (double)ek[kx]);
-      for (int ky = 0; ky < 4; ++ky) {
-        const double fy = ck[ky] / pow(hyb, (double)ek[ky]);
-        T += fx * fy * hist[(kx * 4 + ky) * kCvCells + c];
-      }
+  const double *hist = a.conv_hist + (int64_t)set * 16 * kCvCells;
+  const double hxa = a.hx[ia], hyb = a.hy[ib];
+  double T = 0.0;
+  for (int kx = 0; kx < 4; ++kx) {
+    const double fx = ck[kx] / cv_power(hxa, kx);
+    for (int ky = 0; ky < 4; ++ky) {
+      const double fy = ck[ky] / cv_power(hyb, ky);
+      T += fx * fy * hist[(kx * 4 + ky) * kCvCells + c];
     }
-    const double sq = 0.36 / (hxa * hyb) * (T + diag);   // KernelTraits.h:349-351
-    double lik = 0.0, llo = 0.0;
-    for (int k = 0; k < pc; ++k) {
-      const double *pp = a.epan_part + (int64_t)(pb + k) * 2 * kCvCells;
-      lik += pp[c];
-      llo += pp[kCvCells + c];
-    }
-    const int64_t o = ((int64_t)set * a.nhx + ia) * a.nhy + ib;
-    lik_out[o] = lik;
-    lsq_out[o] = sq - 2.0 * llo;
   }
+  const double sq = 0.36 / (hxa * hyb) * (T + a.sets[set].diag_wm);   // KernelTraits.h:349-351
+  const int64_t o = ((int64_t)set * a.nhx + ia) * a.nhy + ib;
+  lik_out[o] = lik;
+  lsq_out[o] = sq - 2.0 * llo;
 }
 
 }  // namespace bbkde

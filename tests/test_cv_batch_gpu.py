@@ -126,3 +126,22 @@ def test_cv_batch_plans_and_autotuner(ctx):
         used.append(ctx.cv_batch_info()[2])
     assert sorted(used[:3]) == [0, 1, 2]
     assert used[3] == used[4]
+
+
+@pytest.mark.parametrize("sizes,nx,ny,weighted", [
+    ([2], 1, 1, False), ([3, 17], 9, 1, True), ([130], 8, 17, False), ([700, 40], 64, 5, True),
+    ([1200], 63, 64, False)])
+def test_cv_batch_small_items(ctx, sizes, nx, ny, weighted):
+    """Few points (items of a few queries, runs of grid cells), ragged grids around the
+    8-column and 4-row segments of the prefix sums, equal and unequal weights: every
+    score against the per-bandwidth FP64 path on a sample of the grid."""
+    sets = W.config3_datasets(n_sets=len(sizes), sizes=sizes)
+    rng = W.SplitMix64(9)
+    datasets = [(s, rng.uniform(len(s), 0.5, 1.5) if weighted else None) for s in sets]
+    hx, hy = 0.05 * 1.06 ** np.arange(nx), 0.07 * 1.05 ** np.arange(ny)
+    lik, lsq = ctx.cv_batch(bk.EPANECHNIKOV_PRODUCT_2D, datasets, hx, hy)
+    pick = sorted({0, nx // 2, nx - 1}), sorted({0, ny // 2, ny - 1})
+    want_lik, want_lsq = _per_bandwidth(ctx, bk.EPANECHNIKOV_PRODUCT_2D, datasets, hx[pick[0]],
+                                        hy[pick[1]])
+    _close(lik[:, pick[0]][:, :, pick[1]], want_lik, 1e-9)
+    _close(lsq[:, pick[0]][:, :, pick[1]], want_lsq, 1e-9)
