@@ -56,17 +56,16 @@ struct Resolved {
   double h1 = 1, h2 = 1;
   double c1_f32 = 0, c2_f32 = 0;   // log2-based scale numerators (FP32 records)
   double c1_f64 = 0, c2_f64 = 0;   // natural-log scale numerators (FP64 records)
-  double mass_scale = 1.0;
   double norm = 1.0;               // C(h), reference formulas, FP64
 };
 
 struct PackKey {
   int op = -1, dim = 0;
-  double h1 = 0, h2 = 0, c1 = 0, c2 = 0, ms = 0;
+  double h1 = 0, h2 = 0, c1 = 0, c2 = 0;
   uint64_t coord_version = ~0ull, attr_version = ~0ull;
   bool operator==(const PackKey &o) const {
     return op == o.op && dim == o.dim && h1 == o.h1 && h2 == o.h2 && c1 == o.c1 &&
-           c2 == o.c2 && ms == o.ms && coord_version == o.coord_version &&
+           c2 == o.c2 && coord_version == o.coord_version &&
            attr_version == o.attr_version;
   }
 };
@@ -277,11 +276,9 @@ int resolve(bbkde_ctx *c, const bbkde_kernel_desc *k, Resolved &r) {
       break;
     case BBKDE_EPANECHNIKOV_PRODUCT_CONV_2D:
       r.op = OP_EPAN_CONV;
-      r.mass_scale = 1.0 / 1024.0;  // 0.03125 per dimension
       break;
     case BBKDE_EPANECHNIKOV_CONV_1D:
       r.op = OP_EPAN_CONV;
-      r.mass_scale = 1.0 / 32.0;
       break;
   }
   if (k->dim == 1 && r.op == OP_GAUSS_PROD) r.op = OP_GAUSS_ISO;
@@ -306,7 +303,6 @@ int ensure_pack(bbkde_ctx *c, const Resolved &r, bool f64) {
   key.h2 = r.h2;
   key.c1 = f64 ? r.c1_f64 : r.c1_f32;
   key.c2 = f64 ? r.c2_f64 : r.c2_f32;
-  key.ms = r.mass_scale;
   key.coord_version = s.coord_version;
   key.attr_version = s.attr_version;
   if (pc.key == key) return BBKDE_OK;
@@ -326,7 +322,6 @@ int ensure_pack(bbkde_ctx *c, const Resolved &r, bool f64) {
     p.c2 = key.c2;
     p.h1 = r.h1;
     p.h2 = r.h2;
-    p.mass_scale = r.mass_scale;
     if (f64)
       k_pack_f64<<<grid1d(s.n), 256, 0, c->stream>>>(p, pc.rec.as<double4>(), pc.ext.as<double>());
     else
@@ -383,15 +378,40 @@ constexpr Variant kVariants[] = {{8, 256, 2, 0},  {4, 256, 3, 0},  {8, 128, 4, 0
                                  {8, 128, 4, 4},  {4, 128, 6, 8},  {4, 128, 6, 16},
                                  {4, 128, 6, 32}, {8, 256, 2, 16}};
 constexpr int kNumVariants = 11;
-constexpr int kDefaultVariant = 0;
+// Beside them k_pair_sum_split (64 queries per block), the form of small problems.
+constexpr int kSplitVariant = kNumVariants;
 constexpr int kTile = 256;
 constexpr int kBlock64 = 128;
-// Problems below this many pairs skip autotuning (launch-latency bound anyway).
+// Problems below this many pairs skip autotuning: up to kSplitMaxPairs they run
+// k_pair_sum_split, above it a fixed shape (mid_variant). Kernel us, split / fixed:
+// 500 x 400 queries 8 / 13, 2,000 x 2,000 9 / 13, 10,000 x 10,000 36 / 36, 50,000 x
+// 50,000 630 / 595 (2-D Gaussian; 28, 30, 48, 633 in the 2,048-query blocks of shape 0).
 constexpr double kAutotuneMinPairs = 2.0e10;
+constexpr double kSplitMaxPairs = 3.0e8;
 
+// 1-D Gaussians have so few FP32 operations that every 8th reference's exponentials fit
+// there (50,000 x 50,000: 542 us, every 32nd 566, none 586); 2-D ones take every 32nd
+// (593, 638 with every 8th, 617 with none). The other kernels ignore the split.
+inline int mid_variant(const Resolved &r) { return r.dim == 1 ? 7 : 9; }
+
+// Queries per block. FP64: `variant` is the queries per thread (1 or 4, f64_qpt).
 inline int queries_per_block(int variant, bool f64) {
-  if (f64) return kBlock64;
+  if (f64) return variant * kBlock64;
+  if (variant == kSplitVariant) return kSplitQueries;
   return kVariants[variant].qpt * kVariants[variant].block;
+}
+
+// References that a segment is a multiple of.
+inline int segment_step(int variant, bool f64) {
+  return f64 ? kBlock64 : variant == kSplitVariant ? kSplitStep : kTile;
+}
+
+// Four queries per FP64 thread while that still makes two blocks per SM (segments of
+// one staging tile at the least), else one.
+inline int f64_qpt(const bbkde_ctx *c, int64_t n_ref, int64_t q_count) {
+  const int64_t blocks = ((q_count + 4 * kBlock64 - 1) / (4 * kBlock64)) *
+                         ((n_ref + kBlock64 - 1) / kBlock64);
+  return blocks >= 2 * c->sm_count ? 4 : 1;
 }
 
 struct Plan {
@@ -400,30 +420,30 @@ struct Plan {
 };
 
 // Split the reference range into segments so that the grid fills the device
-// with ~16 waves of blocks (load balance through the hardware block scheduler),
-// but never below one staging tile of references per segment (small problems:
-// 10,000 x 10,000 pairs would otherwise run on half the SMs).
-Plan plan_launch(const bbkde_ctx *c, int64_t n_ref, int64_t q_count, int q_per_block,
-                 int tile) {
+// with ~16 waves of blocks (load balance through the hardware block scheduler; the
+// split form, whose blocks are smaller, kSplitWaves), but never below one staging
+// step of references per segment.
+constexpr int kSplitWaves = 4;
+
+Plan plan_launch(int sm_count, int64_t n_ref, int64_t q_count, int variant, bool f64) {
   Plan p;
-  int64_t qtiles = (q_count + q_per_block - 1) / q_per_block;
-  p.gx = (unsigned)std::max<int64_t>(qtiles, 1);
-  int64_t target = (int64_t)c->sm_count * 4 * 16;
-  int64_t want = (target + qtiles - 1) / std::max<int64_t>(qtiles, 1);
-  int64_t max_seg = std::max<int64_t>(1, (n_ref + tile - 1) / tile);
-  p.nseg = std::min<int64_t>(std::max<int64_t>(want, 1), std::min<int64_t>(max_seg, 65535));
+  const int64_t q_per_block = queries_per_block(variant, f64), step = segment_step(variant, f64);
+  const int64_t qtiles = std::max<int64_t>(1, (q_count + q_per_block - 1) / q_per_block);
+  p.gx = (unsigned)qtiles;
+  const int64_t target =
+      (int64_t)sm_count * 4 * (!f64 && variant == kSplitVariant ? kSplitWaves : 16);
+  const int64_t want = (target + qtiles - 1) / qtiles;
+  const int64_t max_seg = std::max<int64_t>(1, (n_ref + step - 1) / step);
+  p.nseg = std::min<int64_t>(want, std::min<int64_t>(max_seg, 65535));
   p.seg_len = (n_ref + p.nseg - 1) / p.nseg;
-  p.seg_len = (p.seg_len + tile - 1) / tile * tile;
+  p.seg_len = (p.seg_len + step - 1) / step * step;
   p.nseg = std::max<int64_t>(1, (n_ref + p.seg_len - 1) / p.seg_len);
   return p;
 }
 
 template <int OP, int D, int QPT, int BLOCK, int MINB, int POLY = 0>
 void launch_shape(dim3 grid, cudaStream_t st, const SumArgs &a) {
-  if constexpr (op_packed(OP))
-    k_pair_sum_f32x2<OP, D, QPT, BLOCK, kTile, MINB, POLY><<<grid, BLOCK, 0, st>>>(a);
-  else
-    k_pair_sum_f32<OP, D, QPT, BLOCK, kTile, MINB><<<grid, BLOCK, 0, st>>>(a);
+  k_pair_sum_f32x2<OP, D, QPT, BLOCK, kTile, MINB, POLY><<<grid, BLOCK, 0, st>>>(a);
 }
 
 template <int OP, int D>
@@ -439,12 +459,16 @@ void launch_f32(int variant, dim3 grid, cudaStream_t st, const SumArgs &a) {
     case 7: launch_shape<OP, D, 4, 128, 6, 8>(grid, st, a); break;
     case 8: launch_shape<OP, D, 4, 128, 6, 16>(grid, st, a); break;
     case 9: launch_shape<OP, D, 4, 128, 6, 32>(grid, st, a); break;
-    default: launch_shape<OP, D, 8, 256, 2, 16>(grid, st, a); break;
+    case 10: launch_shape<OP, D, 8, 256, 2, 16>(grid, st, a); break;
+    default: k_pair_sum_split<OP, D><<<grid, 32 * kSplitWarps, 0, st>>>(a); break;
   }
 }
 template <int OP, int D>
-void launch_f64(dim3 grid, cudaStream_t st, const SumArgs &a) {
-  k_pair_sum_f64<OP, D, kBlock64><<<grid, kBlock64, 0, st>>>(a);
+void launch_f64(int qpt, dim3 grid, cudaStream_t st, const SumArgs &a) {
+  if (qpt == 4)
+    k_pair_sum_f64<OP, D, 4, kBlock64><<<grid, kBlock64, 0, st>>>(a);
+  else
+    k_pair_sum_f64<OP, D, 1, kBlock64><<<grid, kBlock64, 0, st>>>(a);
 }
 
 template <int D>
@@ -452,7 +476,7 @@ void dispatch_op(int op, bool f64, int variant, dim3 grid, cudaStream_t st, cons
   switch (op) {
 #define CASE_(OPV)                                         \
   case OPV:                                                \
-    if (f64) launch_f64<OPV, D>(grid, st, a);              \
+    if (f64) launch_f64<OPV, D>(variant, grid, st, a);     \
     else launch_f32<OPV, D>(variant, grid, st, a);         \
     break;
     CASE_(OP_GAUSS_ISO)
@@ -470,14 +494,30 @@ inline int ilog2(int64_t v) {
   return r;
 }
 
+// Segment combination: groups of threads share the segments once there are enough.
+constexpr int kCombineGroups = 8;
+inline bool combine_grouped(int64_t nseg) { return nseg >= kCombineGroups; }
+inline unsigned combine_blocks(int64_t nseg, int64_t q_count) {
+  return grid1d(q_count, combine_grouped(nseg) ? kRedBlock / kCombineGroups : kRedBlock);
+}
+void launch_combine(cudaStream_t st, const double *partial, int64_t nseg, int64_t q_count,
+                    double scale, double *out, int epi, const double *w, double *block_sums) {
+  const unsigned nb = combine_blocks(nseg, q_count);
+  if (combine_grouped(nseg))
+    k_combine<kCombineGroups><<<nb, kRedBlock, 0, st>>>(partial, (int)nseg, q_count, scale, out,
+                                                        epi, w, block_sums);
+  else
+    k_combine<1><<<nb, kRedBlock, 0, st>>>(partial, (int)nseg, q_count, scale, out, epi, w,
+                                           block_sums);
+}
+
 // Fill SumArgs and launch one pair-sum kernel over [r_i, r_j] x [q_i, q_j].
 int launch_pair_sum(bbkde_ctx *c, const Resolved &r, bool f64, int variant, const void *qx,
                     const void *qy, int64_t r_i, int64_t r_j, int64_t q_i, int64_t q_j,
                     bool exclude_self, double scale, double *out, int64_t *nseg_out) {
   const int64_t n_ref = r_j - r_i + 1;
   const int64_t q_count = q_j - q_i + 1;
-  Plan p = plan_launch(c, n_ref, q_count, queries_per_block(variant, f64),
-                       f64 ? kBlock64 : kTile);
+  Plan p = plan_launch(c->sm_count, n_ref, q_count, variant, f64);
   PackCache &pc = f64 ? c->pack64 : c->pack32;
   SumArgs a;
   a.refs = pc.rec.p;
@@ -510,7 +550,10 @@ int choose_variant(bbkde_ctx *c, const Resolved &r, const void *qx, const void *
                    int *variant) {
   if (c->forced_variant >= 0) { *variant = c->forced_variant; return BBKDE_OK; }
   const double pairs = (double)(r_j - r_i + 1) * (double)(q_j - q_i + 1);
-  if (pairs < kAutotuneMinPairs) { *variant = kDefaultVariant; return BBKDE_OK; }
+  if (pairs < kAutotuneMinPairs) {
+    *variant = pairs <= kSplitMaxPairs ? kSplitVariant : mid_variant(r);
+    return BBKDE_OK;
+  }
   auto key = std::make_tuple(r.op, r.dim, exclude_self ? 1 : 0, ilog2(r_j - r_i + 1),
                              ilog2(q_j - q_i + 1));
   auto it = c->tuned.find(key);
@@ -526,7 +569,7 @@ int choose_variant(bbkde_ctx *c, const Resolved &r, const void *qx, const void *
   }
   TRY(ensure(c, c->partial, (size_t)need * sizeof(double)));
   float best_ms = 0.f;
-  int best = kDefaultVariant;
+  int best = 0;
   for (int v = 0; v < kNumVariants; ++v) {
     float ms = 0.f;
     for (int rep = 0; rep < 2; ++rep) {
@@ -556,7 +599,7 @@ int pair_sum(bbkde_ctx *c, const Resolved &r, int precision, int qset, int64_t r
   TRY(ensure_queries(c, qset, f64, &qx, &qy));
   const int64_t n_ref = r_j - r_i + 1;
   const int64_t q_count = q_j - q_i + 1;
-  int variant = 0;
+  int variant = f64 ? f64_qpt(c, n_ref, q_count) : 0;
   if (!f64) TRY(choose_variant(c, r, qx, qy, r_i, r_j, q_i, q_j, exclude_self, &variant));
   int64_t nseg = 1;
   TRY(launch_pair_sum(c, r, f64, variant, qx, qy, r_i, r_j, q_i, q_j, exclude_self, 1.0,
@@ -573,10 +616,10 @@ int pair_sum(bbkde_ctx *c, const Resolved &r, int precision, int qset, int64_t r
   CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
   int64_t launches = 1;
   if (combine) {
-    const unsigned nb = grid1d(q_count, kRedBlock);
+    const unsigned nb = combine_blocks(nseg, q_count);
     if (epi != EPI_NONE) TRY(ensure(c, c->block_sums, (size_t)nb * sizeof(double)));
-    k_combine<<<nb, kRedBlock, 0, c->stream>>>(partial, (int)nseg, q_count, scale, out_dev,
-                                               epi, w_dev, c->block_sums.as<double>());
+    launch_combine(c->stream, partial, nseg, q_count, scale, out_dev, epi, w_dev,
+                   c->block_sums.as<double>());
     COUNT_LAUNCH(c);
     CUDA_TRY(c, cudaGetLastError());
     ++launches;
@@ -595,7 +638,7 @@ int pair_sum(bbkde_ctx *c, const Resolved &r, int precision, int qset, int64_t r
   c->last_ms = ms;
   c->last_pairs = (double)n_ref * (double)q_count;
   c->last_launches = launches;
-  c->last_variant = f64 ? -1 : variant;
+  c->last_variant = f64 || variant == kSplitVariant ? -1 : variant;
   return BBKDE_OK;
 }
 
@@ -2661,7 +2704,6 @@ extern "C" int bbkde_eval_noalloc(const bbkde_kernel_desc *kernel, int64_t n_ref
   p.c2 = r.c2_f32;
   p.h1 = r.h1;
   p.h2 = r.h2;
-  p.mass_scale = r.mass_scale;
   k_pack_f32<<<grid1d(n_ref), 256, 0, st>>>(p, rec, extc);
   k_to_f32<<<grid1d(n_query), 256, 0, st>>>(query_x, qx, n_query);
   if (dim == 2) k_to_f32<<<grid1d(n_query), 256, 0, st>>>(query_y, qy, n_query);
@@ -2675,17 +2717,13 @@ extern "C" int bbkde_eval_noalloc(const bbkde_kernel_desc *kernel, int64_t n_ref
     cudaGetLastError();
     return BBKDE_CUDA_ERROR;
   }
-  const int variant = kDefaultVariant;
-  const int qpb = queries_per_block(variant, false);
-  const int64_t qtiles = (n_query + qpb - 1) / qpb;
-  const int64_t target = (int64_t)sm_count * 4 * 16;
-  int64_t nseg = std::max<int64_t>(1, (target + qtiles - 1) / qtiles);
-  nseg = std::min<int64_t>(nseg, std::max<int64_t>(1, (n_ref + 511) / 512));
-  nseg = std::min<int64_t>(nseg, (int64_t)((kNoAllocScratchBytes - off_part) / per_seg));
-  nseg = std::min<int64_t>(nseg, 65535);
-  int64_t seg_len = (n_ref + nseg - 1) / nseg;
-  seg_len = (seg_len + kTile - 1) / kTile * kTile;
-  nseg = std::max<int64_t>(1, (n_ref + seg_len - 1) / seg_len);
+  Plan pl = plan_launch(sm_count, n_ref, n_query, kSplitVariant, false);
+  const int64_t fit = (int64_t)((kNoAllocScratchBytes - off_part) / per_seg);
+  if (pl.nseg > fit) {
+    pl.seg_len = (n_ref + fit - 1) / fit;
+    pl.seg_len = (pl.seg_len + kSplitStep - 1) / kSplitStep * kSplitStep;
+    pl.nseg = (n_ref + pl.seg_len - 1) / pl.seg_len;
+  }
 
   SumArgs a;
   a.refs = rec;
@@ -2694,18 +2732,18 @@ extern "C" int bbkde_eval_noalloc(const bbkde_kernel_desc *kernel, int64_t n_ref
   a.qy = qy;
   a.r_begin = 0;
   a.r_end = n_ref;
-  a.seg_len = seg_len;
+  a.seg_len = pl.seg_len;
   a.q_begin = 0;
   a.q_count = n_query;
   a.exclude_self = 0;
   a.scale = 1.0;
   a.out = partial;   // every (segment, query) entry is written: nothing to clear
   a.status = nullptr;
-  dim3 grid((unsigned)qtiles, (unsigned)nseg);
-  if (dim == 2) dispatch_op<2>(r.op, false, variant, grid, st, a);
-  else dispatch_op<1>(r.op, false, variant, grid, st, a);
-  k_combine<<<grid1d(n_query, kRedBlock), kRedBlock, 0, st>>>(
-      partial, (int)nseg, n_query, normalized ? r.norm : 1.0, out, EPI_NONE, nullptr, nullptr);
+  const dim3 grid(pl.gx, (unsigned)pl.nseg);
+  if (dim == 2) dispatch_op<2>(r.op, false, kSplitVariant, grid, st, a);
+  else dispatch_op<1>(r.op, false, kSplitVariant, grid, st, a);
+  launch_combine(st, partial, pl.nseg, n_query, normalized ? r.norm : 1.0, out, EPI_NONE,
+                 nullptr, nullptr);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     noalloc_msg(errbuf, errbuf_len, "kernel launch: %s", cudaGetErrorString(e));

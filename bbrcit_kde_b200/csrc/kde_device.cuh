@@ -15,6 +15,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 namespace bbkde {
@@ -25,7 +26,7 @@ enum Op : int {
   OP_GAUSS_PROD = 1,  // exp2(sx dx^2 + sy dy^2)               product Gaussian, hx != hy
   OP_EPAN_ISO = 2,    // max(1 + s |d|^2, 0)                   Epanechnikov
   OP_EPAN_PROD = 3,   // max(1 + sx dx^2, 0) max(1 + sy dy^2, 0)
-  OP_EPAN_CONV = 4    // prod_k c_k^3 (u_k^2 + 6 u_k + 4), u_k = |d_k| i_k, c_k = max(2-u_k,0)
+  OP_EPAN_CONV = 4    // prod_k c_k^3 (v_k^2 + 3 v_k + 1), v_k = |d_k| i_k, c_k = max(1-v_k,0)
 };
 
 constexpr int kChunk = 32;   // references per FP32 partial before the Kahan fold
@@ -36,90 +37,90 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
-// (2 - u)^3 (u^2 + 6u + 4) on u = |d| / (h a) < 2, else 0. The 1/32 of the
-// reference's polynomial (KernelTraits.h:338-342) is folded into the mass.
-__device__ __forceinline__ float epan_conv_f(float d, float inv) {
-  float u = fabsf(d) * inv;
-  float c = fmaxf(2.0f - u, 0.0f);
-  float q = fmaf(u, u + 6.0f, 4.0f);
-  return (c * c) * (c * q);
-}
+// The Epanechnikov convolution (2 - u)^3 (u^2 + 6u + 4) / 32 on u = |d| / (h a) < 2
+// (KernelTraits.h:338-342) in v = u / 2: (1 - v)^3 (v^2 + 3v + 1), the same value with
+// every power of two folded into the record's scale 1 / (2 h a).
 __device__ __forceinline__ double epan_conv_d(double d, double inv) {
-  double u = fabs(d) * inv;
-  double c = fmax(2.0 - u, 0.0);
-  return c * c * c * (u * u + 6.0 * u + 4.0);
+  const double v = fabs(d) * inv;
+  const double c = 1.0 - v > 0.0 ? 1.0 - v : 0.0;
+  return c * c * c * (v * v + 3.0 * v + 1.0);
 }
 
-// Unnormalised U(q, r) in FP32 for a packed record. D = 2: r = {x, y, m, s},
-// e = second scale (product kernels). D = 1: r = {x, m, s, 0}.
-template <int OP, int D>
-__device__ __forceinline__ float pair_u(float qx, float qy, const float4 &r, float e) {
-  if (D == 2) {
-    float dx = qx - r.x;
-    float dy = qy - r.y;
-    if (OP == OP_GAUSS_ISO) {
-      float d2 = fmaf(dy, dy, dx * dx);
-      return ex2_approx(d2 * r.w);
-    } else if (OP == OP_GAUSS_PROD) {
-      float ax = dx * dx;
-      float ay = dy * dy;
-      return ex2_approx(fmaf(ay, e, ax * r.w));
-    } else if (OP == OP_EPAN_ISO) {
-      float d2 = fmaf(dy, dy, dx * dx);
-      return fmaxf(fmaf(d2, r.w, 1.0f), 0.0f);
-    } else if (OP == OP_EPAN_PROD) {
-      float tx = fmaxf(fmaf(dx * dx, r.w, 1.0f), 0.0f);
-      float ty = fmaxf(fmaf(dy * dy, e, 1.0f), 0.0f);
-      return tx * ty;
-    } else {  // OP_EPAN_CONV
-      return epan_conv_f(dx, r.w) * epan_conv_f(dy, e);
-    }
-  } else {
-    float dx = qx - r.x;
-    if (OP == OP_GAUSS_ISO || OP == OP_GAUSS_PROD) {
-      return ex2_approx((dx * dx) * r.z);
-    } else if (OP == OP_EPAN_ISO || OP == OP_EPAN_PROD) {
-      return fmaxf(fmaf(dx * dx, r.z, 1.0f), 0.0f);
-    } else {
-      return epan_conv_f(dx, r.z);
-    }
+// max(a b + c, 0) for a b + c <= 1: the FP32 pipe's saturating multiply-add.
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+  float y;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+
+// 2^kExpBias e^x for x <= 0 (or NaN) on the FP64 pipe, 11 operations: Tang's table-driven
+// method (ACM TOMS 15, 1989). x = k ln2 / 16 + r with k rounded by the 1.5 * 2^52 shift,
+// ln2 / 16 in two terms, |r| <= ln2 / 32; e^x = 2^(k div 16) 2^(j/16) e^r, j = k mod 16.
+// e^r is its Taylor polynomial of degree 7 with the last term economised on the
+// Chebyshev polynomial T7 of that interval (relative error 8e-18). `tab` holds
+// 2^(j/16), j < 16, with j << 16 taken from the high word and the bias added, so that
+// adding k << 16 there leaves the exponent raised by k div 16; 16 doubles are all 32
+// banks, so a warp's lookups never conflict.
+// The bias keeps every value that the library's exp returns (denormals included) in the
+// normal range, without a slow path; the sum is scaled back once per query. x is
+// clamped at kExpClamp, where the value (2^-1276) is lost in that scaling unless the
+// masses sum to 2^200; the clamp works on the high word and lets a NaN of either sign
+// pass (plus 0x80000 a negative quiet NaN wraps to a small number).
+constexpr int kExpBias = 256;
+constexpr unsigned kExpClamp = 0xC08BA000u;   // high word of -884
+__device__ constexpr double kExpTab[16] = {
+    1.0, 1.0442737824274138, 1.0905077326652577, 1.1387886347566916,
+    1.189207115002721, 1.241857812073484, 1.2968395546510096, 1.3542555469368927,
+    1.4142135623730951, 1.4768261459394993, 1.5422108254079407, 1.6104903319492543,
+    1.681792830507429, 1.7562521603732995, 1.8340080864093424, 1.9152065613971474};
+
+// Entry j of the shared-memory table of exp_neg.
+__device__ __forceinline__ double exp_tab_entry(int j) {
+  return __hiloint2double(__double2hiint(kExpTab[j]) - (j << 16) + (kExpBias << 20),
+                          __double2loint(kExpTab[j]));
+}
+
+__device__ __forceinline__ double exp_neg(double x, const double *tab) {
+  const unsigned h =
+      __viaddmin_u32((unsigned)__double2hiint(x), 0x80000u, kExpClamp + 0x80000u) - 0x80000u;
+  x = __hiloint2double((int)h, __double2loint(x));
+  const double shift = 6755399441055744.0;   // 1.5 * 2^52
+  const double t = fma(x, 23.083120654223414, shift);
+  const int k = __double2loint(t);
+  const double kd = t - shift;
+  const double r = fma(kd, -1.4494042586539372e-18, fma(kd, -0.04332169878499658, x));
+  double p = fma(1.0 / 720.0, r, 0.008333496247359863);
+  p = fma(p, r, 0.041666666666666664);
+  p = fma(p, r, 0.16666666662844765);
+  p = fma(p, r, 0.5);
+  p = fma(p, r, 1.0000000000000022);
+  const double b = tab[k & 15];
+  const double s = __hiloint2double(__double2hiint(b) + (k << 16), __double2loint(b));
+  return fma(s, r * p, s);
+}
+
+// U of N queries and one FP64 record (scales s and e, natural log for the Gaussians,
+// whose values carry the factor 2^kExpBias).
+template <int OP, int D, int N>
+__device__ __forceinline__ void pair_u64(const double (&qx)[N], const double (&qy)[N], double x,
+                                         double y, double s, double e, const double *tab,
+                                         double (&u)[N]) {
+  auto pos = [](double v) { return v > 0.0 ? v : 0.0; };
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double dx = qx[k] - x, dy = D == 2 ? qy[k] - y : 0.0;
+    if (OP == OP_GAUSS_ISO || (OP == OP_GAUSS_PROD && D == 1))
+      u[k] = exp_neg((D == 2 ? dx * dx + dy * dy : dx * dx) * s, tab);
+    else if (OP == OP_GAUSS_PROD)
+      u[k] = exp_neg(dx * dx * s + dy * dy * e, tab);
+    else if (OP == OP_EPAN_ISO)
+      u[k] = pos(1.0 + (D == 2 ? dx * dx + dy * dy : dx * dx) * s);
+    else if (OP == OP_EPAN_PROD)
+      u[k] = D == 2 ? pos(1.0 + dx * dx * s) * pos(1.0 + dy * dy * e) : pos(1.0 + dx * dx * s);
+    else
+      u[k] = D == 2 ? epan_conv_d(dx, s) * epan_conv_d(dy, e) : epan_conv_d(dx, s);
   }
 }
-
-template <int D>
-__device__ __forceinline__ float rec_mass(const float4 &r) { return D == 2 ? r.z : r.y; }
-
-// FP64 record: {x, y, m, s} / {x, m, s, 0} with natural-log scales.
-template <int OP, int D>
-__device__ __forceinline__ double pair_u64(double qx, double qy, const double4 &r, double e) {
-  if (D == 2) {
-    double dx = qx - r.x;
-    double dy = qy - r.y;
-    if (OP == OP_GAUSS_ISO) {
-      return exp((dx * dx + dy * dy) * r.w);
-    } else if (OP == OP_GAUSS_PROD) {
-      return exp(dx * dx * r.w + dy * dy * e);
-    } else if (OP == OP_EPAN_ISO) {
-      return fmax(1.0 + (dx * dx + dy * dy) * r.w, 0.0);
-    } else if (OP == OP_EPAN_PROD) {
-      return fmax(1.0 + dx * dx * r.w, 0.0) * fmax(1.0 + dy * dy * e, 0.0);
-    } else {
-      return epan_conv_d(dx, r.w) * epan_conv_d(dy, e);
-    }
-  } else {
-    double dx = qx - r.x;
-    if (OP == OP_GAUSS_ISO || OP == OP_GAUSS_PROD) {
-      return exp(dx * dx * r.z);
-    } else if (OP == OP_EPAN_ISO || OP == OP_EPAN_PROD) {
-      return fmax(1.0 + dx * dx * r.z, 0.0);
-    } else {
-      return epan_conv_d(dx, r.z);
-    }
-  }
-}
-
-template <int D>
-__device__ __forceinline__ double rec_mass64(const double4 &r) { return D == 2 ? r.z : r.y; }
 
 __host__ __device__ constexpr bool op_has_extra(int op) {
   return op == OP_GAUSS_PROD || op == OP_EPAN_PROD || op == OP_EPAN_CONV;
@@ -143,129 +144,15 @@ struct SumArgs {
 };
 
 // ---------------------------------------------------------------------------
-// FP32-compensated pair sum.
-// grid = (ceil(q_count / (BLOCK*QPT)), segments); block = BLOCK threads.
-// Thread t of block b owns queries b*BLOCK*QPT + k*BLOCK + t, k < QPT.
-// ---------------------------------------------------------------------------
-template <int OP, int D, int QPT, int BLOCK, int TILE>
-__device__ __forceinline__ void chunk_sum(const float4 *__restrict__ s_rec,
-                                          const float *__restrict__ s_ext, int j0,
-                                          const float (&qx)[QPT], const float (&qy)[QPT],
-                                          float (&acc)[QPT]) {
-#pragma unroll 4
-  for (int j = 0; j < kChunk; ++j) {
-    const float4 r = s_rec[j0 + j];
-    const float e = op_has_extra(OP) ? s_ext[j0 + j] : 0.0f;
-    const float m = rec_mass<D>(r);
-#pragma unroll
-    for (int k = 0; k < QPT; ++k) acc[k] = fmaf(m, pair_u<OP, D>(qx[k], qy[k], r, e), acc[k]);
-  }
-}
-
-template <int OP, int D, int QPT, int BLOCK, int TILE>
-__device__ __forceinline__ void chunk_sum_diag(const float4 *__restrict__ s_rec,
-                                               const float *__restrict__ s_ext, int j0,
-                                               int64_t r_glob0, const int64_t (&qg)[QPT],
-                                               const float (&qx)[QPT], const float (&qy)[QPT],
-                                               float (&acc)[QPT]) {
-  for (int j = 0; j < kChunk; ++j) {
-    const float4 r = s_rec[j0 + j];
-    const float e = op_has_extra(OP) ? s_ext[j0 + j] : 0.0f;
-    const float m = rec_mass<D>(r);
-    const int64_t rg = r_glob0 + j;
-#pragma unroll
-    for (int k = 0; k < QPT; ++k) {
-      float u = pair_u<OP, D>(qx[k], qy[k], r, e);
-      acc[k] = fmaf(rg == qg[k] ? 0.0f : m, u, acc[k]);
-    }
-  }
-}
-
-template <int OP, int D, int QPT, int BLOCK, int TILE, int MINB>
-__global__ void __launch_bounds__(BLOCK, MINB) k_pair_sum_f32(SumArgs a) {
-  static_assert(TILE % kChunk == 0, "tile must hold whole chunks");
-  __shared__ float4 s_rec[TILE];
-  __shared__ float s_ext[op_has_extra(OP) ? TILE : 1];
-
-  const float4 *__restrict__ refs = static_cast<const float4 *>(a.refs);
-  const float *__restrict__ ext = static_cast<const float *>(a.extra);
-  const float *__restrict__ gqx = static_cast<const float *>(a.qx);
-  const float *__restrict__ gqy = static_cast<const float *>(a.qy);
-
-  const int tid = threadIdx.x;
-  const int64_t lq0 = (int64_t)blockIdx.x * (BLOCK * QPT);
-  const int64_t r_lo = a.r_begin + (int64_t)blockIdx.y * a.seg_len;
-  const int64_t r_hi = min(r_lo + a.seg_len, a.r_end);
-
-  float qx[QPT], qy[QPT], sum[QPT], comp[QPT];
-  int64_t qg[QPT];
-#pragma unroll
-  for (int k = 0; k < QPT; ++k) {
-    int64_t lq = lq0 + k * BLOCK + tid;
-    bool ok = lq < a.q_count;
-    qg[k] = a.q_begin + lq;
-    qx[k] = ok ? gqx[a.q_begin + lq] : 0.0f;
-    qy[k] = (ok && D == 2) ? gqy[a.q_begin + lq] : 0.0f;
-    sum[k] = 0.0f;
-    comp[k] = 0.0f;
-  }
-  const int64_t qg_lo = a.q_begin + lq0;
-  const int64_t qg_hi = qg_lo + BLOCK * QPT;
-
-  for (int64_t t0 = r_lo; t0 < r_hi; t0 += TILE) {
-    __syncthreads();
-    for (int i = tid; i < TILE; i += BLOCK) {
-      int64_t r = t0 + i;
-      if (r < r_hi) {
-        s_rec[i] = refs[r];
-        if (op_has_extra(OP)) s_ext[i] = ext[r];
-      } else {
-        // Zero-mass padding: contributes exactly 0 for every operator.
-        s_rec[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (op_has_extra(OP)) s_ext[i] = 0.0f;
-      }
-    }
-    __syncthreads();
-    const bool diag = a.exclude_self && t0 < qg_hi && qg_lo < t0 + TILE;
-    for (int j0 = 0; j0 < TILE; j0 += kChunk) {
-      float acc[QPT];
-#pragma unroll
-      for (int k = 0; k < QPT; ++k) acc[k] = 0.0f;
-      if (!diag)
-        chunk_sum<OP, D, QPT, BLOCK, TILE>(s_rec, s_ext, j0, qx, qy, acc);
-      else
-        chunk_sum_diag<OP, D, QPT, BLOCK, TILE>(s_rec, s_ext, j0, t0 + j0, qg, qx, qy, acc);
-      // Kahan fold of the chunk partial.
-#pragma unroll
-      for (int k = 0; k < QPT; ++k) {
-        float y = acc[k] - comp[k];
-        float t = sum[k] + y;
-        comp[k] = (t - sum[k]) - y;
-        sum[k] = t;
-      }
-    }
-  }
-
-  double *out = a.out + (int64_t)blockIdx.y * a.q_count;
-#pragma unroll
-  for (int k = 0; k < QPT; ++k) {
-    int64_t lq = lq0 + k * BLOCK + tid;
-    if (lq < a.q_count) out[lq] = a.scale * ((double)sum[k] - (double)comp[k]);
-  }
-}
-
-// ---------------------------------------------------------------------------
 // FP32-compensated pair sum on packed f32x2 arithmetic (sm_100 FADD2 / FMUL2 /
 // FFMA2): each instruction evaluates the same operation for two queries, so a
 // Gaussian pair costs 3 packed-FP32 issue slots + 1 MUFU.EX2 instead of 6 + 1.
-// The arithmetic per query is identical to k_pair_sum_f32 (same operations,
-// same IEEE round-to-nearest), only issued two lanes at a time.
 //
 // Shared-memory records are pre-duplicated so every operand is a ready
 // register pair: r0 = {-x, -x, -y, -y}, r1 = {m, m, s, s}, r2 = {e, e, _, _}
 // (2-D) and r0 = {-x, -x, 0, 0}, r1 = {m, m, s, s} (1-D); q - x is evaluated as
 // q + (-x), which IEEE defines identically.
-// Operators: OP_GAUSS_ISO, OP_GAUSS_PROD, OP_EPAN_ISO, OP_EPAN_PROD.
+// All operators.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 
@@ -293,38 +180,52 @@ __device__ __forceinline__ float2 exp2_poly2(float2 x) {
                      __uint_as_float(__float_as_uint(p.y) + (__float_as_uint(t.y) << 23)));
 }
 
+// max(1 + s d2, 0) for two lanes: two saturating multiply-adds (1 + s d2 <= 1) instead
+// of a packed one and two maxima, which go to another pipe but cost issue slots.
+__device__ __forceinline__ float2 epan_factor2(const float2 d2, const float2 s) {
+  return make_float2(fma_sat(d2.x, s.x, 1.0f), fma_sat(d2.y, s.y, 1.0f));
+}
+
+// (1 - v)^3 (v^2 + 3v + 1) for two lanes, v = |d| inv, 0 beyond v = 1 (epan_conv_d).
+__device__ __forceinline__ float2 epan_conv2(const float2 d, const float2 inv) {
+  const float2 v = make_float2(fabsf(d.x) * inv.x, fabsf(d.y) * inv.y);
+  const float2 c = make_float2(fma_sat(v.x, -1.0f, 1.0f), fma_sat(v.y, -1.0f, 1.0f));
+  const float2 q = __ffma2_rn(v, __fadd2_rn(v, f2(3.0f)), f2(1.0f));
+  return __fmul2_rn(__fmul2_rn(c, c), __fmul2_rn(c, q));
+}
+
 // U of two pairs, one per packed lane: coordinate differences from q + (-r), the
 // reference's scales s (and sy for the product kernels).
 template <int OP, int D, bool POLY = false>
 __device__ __forceinline__ float2 pair_u2r(const float2 qx, const float2 qy, const float2 nrx,
                                            const float2 nry, const float2 s, const float2 sy) {
   float2 dx = __fadd2_rn(qx, nrx);
-  if (D == 2) {
+  if constexpr (D == 2) {
     float2 dy = __fadd2_rn(qy, nry);
-    if (OP == OP_GAUSS_ISO) {
+    if constexpr (OP == OP_GAUSS_ISO) {
       float2 d2 = __ffma2_rn(dy, dy, __fmul2_rn(dx, dx));
       float2 e = __fmul2_rn(d2, s);
       return POLY ? exp2_poly2(e) : make_float2(ex2_approx(e.x), ex2_approx(e.y));
-    } else if (OP == OP_GAUSS_PROD) {
+    } else if constexpr (OP == OP_GAUSS_PROD) {
       float2 e = __ffma2_rn(__fmul2_rn(dy, dy), sy, __fmul2_rn(__fmul2_rn(dx, dx), s));
       return POLY ? exp2_poly2(e) : make_float2(ex2_approx(e.x), ex2_approx(e.y));
-    } else if (OP == OP_EPAN_ISO) {
+    } else if constexpr (OP == OP_EPAN_ISO) {
       float2 d2 = __ffma2_rn(dy, dy, __fmul2_rn(dx, dx));
-      float2 u = __ffma2_rn(d2, s, f2(1.0f));
-      return make_float2(fmaxf(u.x, 0.0f), fmaxf(u.y, 0.0f));
-    } else {  // OP_EPAN_PROD
-      float2 ux = __ffma2_rn(__fmul2_rn(dx, dx), s, f2(1.0f));
-      float2 uy = __ffma2_rn(__fmul2_rn(dy, dy), sy, f2(1.0f));
-      return __fmul2_rn(make_float2(fmaxf(ux.x, 0.0f), fmaxf(ux.y, 0.0f)),
-                        make_float2(fmaxf(uy.x, 0.0f), fmaxf(uy.y, 0.0f)));
+      return epan_factor2(d2, s);
+    } else if constexpr (OP == OP_EPAN_PROD) {
+      return __fmul2_rn(epan_factor2(__fmul2_rn(dx, dx), s),
+                        epan_factor2(__fmul2_rn(dy, dy), sy));
+    } else {  // OP_EPAN_CONV
+      return __fmul2_rn(epan_conv2(dx, s), epan_conv2(dy, sy));
     }
   } else {
-    if (OP == OP_GAUSS_ISO || OP == OP_GAUSS_PROD) {
+    if constexpr (OP == OP_GAUSS_ISO || OP == OP_GAUSS_PROD) {
       float2 e = __fmul2_rn(__fmul2_rn(dx, dx), s);
       return POLY ? exp2_poly2(e) : make_float2(ex2_approx(e.x), ex2_approx(e.y));
+    } else if constexpr (OP == OP_EPAN_ISO || OP == OP_EPAN_PROD) {
+      return epan_factor2(__fmul2_rn(dx, dx), s);
     } else {
-      float2 u = __ffma2_rn(__fmul2_rn(dx, dx), s, f2(1.0f));
-      return make_float2(fmaxf(u.x, 0.0f), fmaxf(u.y, 0.0f));
+      return epan_conv2(dx, s);
     }
   }
 }
@@ -335,10 +236,6 @@ __device__ __forceinline__ float2 pair_u2(const float2 qx, const float2 qy, cons
                                           const float4 &r1, const float4 &r2) {
   return pair_u2r<OP, D, POLY>(qx, qy, make_float2(r0.x, r0.y), make_float2(r0.z, r0.w),
                                make_float2(r1.z, r1.w), make_float2(r2.x, r2.y));
-}
-
-__host__ __device__ constexpr bool op_packed(int op) {
-  return op == OP_GAUSS_ISO || op == OP_GAUSS_PROD || op == OP_EPAN_ISO || op == OP_EPAN_PROD;
 }
 
 // One reference (shared-memory record j) against this thread's query pairs.
@@ -476,48 +373,210 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pair_sum_f32x2(SumArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// FP64 pair sum (reference arithmetic). One query per thread.
+// FP32-compensated pair sum of small problems: a block owns 64 queries and its eight
+// warps take the references of its segment in turn, 64 at a time (two references per
+// packed operation, columns in shared memory), so that the sums of a segment meet in
+// the block and few segments fill the chip. The warps' Kahan sums are added in FP64
+// in warp order. The MUFU bound of 10,000 x 10,000 2-D Gaussian pairs is 21.5 us: 36 us
+// measured (launch and ramp about 7), 48 in the 2,048-query blocks of shape 0, which
+// left 148 SMs 200 blocks; 500 x 400: 8 us, 28 before. 128 queries, 4 warps or three
+// resident blocks per SM measured the same or slower; at 2.5e9 pairs the 4-query
+// shape of k_pair_sum_f32x2 is 6% faster.
 // ---------------------------------------------------------------------------
-template <int OP, int D, int BLOCK>
+constexpr int kSplitQueries = 64;
+constexpr int kSplitWarps = 8;
+constexpr int kSplitUnit = 64;                          // references a warp stages at a time
+constexpr int kSplitStep = kSplitWarps * kSplitUnit;    // references of one turn of the block
+
+template <int OP, int D>
+__global__ void __launch_bounds__(32 * kSplitWarps, 4) k_pair_sum_split(SumArgs a) {
+  constexpr int NW = kSplitWarps, U = kSplitUnit, QPT = kSplitQueries / 32, PER = U / 32;
+  constexpr bool kExt = op_has_extra(OP) && D == 2;
+  constexpr int COLS = (D == 2 ? 4 : 3) + (kExt ? 1 : 0);   // -x, m, s (, -y (, second s))
+  static_assert(U % kChunk == 0, "whole chunks");
+  __shared__ __align__(16) float s_ref[NW][COLS][U];
+  __shared__ double s_sum[NW][kSplitQueries];
+
+  const float4 *__restrict__ refs = static_cast<const float4 *>(a.refs);
+  const float *__restrict__ ext = static_cast<const float *>(a.extra);
+  const float *__restrict__ gqx = static_cast<const float *>(a.qx);
+  const float *__restrict__ gqy = static_cast<const float *>(a.qy);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t lq0 = (int64_t)blockIdx.x * kSplitQueries;
+  const int64_t qg0 = a.q_begin + lq0;
+  const int64_t r_lo = a.r_begin + (int64_t)blockIdx.y * a.seg_len;
+  const int64_t r_hi = min(r_lo + a.seg_len, a.r_end);
+
+  float2 qx[QPT], qy[QPT];
+  float sum[QPT], comp[QPT];
+#pragma unroll
+  for (int k = 0; k < QPT; ++k) {
+    const bool ok = lq0 + 32 * k + lane < a.q_count;
+    qx[k] = f2(ok ? gqx[qg0 + 32 * k + lane] : 0.0f);
+    qy[k] = f2(ok && D == 2 ? gqy[qg0 + 32 * k + lane] : 0.0f);
+    sum[k] = 0.0f;
+    comp[k] = 0.0f;
+  }
+  float (&st)[COLS][U] = s_ref[warp];
+  float4 rec[PER];
+  float ex[PER];
+  auto fetch = [&](int64_t t0) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int64_t r = t0 + 32 * u + lane;
+      const bool in = r < r_hi;
+      rec[u] = in ? __ldg(refs + r) : make_float4(0.f, 0.f, 0.f, 0.f);   // zero-mass padding
+      if (kExt) ex[u] = in ? __ldg(ext + r) : 0.0f;
+    }
+  };
+  int64_t t0 = r_lo + warp * U;
+  if (t0 < r_hi) fetch(t0);
+  for (; t0 < r_hi; t0 += kSplitStep) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int i = 32 * u + lane;
+      st[0][i] = -rec[u].x;
+      st[1][i] = D == 2 ? rec[u].z : rec[u].y;
+      st[2][i] = D == 2 ? rec[u].w : rec[u].z;
+      if (D == 2) st[3][i] = -rec[u].y;
+      if (kExt) st[COLS - 1][i] = ex[u];
+    }
+    __syncwarp();
+    if (t0 + kSplitStep < r_hi) fetch(t0 + kSplitStep);
+    const bool diag = a.exclude_self && t0 < qg0 + kSplitQueries && qg0 < t0 + U;
+#pragma unroll 1
+    for (int j0 = 0; j0 < U; j0 += kChunk) {
+      float2 acc[QPT];
+#pragma unroll
+      for (int k = 0; k < QPT; ++k) acc[k] = f2(0.0f);
+      auto four = [&](int j, auto diagonal) {
+        auto col = [&](int c) { return *reinterpret_cast<const float4 *>(&st[c][j0 + j]); };
+        const float4 x4 = col(0), m4 = col(1), s4 = col(2);
+        const float4 y4 = D == 2 ? col(D == 2 ? 3 : 0) : x4, e4 = kExt ? col(COLS - 1) : s4;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          auto half = [&](const float4 &v) {
+            return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
+          };
+#pragma unroll
+          for (int k = 0; k < QPT; ++k) {
+            float2 m = half(m4);
+            if (decltype(diagonal)::value) {   // zero the mass of the pair r == q
+              const int64_t rel = qg0 + 32 * k + lane - (t0 + j0 + j + 2 * h);
+              if (rel == 0) m.x = 0.0f;
+              if (rel == 1) m.y = 0.0f;
+            }
+            acc[k] = __ffma2_rn(
+                m, pair_u2r<OP, D>(qx[k], qy[k], half(x4), half(y4), half(s4), half(e4)),
+                acc[k]);
+          }
+        }
+      };
+      if (!diag) {
+#pragma unroll 4
+        for (int j = 0; j < kChunk; j += 4) four(j, std::false_type{});
+      } else {
+#pragma unroll 1
+        for (int j = 0; j < kChunk; j += 4) four(j, std::true_type{});
+      }
+      // Kahan fold of the chunk partial (even + odd references).
+#pragma unroll
+      for (int k = 0; k < QPT; ++k) {
+        const float y = (acc[k].x + acc[k].y) - comp[k];
+        const float t = sum[k] + y;
+        comp[k] = (t - sum[k]) - y;
+        sum[k] = t;
+      }
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int k = 0; k < QPT; ++k)
+    s_sum[warp][32 * k + lane] = (double)sum[k] - (double)comp[k];
+  __syncthreads();
+  if (tid < kSplitQueries && lq0 + tid < a.q_count) {
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) v += s_sum[w][tid];
+    a.out[(int64_t)blockIdx.y * a.q_count + lq0 + tid] = a.scale * v;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 pair sum (reference arithmetic). Thread t of block b owns the queries
+// (b QPT + k) BLOCK + t. The FP64 pipe (64 lanes per clock per SM) is the bound: 18
+// operations per product-Gaussian pair, 11 of them exp_neg; four queries per thread
+// give it independent chains and share the record loads. 20,011 x 15,013 product-Gaussian
+// pairs: 392 us (7.7e11 pairs/s, 74% of the bound), 703 us with the library's exp and one
+// query per thread; 2 queries 422, 8 queries 398.
+// ---------------------------------------------------------------------------
+template <int OP, int D, int QPT, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_pair_sum_f64(SumArgs a) {
-  __shared__ double4 s_rec[BLOCK];
-  __shared__ double s_ext[op_has_extra(OP) ? BLOCK : 1];
+  constexpr bool kExt = op_has_extra(OP) && D == 2;
+  constexpr bool kGauss = OP == OP_GAUSS_ISO || OP == OP_GAUSS_PROD;
+  __shared__ double2 s_a[BLOCK];                  // {x, y} / {x, m}
+  __shared__ double2 s_b[BLOCK];                  // {m, s} / {s, -}
+  __shared__ double s_ext[kExt ? BLOCK : 1];
+  __shared__ double s_tab[16];
   const double4 *__restrict__ refs = static_cast<const double4 *>(a.refs);
   const double *__restrict__ ext = static_cast<const double *>(a.extra);
   const double *__restrict__ gqx = static_cast<const double *>(a.qx);
   const double *__restrict__ gqy = static_cast<const double *>(a.qy);
 
   const int tid = threadIdx.x;
-  const int64_t lq = (int64_t)blockIdx.x * BLOCK + tid;
-  const bool ok = lq < a.q_count;
-  const int64_t qg = a.q_begin + lq;
-  const double qx = ok ? gqx[qg] : 0.0;
-  const double qy = (ok && D == 2) ? gqy[qg] : 0.0;
+  if (tid < 16) s_tab[tid] = exp_tab_entry(tid);
+  const int64_t lq0 = (int64_t)blockIdx.x * (BLOCK * QPT);
+  const int64_t qg_lo = a.q_begin + lq0, qg_hi = qg_lo + BLOCK * QPT;
+  double qx[QPT], qy[QPT], total[QPT];
+#pragma unroll
+  for (int k = 0; k < QPT; ++k) {
+    const int64_t lq = lq0 + k * BLOCK + tid;
+    const bool ok = lq < a.q_count;
+    qx[k] = ok ? gqx[a.q_begin + lq] : 0.0;
+    qy[k] = ok && D == 2 ? gqy[a.q_begin + lq] : 0.0;
+    total[k] = 0.0;
+  }
   const int64_t r_lo = a.r_begin + (int64_t)blockIdx.y * a.seg_len;
   const int64_t r_hi = min(r_lo + a.seg_len, a.r_end);
 
-  double total = 0.0;
   for (int64_t t0 = r_lo; t0 < r_hi; t0 += BLOCK) {
     __syncthreads();
-    int64_t r = t0 + tid;
+    const int64_t r = t0 + tid;
     if (r < r_hi) {
-      s_rec[tid] = refs[r];
-      if (op_has_extra(OP)) s_ext[tid] = ext[r];
-    } else {
-      s_rec[tid] = make_double4(0, 0, 0, 0);
-      if (op_has_extra(OP)) s_ext[tid] = 0.0;
+      const double4 v = refs[r];
+      s_a[tid] = make_double2(v.x, v.y);
+      s_b[tid] = make_double2(v.z, v.w);
+      if (kExt) s_ext[tid] = ext[r];
     }
     __syncthreads();
-    const int n = (int)((r_hi - t0) < BLOCK ? (r_hi - t0) : (int64_t)BLOCK);
-    for (int j = 0; j < n; ++j) {
-      const double4 rr = s_rec[j];
-      const double e = op_has_extra(OP) ? s_ext[j] : 0.0;
-      double m = rec_mass64<D>(rr);
-      if (a.exclude_self && t0 + j == qg) m = 0.0;
-      total += m * pair_u64<OP, D>(qx, qy, rr, e);
+    const int n = (int)min(r_hi - t0, (int64_t)BLOCK);
+    const bool diag = a.exclude_self && t0 < qg_hi && qg_lo < t0 + BLOCK;
+    auto one = [&](int j, auto diagonal) {
+      const double2 ra = s_a[j], rb = s_b[j];
+      const double e = kExt ? s_ext[j] : 0.0;
+      const double m = D == 2 ? rb.x : ra.y, s = D == 2 ? rb.y : rb.x;
+      double u[QPT];
+      pair_u64<OP, D>(qx, qy, ra.x, ra.y, s, e, s_tab, u);
+#pragma unroll
+      for (int k = 0; k < QPT; ++k) {
+        const bool self = decltype(diagonal)::value && t0 + j == qg_lo + k * BLOCK + tid;
+        total[k] += (self ? 0.0 : m) * u[k];
+      }
+    };
+    if (!diag) {
+#pragma unroll 2
+      for (int j = 0; j < n; ++j) one(j, std::false_type{});
+    } else {
+#pragma unroll 1
+      for (int j = 0; j < n; ++j) one(j, std::true_type{});
     }
   }
-  if (ok) a.out[(int64_t)blockIdx.y * a.q_count + lq] = a.scale * total;
+#pragma unroll
+  for (int k = 0; k < QPT; ++k) {
+    const int64_t lq = lq0 + k * BLOCK + tid;
+    const double v = kGauss ? ldexp(total[k], -kExpBias) : total[k];
+    if (lq < a.q_count) a.out[(int64_t)blockIdx.y * a.q_count + lq] = a.scale * v;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -529,18 +588,17 @@ struct PackArgs {
   int op, dim;
   double c1, c2;      // scale numerators: s = c1 / (h1 a)^2 style (see host code)
   double h1, h2;      // bandwidths
-  double mass_scale;  // folded constant factor of the unnormalised kernel
 };
 
 // The record scales per operator, with a = abw_r:
 //   GAUSS_*:  s = c1 / (h1 a)^2 (c1 = -log2(e)/2, or -log2(e)/4 for the
 //             Gaussian convolution), e = c2 / (h2 a)^2
 //   EPAN_ISO / EPAN_PROD: s = -1 / (h1 a)^2, e = -1 / (h2 a)^2
-//   EPAN_CONV: s = 1 / (h1 a), e = 1 / (h2 a); mass scaled by 1/32 per dim.
+//   EPAN_CONV: s = 1 / (2 h1 a), e = 1 / (2 h2 a)
 __device__ __forceinline__ void pack_scales(const PackArgs &p, double a, double &s, double &e) {
   if (p.op == OP_EPAN_CONV) {
-    s = 1.0 / (p.h1 * a);
-    e = 1.0 / (p.h2 * a);
+    s = 0.5 / (p.h1 * a);
+    e = 0.5 / (p.h2 * a);
   } else {
     s = p.c1 / (p.h1 * p.h1 * a * a);
     e = p.c2 / (p.h2 * p.h2 * a * a);
@@ -553,7 +611,7 @@ __global__ void k_pack_f32(PackArgs p, float4 *rec, float *ext) {
   double a = p.abw ? p.abw[i] : 1.0;
   double s, e;
   pack_scales(p, a, s, e);
-  float m = (float)(p.mass[i] * p.mass_scale);
+  float m = (float)(p.mass[i]);
   if (p.dim == 2)
     rec[i] = make_float4((float)p.x[i], (float)p.y[i], m, (float)s);
   else
@@ -567,7 +625,7 @@ __global__ void k_pack_f64(PackArgs p, double4 *rec, double *ext) {
   double a = p.abw ? p.abw[i] : 1.0;
   double s, e;
   pack_scales(p, a, s, e);
-  double m = p.mass[i] * p.mass_scale;
+  double m = p.mass[i];
   if (p.dim == 2)
     rec[i] = make_double4(p.x[i], p.y[i], m, s);
   else
@@ -615,15 +673,31 @@ __device__ __forceinline__ double block_reduce_sum(double v, double *sm) {
 
 // out[q] = scale * sum_s partial[s][q]; with EPI_W_LOG / EPI_W_VALUE also writes
 // block_sums[blockIdx.x] = sum over the block's q of w[q] * log(out[q]) / w[q] * out[q].
+// G groups of kRedBlock / G threads take the segments in turn (group g the segments g,
+// g + G, ...; their sums are added in group order): one thread per query left most SMs
+// idle and its loads in one chain (10,000 queries x 40 segments 9.5 us, 8 groups 4).
+template <int G>
 __global__ void __launch_bounds__(kRedBlock)
 k_combine(const double *partial, int nseg, int64_t q_count, double scale, double *out,
           int epi, const double *w, double *block_sums) {
+  constexpr int QB = kRedBlock / G;
   __shared__ double sm[kRedBlock];
-  int64_t q = (int64_t)blockIdx.x * kRedBlock + threadIdx.x;
-  double v = 0.0;
+  const int g = threadIdx.x / QB;
+  const int64_t q = (int64_t)blockIdx.x * QB + threadIdx.x % QB;
+  double s = 0.0;
   if (q < q_count) {
-    double s = 0.0;
-    for (int i = 0; i < nseg; ++i) s += partial[(int64_t)i * q_count + q];
+#pragma unroll 4
+    for (int i = g; i < nseg; i += G) s += partial[(int64_t)i * q_count + q];
+  }
+  if (G > 1) {
+    sm[threadIdx.x] = s;
+    __syncthreads();
+    if (g == 0)
+      for (int k = 1; k < G; ++k) s += sm[k * QB + threadIdx.x];
+    __syncthreads();
+  }
+  double v = 0.0;
+  if (g == 0 && q < q_count) {
     s *= scale;
     out[q] = s;
     if (epi == EPI_W_LOG) v = w[q] * log(s);
