@@ -300,10 +300,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_infer_tc(TcArgs ta) {
 // ===========================================================================
 // Training step on tcgen05: forward and backward of 128 points per CTA.
 //
-// One warpgroup, thread t = point t = TMEM lane t. The four 128 x 128 x 128
-// products of a step run on the tensor cores from the same stored BF16
-// matrices (canonical K-major at tc_off), reading them transposed (MN-major)
-// where the product needs it:
+// Four warpgroups; thread (row r, column group cg) owns point r = TMEM lane r and the
+// 32 features 32 cg .. 32 cg + 31 of every layer (warps w, w + 4, w + 8, w + 12 read
+// lane quarter w % 4). The step is a chain of four products with an element-wise pass
+// between them, so its time is the latency of those passes: four threads per point
+// run each pass over 32 features instead of 128, and the per-feature sums are taken
+// while the next products run. Measured, 8,192 points:
+// 18 us a launch in the step's graph, 33 with one thread per point; MUFU (two operations
+// per SiLU, twice per layer) and the 31-step butterflies of the feature sums are what
+// is left of the passes.
+//
+// The four 128 x 128 x 128 products of a step run on the tensor cores from the same
+// stored BF16 matrices (canonical K-major at tc_off), reading them transposed
+// (MN-major) where the product needs it:
 //   forward   Z2 = A1 W2^T, Z3 = A2 W3^T                 (A, B K-major)
 //   input     dA2 = dZ3 W3, dA1 = dZ2 W2                  (A K-major, B MN-major)
 //   weights   dW3 = dZ3^T A2, dW2 = dZ2^T A1 (K = points) (A, B MN-major)
@@ -311,7 +320,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_infer_tc(TcArgs ta) {
 // then dA1; [256, 384) dW3, then dW2. The 2 -> 128 and 128 -> 1 layers and every
 // per-feature sum over the points (bias gradients, dW1, dw4) run in FP32 on the
 // CUDA cores; the sums are warp butterflies then a fixed-order sum over the four
-// warps, so a step is deterministic. Rounding points (the FP64 restatement in
+// lane quarters, so a step is deterministic. Rounding points (the FP64 restatement in
 // the tests follows them): A1 = bf16(silu(z1)), A2 = bf16(silu(z2)), dZ3 =
 // bf16(dz3), dZ2 = bf16(dz2); z2, z3, dA and dW stay FP32; bias and vector
 // gradients sum the FP32 dz. Per CTA the gradient partial is written in the
@@ -319,6 +328,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_infer_tc(TcArgs ta) {
 // mbarrier wait is bounded; on expiry *status is set and the CTA stops.
 // ===========================================================================
 constexpr int kTcTrainPts = 128;
+constexpr int kTcTrainGroups = 4;                        // column groups (warpgroups)
+constexpr int kTcTrainThreads = 128 * kTcTrainGroups;
 constexpr uint32_t kTcTrainCols = 512;
 
 struct TcTrainSmem {
@@ -328,7 +339,8 @@ struct TcTrainSmem {
   static constexpr size_t kA2 = kA1 + kTcMatBytes;
   static constexpr size_t kDZ = kA2 + kTcMatBytes;               // dZ3, then dZ2
   static constexpr size_t kF = kDZ + kTcMatBytes;                // FP32 vectors
-  static constexpr size_t kFloats = 2 * kH + 4 * kH + 4 * kH;    // W1, b1 b2 b3 w4, red[4][kH]
+  // W1, b1 b2 b3 w4, three feature sums red[3][4 quarters][kH], out[4 groups][128]
+  static constexpr size_t kFloats = 2 * kH + 4 * kH + 3 * 4 * kH + 4 * kTcTrainPts;
   static constexpr size_t kBar = kF + kFloats * sizeof(float);
   static constexpr size_t kTmem = kBar + 8;
   static constexpr size_t kFail = kTmem + 8;
@@ -357,7 +369,19 @@ __device__ __forceinline__ float warp_transpose_sum(float (&v)[32], int lane) {
   return v[0];
 }
 
-__global__ void __launch_bounds__(kTcRows, 1) k_mlp_train_tc(TcTrainArgs ta) {
+// 32 floats to global memory, one whole 32-byte sector per store (sm_100's 256-bit
+// stores); rows of dW2 and dW3 start on a multiple of 32 bytes.
+static_assert(kPartStride % 8 == 0 && kOffW2 % 8 == 0 && kOffW3 % 8 == 0, "sector-aligned rows");
+__device__ __forceinline__ void store32(float *dst, const float (&v)[32]) {
+#pragma unroll
+  for (int i = 0; i < 32; i += 8)
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + i),
+                 "f"(v[i]), "f"(v[i + 1]), "f"(v[i + 2]), "f"(v[i + 3]), "f"(v[i + 4]),
+                 "f"(v[i + 5]), "f"(v[i + 6]), "f"(v[i + 7])
+                 : "memory");
+}
+
+__global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs ta) {
   using L = TcTrainSmem;
   extern __shared__ __align__(16) unsigned char smem[];
   const TrainArgs &a = ta.t;
@@ -365,19 +389,21 @@ __global__ void __launch_bounds__(kTcRows, 1) k_mlp_train_tc(TcTrainArgs ta) {
                 *A2 = smem + L::kA2, *DZ = smem + L::kDZ;
   float *fp = reinterpret_cast<float *>(smem + L::kF);
   float *W1 = fp, *b1 = W1 + 2 * kH, *b2 = b1 + kH, *b3 = b2 + kH, *w4 = b3 + kH;
-  float *red = w4 + kH;   // [4 warps][kH]
+  float *red = w4 + kH;          // [3][4 lane quarters][kH]
+  float *outp = red + 12 * kH;   // [4 column groups][128]
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L::kBar);
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L::kTmem);
   volatile int *fail = reinterpret_cast<volatile int *>(smem + L::kFail);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int quarter = warp & 3, row = quarter * 32 + lane, c0 = (warp >> 2) * 32;
 
-  tc_stage_weights(W2, W3, a.w2, a.w3, tid, kTcRows);
-  for (int i = tid; i < 2 * kH; i += kTcRows) W1[i] = a.params[kOffW1 + i];
-  for (int i = tid; i < kH; i += kTcRows) {
-    b1[i] = a.params[kOffB1 + i];
-    b2[i] = a.params[kOffB2 + i];
-    b3[i] = a.params[kOffB3 + i];
-    w4[i] = a.params[kOffW4 + i];
+  tc_stage_weights(W2, W3, a.w2, a.w3, tid, kTcTrainThreads);
+  for (int i = tid; i < 2 * kH; i += kTcTrainThreads) W1[i] = a.params[kOffW1 + i];
+  if (tid < kH) {
+    b1[tid] = a.params[kOffB1 + tid];
+    b2[tid] = a.params[kOffB2 + tid];
+    b3[tid] = a.params[kOffB3 + tid];
+    w4[tid] = a.params[kOffW4 + tid];
   }
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)));
@@ -389,15 +415,15 @@ __global__ void __launch_bounds__(kTcRows, 1) k_mlp_train_tc(TcTrainArgs ta) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   // This thread's point.
-  const int64_t p = (int64_t)blockIdx.x * kTcTrainPts + tid;
+  const int64_t p = (int64_t)blockIdx.x * kTcTrainPts + row;
   const bool valid = p < a.batch;
   float x = 0.f, y = 0.f, target = 0.f;
   if (valid) {
-    const int64_t row = a.index[p];
-    const float2 q = a.xy[row];
+    const int64_t r = train_row(a, p);
+    const float2 q = a.xy[r];
     x = (q.x - a.norm.cx) * a.norm.sx;
     y = (q.y - a.norm.cy) * a.norm.sy;
-    target = (a.target[row] - a.norm.mu) / a.norm.sigma;
+    target = (a.target[r] - a.norm.mu) / a.norm.sigma;
   }
   fence_async_smem();
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -405,7 +431,8 @@ __global__ void __launch_bounds__(kTcRows, 1) k_mlp_train_tc(TcTrainArgs ta) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+  // this thread's lane and column group of each accumulator
+  const uint32_t mine = ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
   const uint32_t tZ2 = tmem, tZ3 = tmem + 128, tW = tmem + 256;
   const uint32_t mbar = smem_u32(bar);
   const uint32_t sW2 = smem_u32(W2), sW3 = smem_u32(W3), sA1 = smem_u32(A1),
@@ -416,8 +443,8 @@ __global__ void __launch_bounds__(kTcRows, 1) k_mlp_train_tc(TcTrainArgs ta) {
   float *gp = a.grad_part + (int64_t)blockIdx.x * kPartStride;
 
   // Issue the products of `body` from thread 0 once every thread's operand
-  // rows are in shared memory; wait for them (bounded). Uniform verdict.
-  auto run = [&](auto body) -> bool {
+  // rows are in shared memory, run `meanwhile`, wait (bounded). Uniform verdict.
+  auto run = [&](auto body, auto meanwhile) -> bool {
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -426,158 +453,149 @@ __global__ void __launch_bounds__(kTcRows, 1) k_mlp_train_tc(TcTrainArgs ta) {
       body();
       tc_commit(mbar);
     }
+    meanwhile();
     if (!tc_wait(mbar, phase)) fail[0] = 1;
     phase ^= 1u;
     tc_fence_after();
     __syncthreads();
     return fail[0] == 0;
   };
-  // Per-feature sums over the CTA's points of v (32 features from c0): the warp
-  // butterfly, then warp partials summed in warp order by thread c0 + lane.
-  auto colsum = [&](float (&v)[32], int c0, float *dst, int stride) {
-    const float s = warp_transpose_sum(v, lane);
-    red[warp * kH + c0 + lane] = s;
-    __syncthreads();
-    if (tid < 32) {
-      const int n = c0 + tid;
-      dst[n * stride] = ((red[n] + red[kH + n]) + red[2 * kH + n]) + red[3 * kH + n];
-    }
-    __syncthreads();
+  // Per-feature sums over the CTA's points: the warp butterfly of v (this thread's 32
+  // features) into row `k` of red, later summed over the lane quarters in order.
+  auto colsum = [&](int k, float (&v)[32]) {
+    const float t = warp_transpose_sum(v, lane);
+    red[(4 * k + quarter) * kH + c0 + lane] = t;
   };
+  auto quarters = [&](int k, int n) {
+    const float *r = red + 4 * k * kH + n;
+    return ((r[0] + r[kH]) + r[2 * kH]) + r[3 * kH];
+  };
+  auto nothing = [] {};
   bool ok = true;
 
   // ---- forward -----------------------------------------------------------
-#pragma unroll 1
-  for (int k0 = 0; k0 < kH; k0 += 8) {
-    float v[8];
+  {
+    float v[32];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int n = k0 + i;
+    for (int i = 0; i < 32; ++i) {
+      const int n = c0 + i;
       v[i] = silu(fmaf(W1[2 * n], x, fmaf(W1[2 * n + 1], y, b1[n])));
     }
-    tc_store8<false>(A1, nullptr, tid, k0, v);
+#pragma unroll
+    for (int j = 0; j < 32; j += 8) tc_store8<false>(A1, nullptr, row, c0 + j, v + j);
   }
-  ok = run([&] { tc_gemm128(tZ2, sA1, false, sW2, false, false); });
+  ok = run([&] { tc_gemm128(tZ2, sA1, false, sW2, false, false); }, nothing);
   if (ok) {
-#pragma unroll 1
-    for (int c = 0; c < kH; c += 32) {
-      float v[32];
-      tc_ld32(tZ2 + lanes + (uint32_t)c, v);
+    float v[32];
+    tc_ld32(tZ2 + mine, v);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = silu(v[i] + b2[c + i]);
+    for (int i = 0; i < 32; ++i) v[i] = silu(v[i] + b2[c0 + i]);
 #pragma unroll
-      for (int j = 0; j < 32; j += 8) tc_store8<false>(A2, nullptr, tid, c + j, v + j);
-    }
-    ok = run([&] { tc_gemm128(tZ3, sA2, false, sW3, false, false); });
-  }
-  float out = 0.f;
-  if (ok) {
-#pragma unroll 1
-    for (int c = 0; c < kH; c += 32) {
-      float v[32];
-      tc_ld32(tZ3 + lanes + (uint32_t)c, v);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) out = fmaf(w4[c + i], silu(v[i] + b3[c + i]), out);
-    }
+    for (int j = 0; j < 32; j += 8) tc_store8<false>(A2, nullptr, row, c0 + j, v + j);
+    ok = run([&] { tc_gemm128(tZ3, sA2, false, sW3, false, false); }, nothing);
   }
   // ---- output layer and dz3 ----------------------------------------------
-  const float e = valid ? out + b4 - target : 0.f;
-  const float dy = 2.f * e * inv_b;   // dL/dy
+  float e = 0.f, dy = 0.f;
   if (ok) {
-#pragma unroll 1
-    for (int c = 0; c < kH; c += 32) {
-      float z[32], dz[32], aw[32];
-      tc_ld32(tZ3 + lanes + (uint32_t)c, z);
+    float z[32], s[32];
+    tc_ld32(tZ3 + mine, z);
+    float part = 0.f;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float zz = z[i] + b3[c + i];
-        dz[i] = dy * w4[c + i] * silu_grad(zz);
-        aw[i] = dy * silu(zz);
-      }
-#pragma unroll
-      for (int j = 0; j < 32; j += 8) tc_store8<false>(DZ, nullptr, tid, c + j, dz + j);
-      colsum(dz, c, gp + kOffB3, 1);
-      colsum(aw, c, gp + kOffW4, 1);
+    for (int i = 0; i < 32; ++i) {
+      z[i] += b3[c0 + i];
+      s[i] = silu(z[i]);
+      part = fmaf(w4[c0 + i], s[i], part);
     }
+    outp[(c0 >> 5) * kTcTrainPts + row] = part;
+    __syncthreads();
+    const float out = ((outp[row] + outp[kTcTrainPts + row]) + outp[2 * kTcTrainPts + row]) +
+                      outp[3 * kTcTrainPts + row];
+    e = valid ? out + b4 - target : 0.f;
+    dy = 2.f * e * inv_b;   // dL/dy
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      z[i] = dy * w4[c0 + i] * silu_grad(z[i]);
+      s[i] *= dy;
+    }
+#pragma unroll
+    for (int j = 0; j < 32; j += 8) tc_store8<false>(DZ, nullptr, row, c0 + j, z + j);
+    colsum(0, z);
+    colsum(1, s);
     // dA2 = dZ3 W3 -> [128, 256); dW3 = dZ3^T A2 -> [256, 384)
-    ok = run([&] {
-      tc_gemm128(tZ3, sDZ, false, sW3, true, false);
-      tc_gemm128(tW, sDZ, true, sA2, true, false);
-    });
+    ok = run(
+        [&] {
+          tc_gemm128(tZ3, sDZ, false, sW3, true, false);
+          tc_gemm128(tW, sDZ, true, sA2, true, false);
+        },
+        [&] {
+          if (tid < kH) gp[kOffB3 + tid] = quarters(0, tid);
+          else if (tid < 2 * kH) gp[kOffW4 + tid - kH] = quarters(1, tid - kH);
+        });
   }
   // ---- dz2, dW3 ------------------------------------------------------------
   if (ok) {
-#pragma unroll 1
-    for (int c = 0; c < kH; c += 32) {
-      float d[32], z[32];
-      tc_ld32(tZ3 + lanes + (uint32_t)c, d);
-      tc_ld32(tZ2 + lanes + (uint32_t)c, z);
+    float d[32], z[32];
+    tc_ld32(tZ3 + mine, d);
+    tc_ld32(tZ2 + mine, z);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) d[i] *= silu_grad(z[i] + b2[c + i]);
+    for (int i = 0; i < 32; ++i) d[i] *= silu_grad(z[i] + b2[c0 + i]);
 #pragma unroll
-      for (int j = 0; j < 32; j += 8) tc_store8<false>(DZ, nullptr, tid, c + j, d + j);
-      colsum(d, c, gp + kOffB2, 1);
-    }
-#pragma unroll 1
-    for (int c = 0; c < kH; c += 32) {   // row tid of dW3
-      float g[32];
-      tc_ld32(tW + lanes + (uint32_t)c, g);
-      // 16-byte stores: partials are kPartStride floats apart (a multiple of 4)
-      float4 *dst = reinterpret_cast<float4 *>(gp + kOffW3 + tid * kH + c);
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        dst[i] = make_float4(g[4 * i], g[4 * i + 1], g[4 * i + 2], g[4 * i + 3]);
-    }
+    for (int j = 0; j < 32; j += 8) tc_store8<false>(DZ, nullptr, row, c0 + j, d + j);
+    colsum(0, d);
+    tc_ld32(tW + mine, z);   // row `row` of dW3
+    store32(gp + kOffW3 + row * kH + c0, z);
     // dA1 = dZ2 W2 -> [128, 256); dW2 = dZ2^T A1 -> [256, 384)
-    ok = run([&] {
-      tc_gemm128(tZ3, sDZ, false, sW2, true, false);
-      tc_gemm128(tW, sDZ, true, sA1, true, false);
-    });
+    ok = run(
+        [&] {
+          tc_gemm128(tZ3, sDZ, false, sW2, true, false);
+          tc_gemm128(tW, sDZ, true, sA1, true, false);
+        },
+        [&] {
+          if (tid < kH) gp[kOffB2 + tid] = quarters(0, tid);
+        });
   }
-  // ---- dz1 and the first layer; dW2 --------------------------------------
+  // ---- dz1 and the first layer; dW2; db4 and the loss ----------------------
   if (ok) {
-#pragma unroll 1
-    for (int c = 0; c < kH; c += 32) {
-      float d[32], dxv[32], dyv[32];
-      tc_ld32(tZ3 + lanes + (uint32_t)c, d);
+    float d[32], v[32];
+    tc_ld32(tW + mine, d);   // row `row` of dW2
+    store32(gp + kOffW2 + row * kH + c0, d);
+    tc_ld32(tZ3 + mine, d);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int n = c + i;
-        d[i] *= silu_grad(fmaf(W1[2 * n], x, fmaf(W1[2 * n + 1], y, b1[n])));
-        dxv[i] = d[i] * x;
-        dyv[i] = d[i] * y;
-      }
-      colsum(d, c, gp + kOffB1, 1);
-      colsum(dxv, c, gp + kOffW1, 2);       // dW1[n][0]
-      colsum(dyv, c, gp + kOffW1 + 1, 2);   // dW1[n][1]
+    for (int i = 0; i < 32; ++i) {
+      const int n = c0 + i;
+      d[i] *= silu_grad(fmaf(W1[2 * n], x, fmaf(W1[2 * n + 1], y, b1[n])));
+      v[i] = d[i] * x;
     }
-#pragma unroll 1
-    for (int c = 0; c < kH; c += 32) {   // row tid of dW2
-      float g[32];
-      tc_ld32(tW + lanes + (uint32_t)c, g);
-      float4 *dst = reinterpret_cast<float4 *>(gp + kOffW2 + tid * kH + c);
+    colsum(1, v);   // dW1[n][0]
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        dst[i] = make_float4(g[4 * i], g[4 * i + 1], g[4 * i + 2], g[4 * i + 3]);
+    for (int i = 0; i < 32; ++i) v[i] = d[i] * y;
+    colsum(2, v);   // dW1[n][1]
+    colsum(0, d);
+  }
+  if (c0 == 0) {   // the first column group's four warps: sums over their points
+    float sd = dy, se = e * e;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sd += __shfl_xor_sync(0xffffffffu, sd, o);
+      se += __shfl_xor_sync(0xffffffffu, se, o);
+    }
+    if (lane == 0) {
+      outp[quarter] = sd;
+      outp[4 + quarter] = se;
     }
   }
-  // ---- db4 and the loss: fixed-order sums over the points ---------------
-  red[tid] = dy;
-  red[kH + tid] = e * e;
-  __syncthreads();
-  if (tid == 0) {
-    float sd = 0.f, se = 0.f;
-    for (int i = 0; i < kTcTrainPts; ++i) {
-      sd += red[i];
-      se += red[kH + i];
-    }
-    gp[kOffB4] = sd;
-    a.loss_part[blockIdx.x] = se * inv_b;
-  }
-  if (!ok && tid == 0) atomicExch(ta.status, 1);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (ok && tid < 3 * kH) {
+    const int k = tid / kH, n = tid % kH;
+    gp[k == 0 ? kOffB1 + n : kOffW1 + 2 * n + (k - 1)] = quarters(k, n);
+  }
+  if (tid == 0) {
+    gp[kOffB4] = ((outp[0] + outp[1]) + outp[2]) + outp[3];
+    a.loss_part[blockIdx.x] = (((outp[4] + outp[5]) + outp[6]) + outp[7]) * inv_b;
+    if (!ok) atomicExch(ta.status, 1);
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(kTcTrainCols));

@@ -28,8 +28,6 @@ struct bbkde_surrogate {
   __nv_bfloat16 *w2 = nullptr, *w3 = nullptr;
   float *grad_part = nullptr, *loss_part = nullptr, *loss = nullptr;
   size_t part_cap = 0;
-  int64_t *index = nullptr;
-  size_t index_cap = 0;
   float2 *xy = nullptr;
   float *target = nullptr;
   size_t data_cap = 0;
@@ -110,7 +108,7 @@ int refresh_bf16(bbkde_surrogate *s) {
   a.w3 = s->w3;
   a.nparts = 0;
   a.step = 0;
-  k_mlp_reduce<<<(kParams + 255) / 256, 256, 0, s->stream>>>(a);
+  k_mlp_reduce<<<kReduceBlocks, kReduceGroups * kReduceParams, 0, s->stream>>>(a);
   S_CUDA(s, cudaGetLastError());
   return BBKDE_OK;
 }
@@ -150,7 +148,7 @@ int ensure_parts(bbkde_surrogate *s, int64_t batch) {
     }
     s->part_cap = blocks;
   }
-  return grow(s, s->index, s->index_cap, (size_t)batch);
+  return BBKDE_OK;
 }
 
 TrainArgs train_args(bbkde_surrogate *s, int64_t batch) {
@@ -161,8 +159,9 @@ TrainArgs train_args(bbkde_surrogate *s, int64_t batch) {
   t.norm = s->norm;
   t.xy = s->xy;
   t.target = s->target;
-  t.index = s->index;
   t.batch = batch;
+  t.rows = 0;
+  t.seed = t.step = 0;
   t.grad_part = s->grad_part;
   t.loss_part = s->loss_part;
   return t;
@@ -183,16 +182,11 @@ unsigned launch_train(bbkde_surrogate *s, const TrainArgs &targs) {
     TcTrainArgs ta;
     ta.t = targs;
     ta.status = s->status;
-    k_mlp_train_tc<<<blocks, kTcRows, TcTrainSmem::kBytes, s->stream>>>(ta);
+    k_mlp_train_tc<<<blocks, kTcTrainThreads, TcTrainSmem::kBytes, s->stream>>>(ta);
   } else {
     k_mlp_train<<<blocks, kTrainWarps * 32, kTrainSmem, s->stream>>>(targs);
   }
   return blocks;
-}
-
-__global__ void k_iota(int64_t *idx, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) idx[i] = i;
 }
 
 }  // namespace
@@ -271,7 +265,7 @@ int bbkde_surrogate_destroy(bbkde_surrogate *s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   for (void *p : {(void *)s->params, (void *)s->m, (void *)s->v, (void *)s->grad,
                   (void *)s->loss, (void *)s->w2, (void *)s->w3, (void *)s->grad_part,
-                  (void *)s->loss_part, (void *)s->index, (void *)s->xy, (void *)s->target,
+                  (void *)s->loss_part, (void *)s->xy, (void *)s->target,
                   (void *)s->pred, (void *)s->status})
     if (p) cudaFree(p);
   if (s->stream) cudaStreamDestroy(s->stream);
@@ -318,7 +312,6 @@ int bbkde_surrogate_gradient(bbkde_surrogate *s, int64_t n, const double *xy,
   S_CUDA(s, cudaSetDevice(s->device));
   S_TRY(upload_data(s, n, xy, target));
   S_TRY(ensure_parts(s, n));
-  k_iota<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(s->index, n);
   const unsigned blocks = launch_train(s, train_args(s, n));
   AdamArgs a = {};
   a.grad_part = s->grad_part;
@@ -330,7 +323,7 @@ int bbkde_surrogate_gradient(bbkde_surrogate *s, int64_t n, const double *xy,
   a.grad_out = s->grad;
   a.loss_out = s->loss;
   a.step = 0;
-  k_mlp_reduce<<<(kParams + 255) / 256, 256, 0, s->stream>>>(a);
+  k_mlp_reduce<<<kReduceBlocks, kReduceGroups * kReduceParams, 0, s->stream>>>(a);
   S_CUDA(s, cudaGetLastError());
   float l = 0.f;
   if (grad)
@@ -375,13 +368,14 @@ int bbkde_surrogate_train(bbkde_surrogate *s, int64_t n, const double *xy, const
   const double b1 = cfg->beta1 > 0 ? cfg->beta1 : 0.9, b2 = cfg->beta2 > 0 ? cfg->beta2 : 0.999;
   const double eps = cfg->eps > 0 ? cfg->eps : 1e-8;
   const double lr0 = cfg->lr, lr1 = cfg->lr_final;
-  const TrainArgs targs = train_args(s, batch);
+  TrainArgs targs = train_args(s, batch);
+  targs.rows = n;
+  targs.seed = cfg->seed;
   auto enqueue_step = [&](int64_t k) -> cudaError_t {
     // k: 0-based step of this call; Adam's step counter continues across calls.
     const double frac = cfg->steps > 1 ? (double)k / (double)(cfg->steps - 1) : 1.0;
     const double lr = lr1 + 0.5 * (lr0 - lr1) * (1.0 + std::cos(3.14159265358979323846 * frac));
-    k_mlp_batch<<<(unsigned)((batch + 255) / 256), 256, 0, s->stream>>>(
-        s->index, batch, n, cfg->seed, (uint64_t)(s->adam_step + k));
+    targs.step = (uint64_t)(s->adam_step + k);
     launch_train(s, targs);
     AdamArgs a = {};
     a.grad_part = s->grad_part;
@@ -398,7 +392,7 @@ int bbkde_surrogate_train(bbkde_surrogate *s, int64_t n, const double *xy, const
     a.beta2 = (float)b2;
     a.eps = (float)eps;
     a.step = (int)(s->adam_step + k + 1);
-    k_mlp_reduce<<<(kParams + 255) / 256, 256, 0, s->stream>>>(a);
+    k_mlp_reduce<<<kReduceBlocks, kReduceGroups * kReduceParams, 0, s->stream>>>(a);
     return cudaGetLastError();
   };
   const int64_t chunk = 100;
