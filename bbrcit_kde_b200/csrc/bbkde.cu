@@ -112,6 +112,9 @@ struct bbkde_ctx {
   PackCache pack32, pack64;
   QueryCache q32[2];          // FP32 query coordinates, one slot per point set
   DevBuf partial, out_dev, block_sums, scalars, staging, status;
+  // Small uploads and results pass through page-locked host memory that the kernels
+  // read and write directly (kPinnedBytes; allocated on first use).
+  void *pinned = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
   double last_ms = 0, last_pairs = 0;
   int64_t last_launches = 0;
@@ -179,6 +182,21 @@ int ensure(bbkde_ctx *c, DevBuf &b, size_t bytes) {
   }
   b.cap = bytes;
   return BBKDE_OK;
+}
+
+// Up to this many bytes an upload is read, and a result written, by a kernel straight
+// from and to page-locked host memory: at 64 KB the link takes ~2 us, a copy of pageable
+// memory ~8 us of staging each (five per uploaded set).
+constexpr size_t kPinnedBytes = 64 << 10;
+
+// The context's page-locked buffer, or null where it cannot be had (the caller then
+// copies as it would for a large set).
+void *pinned_buffer(bbkde_ctx *c) {
+  if (!c->pinned && cudaHostAlloc(&c->pinned, kPinnedBytes, cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    c->pinned = nullptr;
+  }
+  return c->pinned;
 }
 
 void release(DevBuf &b) {
@@ -347,12 +365,10 @@ int ensure_queries(bbkde_ctx *c, int set, bool f64, const void **qx, const void 
     TRY(ensure(c, qc.x, (size_t)n * sizeof(float)));
     TRY(ensure(c, qc.y, (size_t)n * sizeof(float)));
     if (s.n > 0) {
-      k_to_f32<<<grid1d(s.n), 256, 0, c->stream>>>(s.x.as<double>(), qc.x.as<float>(), s.n);
+      k_to_f32<<<grid1d(s.n), 256, 0, c->stream>>>(
+          s.x.as<double>(), s.dim == 2 ? s.y.as<double>() : nullptr, qc.x.as<float>(),
+          qc.y.as<float>(), s.n);
       COUNT_LAUNCH(c);
-      if (s.dim == 2) {
-        k_to_f32<<<grid1d(s.n), 256, 0, c->stream>>>(s.y.as<double>(), qc.y.as<float>(), s.n);
-        COUNT_LAUNCH(c);
-      }
       CUDA_TRY(c, cudaGetLastError());
     }
     qc.set = set;
@@ -631,7 +647,6 @@ int pair_sum(bbkde_ctx *c, const Resolved &r, int precision, int qset, int64_t r
       ++launches;
     }
   }
-  CUDA_TRY(c, cudaEventRecord(c->ev2, c->stream));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   float ms = 0.f;
   CUDA_TRY(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
@@ -670,15 +685,21 @@ int eval_common(bbkde_ctx *c, const bbkde_kernel_desc *k, int64_t r_i, int64_t r
     return fail(c, BBKDE_INVALID_ARGUMENT, "point dimension does not match the kernel");
   const int64_t q_count = q_j - q_i + 1;
   double *dst = out;
-  if (!out_is_device) {
-    TRY(ensure(c, c->out_dev, (size_t)q_count * sizeof(double)));
+  const size_t out_bytes = (size_t)q_count * sizeof(double);
+  double *host =
+      !out_is_device && out_bytes <= kPinnedBytes ? static_cast<double *>(pinned_buffer(c)) : nullptr;
+  if (host) {
+    dst = host;
+  } else if (!out_is_device) {
+    TRY(ensure(c, c->out_dev, out_bytes));
     dst = c->out_dev.as<double>();
   }
   TRY(pair_sum(c, r, precision, BBKDE_QUERY, r_i, r_j, q_i, q_j,
                normalized ? r.norm : 1.0, false, dst, EPI_NONE, nullptr));
-  if (!out_is_device) {
-    CUDA_TRY(c, cudaMemcpyAsync(out, dst, (size_t)q_count * sizeof(double),
-                                cudaMemcpyDeviceToHost, c->stream));
+  if (host) {   // pair_sum has waited for the stream
+    std::memcpy(out, host, out_bytes);
+  } else if (!out_is_device) {
+    CUDA_TRY(c, cudaMemcpyAsync(out, dst, out_bytes, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   }
   return BBKDE_OK;
@@ -789,6 +810,7 @@ int bbkde_ctx_destroy(bbkde_ctx *c) {
   for (auto &q : c->q32) { release(q.x); release(q.y); }
   release(c->partial); release(c->out_dev); release(c->block_sums);
   release(c->scalars); release(c->staging); release(c->status);
+  if (c->pinned) cudaFreeHost(c->pinned);
   for (DevBuf *b : {&c->cv_x, &c->cv_y, &c->cv_w, &c->cv_cells, &c->cv_sets, &c->cv_items,
                     &c->cv_counter, &c->cv_h, &c->cv_lut, &c->cv_part, &c->cv_hist,
                     &c->cv_out, &c->cv_parts})
@@ -841,27 +863,54 @@ int bbkde_upload(bbkde_ctx *c, int role, int dim, int64_t n, const double *coord
   TRY(ensure(c, s.mass, nb));
   TRY(ensure(c, s.abw, nb));
   TRY(ensure(c, s.weight, nb));
-  TRY(ensure(c, c->staging, nb * dim));
+  // Queries are read in FP32 by every FP32 path: converted here, in the same pass.
+  QueryCache &qc = c->q32[role];
+  const bool f32 = role == BBKDE_QUERY;
+  if (f32) {
+    TRY(ensure(c, qc.x, nb / 2));
+    TRY(ensure(c, qc.y, nb / 2));
+    qc.coord_version = ~0ull;
+  }
   if (n > 0) {
-    CUDA_TRY(c, cudaMemcpyAsync(c->staging.p, coords, (size_t)n * dim * sizeof(double),
-                                cudaMemcpyHostToDevice, c->stream));
-    k_deinterleave<<<grid1d(n), 256, 0, c->stream>>>(c->staging.as<double>(), dim, n,
-                                                     s.x.as<double>(), s.y.as<double>());
+    IngestArgs in = {};
+    in.dim = dim;
+    in.n = n;
+    in.x = s.x.as<double>();
+    in.y = s.y.as<double>();
+    in.m = s.mass.as<double>();
+    in.a = s.abw.as<double>();
+    in.w = s.weight.as<double>();
+    in.fx = f32 ? qc.x.as<float>() : nullptr;
+    in.fy = qc.y.as<float>();
+    const double *cols[3] = {mass, abw, weight};
+    const double **to[3] = {&in.mass, &in.abw, &in.weight};
+    double *home[3] = {in.m, in.a, in.w};
+    size_t bytes = (size_t)n * dim * sizeof(double);
+    for (const double *col : cols) bytes += col ? nb : 0;
+    char *host = bytes <= kPinnedBytes ? static_cast<char *>(pinned_buffer(c)) : nullptr;
+    if (host) {
+      auto put = [&](const double *src, size_t len) {
+        std::memcpy(host, src, len);
+        const double *at = reinterpret_cast<const double *>(host);
+        host += len;
+        return at;
+      };
+      in.coords = put(coords, (size_t)n * dim * sizeof(double));
+      for (int k = 0; k < 3; ++k)
+        if (cols[k]) *to[k] = put(cols[k], nb);
+    } else {
+      TRY(ensure(c, c->staging, nb * dim));
+      CUDA_TRY(c, cudaMemcpyAsync(c->staging.p, coords, (size_t)n * dim * sizeof(double),
+                                  cudaMemcpyHostToDevice, c->stream));
+      in.coords = c->staging.as<double>();
+      for (int k = 0; k < 3; ++k) {
+        if (!cols[k]) continue;
+        CUDA_TRY(c, cudaMemcpyAsync(home[k], cols[k], nb, cudaMemcpyHostToDevice, c->stream));
+        *to[k] = home[k];
+      }
+    }
+    k_ingest<<<grid1d(n, 128), 128, 0, c->stream>>>(in);
     COUNT_LAUNCH(c);
-    CUDA_TRY(c, cudaGetLastError());
-    if (mass)
-      CUDA_TRY(c, cudaMemcpyAsync(s.mass.p, mass, nb, cudaMemcpyHostToDevice, c->stream));
-    else
-      k_fill<<<grid1d(n), 256, 0, c->stream>>>(s.mass.as<double>(), 1.0, n), COUNT_LAUNCH(c);
-    if (abw)
-      CUDA_TRY(c, cudaMemcpyAsync(s.abw.p, abw, nb, cudaMemcpyHostToDevice, c->stream));
-    else
-      k_fill<<<grid1d(n), 256, 0, c->stream>>>(s.abw.as<double>(), 1.0, n), COUNT_LAUNCH(c);
-    if (weight)
-      CUDA_TRY(c, cudaMemcpyAsync(s.weight.p, weight, nb, cudaMemcpyHostToDevice, c->stream));
-    else
-      CUDA_TRY(c, cudaMemcpyAsync(s.weight.p, s.mass.p, nb, cudaMemcpyDeviceToDevice,
-                                  c->stream));
     CUDA_TRY(c, cudaGetLastError());
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   }
@@ -869,6 +918,10 @@ int bbkde_upload(bbkde_ctx *c, int role, int dim, int64_t n, const double *coord
   s.n = n;
   ++s.coord_version;
   ++s.attr_version;
+  if (f32) {
+    qc.set = role;
+    qc.coord_version = s.coord_version;
+  }
   return BBKDE_OK;
 }
 
@@ -2705,8 +2758,8 @@ extern "C" int bbkde_eval_noalloc(const bbkde_kernel_desc *kernel, int64_t n_ref
   p.h1 = r.h1;
   p.h2 = r.h2;
   k_pack_f32<<<grid1d(n_ref), 256, 0, st>>>(p, rec, extc);
-  k_to_f32<<<grid1d(n_query), 256, 0, st>>>(query_x, qx, n_query);
-  if (dim == 2) k_to_f32<<<grid1d(n_query), 256, 0, st>>>(query_y, qy, n_query);
+  k_to_f32<<<grid1d(n_query), 256, 0, st>>>(query_x, dim == 2 ? query_y : nullptr, qx, qy,
+                                            n_query);
 
   // Segment the reference range as the context path does, within the scratch.
   int sm_count = 0;

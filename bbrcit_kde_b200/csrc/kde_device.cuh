@@ -633,22 +633,39 @@ __global__ void k_pack_f64(PackArgs p, double4 *rec, double *ext) {
   if (ext) ext[i] = e;
 }
 
-__global__ void k_to_f32(const double *src, float *dst, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = (float)src[i];
-}
-
-// AoS (stride dim) -> SoA columns.
-__global__ void k_deinterleave(const double *aos, int dim, int64_t n, double *x, double *y) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// FP32 copies of the coordinate columns (y null for D = 1).
+__global__ void k_to_f32(const double *x, const double *y, float *fx, float *fy, int64_t n) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  x[i] = aos[i * dim];
-  if (dim == 2) y[i] = aos[i * dim + 1];
+  fx[i] = (float)x[i];
+  if (y) fy[i] = (float)y[i];
 }
 
-__global__ void k_fill(double *dst, double v, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = v;
+// One uploaded point set -> FP64 columns, in one pass: AoS coordinates (stride dim) are
+// split, missing masses and local bandwidths are 1, a missing weight is the mass. A
+// given column that is its own destination was copied there already. fx / fy (or null)
+// get the FP32 coordinates.
+struct IngestArgs {
+  const double *coords, *mass, *abw, *weight;
+  int dim;
+  int64_t n;
+  double *x, *y, *m, *a, *w;
+  float *fx, *fy;
+};
+__global__ void k_ingest(IngestArgs p) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= p.n) return;
+  const double x = p.coords[i * p.dim], y = p.dim == 2 ? p.coords[i * p.dim + 1] : 0.0;
+  p.x[i] = x;
+  if (p.dim == 2) p.y[i] = y;
+  if (p.fx) {
+    p.fx[i] = (float)x;
+    if (p.dim == 2) p.fy[i] = (float)y;
+  }
+  const double m = p.mass ? p.mass[i] : 1.0;
+  if (p.mass != p.m) p.m[i] = m;
+  if (p.abw != p.a) p.a[i] = p.abw ? p.abw[i] : 1.0;
+  if (p.weight != p.w) p.w[i] = p.weight ? p.weight[i] : m;
 }
 
 // ---------------------------------------------------------------------------
