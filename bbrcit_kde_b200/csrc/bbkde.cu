@@ -141,7 +141,7 @@ struct bbkde_ctx {
   DevBuf gr_pred, gr_order, gr_tmin, gr_tmax, gr_bad, gr_terr, gr_flag, gr_flag_ord, gr_list,
       gr_nsel, gr_counts, gr_gmax, gr_lat_order, gr_lat_exact, gr_lat_net, gr_q_order, gr_q_exact,
       gr_q_net, gr_resid, gr_cand_ord, gr_cand_xy, gr_cand_net, gr_out, gr_part, gr_rl_idx,
-      gr_rl_xy, gr_rl_net;
+      gr_rl_xy, gr_rl_net, gr_quad_order, gr_quad_flag, gr_quad_list;
   cudaEvent_t ev3 = nullptr;
   // smallest positive abw of the reference set, for the (coordinate, attribute)
   // versions it was computed at
@@ -825,7 +825,8 @@ int bbkde_ctx_destroy(bbkde_ctx *c) {
                     &c->gr_counts, &c->gr_gmax, &c->gr_lat_order, &c->gr_lat_exact,
                     &c->gr_lat_net, &c->gr_q_order, &c->gr_q_exact, &c->gr_q_net, &c->gr_resid,
                     &c->gr_cand_ord, &c->gr_cand_xy, &c->gr_cand_net, &c->gr_out,
-                    &c->gr_part, &c->gr_rl_idx, &c->gr_rl_xy, &c->gr_rl_net})
+                    &c->gr_part, &c->gr_rl_idx, &c->gr_rl_xy, &c->gr_rl_net, &c->gr_quad_order,
+                    &c->gr_quad_flag, &c->gr_quad_list})
     release(*b);
   if (c->cv_graph) cudaGraphExecDestroy(c->cv_graph);
   if (c->ev3) cudaEventDestroy(c->ev3);
@@ -1558,6 +1559,14 @@ constexpr double kGridProbeSpan = 0.75;
 // saves on coarse lattices (measured on the Gaussian mixture: a 32-point tile of
 // 10 narrowest widths 20% faster, of 33 and 80 widths 5-7% slower).
 constexpr double kGridLatticeSpan = 16.0;
+// Exact 16-point tiles of a separable kernel run as 32-point ones: an exact grid always
+// (262,144 references, ms in 16- / 32-point tiles: 1,000 x 900 points 1.44 / 1.08, 500 x
+// 450 1.18 / 0.53, 250 x 225 0.51 / 0.32, 64 x 64 0.44 / 0.38), the pipeline's flagged
+// tiles from this many on (building the list of 2 x 2 blocks is ten small launches,
+// about 50 us) in blocks with at least kGridQuadMin of their tiles flagged (the 32-point
+// kernel sums about 1.7x the pairs per second; 8,714 tiles 8.8 -> 7.7 ms).
+constexpr int kGridWideMin = 1024;
+constexpr int kGridQuadMin = 3;
 
 // Curve order of n points (x[i * stride], y[i * stride]; y null for 1-D) into
 // `perm` (n ints).
@@ -1648,17 +1657,16 @@ void launch_cull_op(unsigned nblk, cudaStream_t st, const CullArgs &a) {
   k_pair_sum_culled<OP, D><<<nblk, 32 * kCullWarps, 0, st>>>(a);
 }
 
-// Tile-16 lists shorter than this many tiles per SM are split: each tile's
-// reference groups are shared by a cluster of 2, 4 or 8 blocks (the resident
-// tile-16 blocks per SM: 12 by shared memory; 16-block clusters measured slower:
-// 1.57 vs 1.31 ms on the 8192^2 fallback).
+// Resident tile-16 blocks per SM (12 by shared memory). Short lists are split: each
+// tile's references are shared by a cluster of 2, 4 or 8 blocks (sep_parts; 16-block
+// clusters measured slower: 1.57 vs 1.31 ms on the 8192^2 fallback).
 constexpr int kSepResidentPerSm = 12;
 
-template <int OP, int S>
+template <int OP, int T, int S>
 cudaError_t launch_cull_sep_split(unsigned nblk, cudaStream_t st, const CullArgs &a) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nblk * S);
-  cfg.blockDim = dim3(16 * 16 / 8);
+  cfg.blockDim = dim3(T * T / 8);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -1668,7 +1676,7 @@ cudaError_t launch_cull_sep_split(unsigned nblk, cudaStream_t st, const CullArgs
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_pair_sum_culled_sep<OP, 16, S>, a);
+  return cudaLaunchKernelEx(&cfg, k_pair_sum_culled_sep<OP, T, S>, a);
 }
 
 // Tensor-core form of the tile-32 factored sum: the dynamic shared memory it
@@ -1693,24 +1701,25 @@ cudaError_t launch_cull_sep_tc(unsigned nblk, cudaStream_t st, const CullArgs &a
                    : launch_cull_sep_tc_nt<OP, kSepTcShortThreads>(nblk, st, a);
 }
 
-// parts = 1: one block per tile; 2, 4, 8 (tile 16 only): clusters of that many.
+// parts = 1: one block per tile; 2, 4, 8: clusters of that many.
 // tc: tile 32 on the tensor cores (k_pair_sum_culled_sep_tc).
+template <int OP, int T>
+cudaError_t launch_cull_sep_tile(int parts, unsigned nblk, cudaStream_t st, const CullArgs &a) {
+  switch (parts) {
+    case 2: return launch_cull_sep_split<OP, T, 2>(nblk, st, a);
+    case 4: return launch_cull_sep_split<OP, T, 4>(nblk, st, a);
+    case 8: return launch_cull_sep_split<OP, T, 8>(nblk, st, a);
+    default:
+      k_pair_sum_culled_sep<OP, T><<<nblk, T * T / 8, 0, st>>>(a);
+      return cudaGetLastError();
+  }
+}
 template <int OP>
 cudaError_t launch_cull_sep(int tile, int parts, unsigned nblk, cudaStream_t st,
                             const CullArgs &a, bool tc = false, bool long_list = false) {
   if (tile == 32 && tc) return launch_cull_sep_tc<OP>(nblk, st, a, long_list);
-  if (tile == 32) {
-    k_pair_sum_culled_sep<OP, 32><<<nblk, 32 * 32 / 8, 0, st>>>(a);
-    return cudaGetLastError();
-  }
-  switch (parts) {
-    case 2: return launch_cull_sep_split<OP, 2>(nblk, st, a);
-    case 4: return launch_cull_sep_split<OP, 4>(nblk, st, a);
-    case 8: return launch_cull_sep_split<OP, 8>(nblk, st, a);
-    default:
-      k_pair_sum_culled_sep<OP, 16><<<nblk, 16 * 16 / 8, 0, st>>>(a);
-      return cudaGetLastError();
-  }
+  return tile == 32 ? launch_cull_sep_tile<OP, 32>(parts, nblk, st, a)
+                    : launch_cull_sep_tile<OP, 16>(parts, nblk, st, a);
 }
 
 // Resident factored blocks per SM: 4 at tile 32 (registers), 12 at tile 16.
@@ -1744,10 +1753,12 @@ int sep_schedule(bbkde_ctx *c, CullArgs &a, unsigned nblk) {
   return BBKDE_OK;
 }
 
-// Parts per tile for a factored launch of nblk tiles of edge `tile`.
+// Parts per tile for a factored launch of nblk tiles of edge `tile`: enough for two waves
+// of blocks (1,089 tile-16 lattice tiles of a 4,096^2 pipeline, one wave: 5.6 ms in one
+// part, 3.7 in two, 3.4 in four; 8,714 flagged tiles 7.7 in one, 8.1 in two).
+constexpr double kSepSplitWaves = 2.0;
 int sep_parts(const bbkde_ctx *c, int tile, unsigned nblk) {
-  if (tile != 16) return 1;
-  const double per = (double)c->sm_count * kSepResidentPerSm / (double)nblk;
+  const double per = kSepSplitWaves * c->sm_count * sep_resident(tile) / (double)nblk;
   return per >= 8 ? 8 : per >= 4 ? 4 : per >= 2 ? 2 : 1;
 }
 
@@ -1792,7 +1803,7 @@ int launch_culled(bbkde_ctx *c, const Resolved &r, unsigned nblk, const CullQuer
   if (tc) CUDA_TRY(c, cudaMemsetAsync(a.status, 0, sizeof(int), c->stream));
   const bool d2 = r.dim == 2;
   if (sep_tile > 0) {
-    const int parts = sep_parts(c, sep_tile, nblk);
+    const int parts = tc ? 1 : sep_parts(c, sep_tile, nblk);
     // More than one wave: launch the tiles most expensive first.
     if (parts == 1 && q.mode == 1 &&
         (int64_t)nblk > (int64_t)c->sm_count * sep_resident(sep_tile)) {
@@ -2181,12 +2192,43 @@ int grid_exact(bbkde_ctx *c, const Resolved &r, const GridDesc &g, const int *li
   q.out = out;
   q.scale = r.norm;
   const int sep = (!pair_form && r.dim == 2 && op_separable(r.op)) ? g.tile : 0;
+  // A tensor-core block cannot share its tile: lists below one wave of them run split on
+  // the FP32 pipe (289 lattice tiles of a 4,096^2 pipeline: 6.0 ms and 2.5 ms).
   const bool tc = sep == 32 && (tensor_cores == 2 ||
-                                (tensor_cores == 0 && !full && rel >= kSepTcMinRel));
+                                (tensor_cores == 0 && !full && rel >= kSepTcMinRel &&
+                                 n >= (int64_t)kSepTcResident * c->sm_count));
   const int64_t pieces = (int64_t)(g.tile / kCullPiece) * (g.tile / kCullPiece);
   const int64_t nblk = sep > 0 ? n : n * pieces;
   if (nblk > INT32_MAX) return fail(c, BBKDE_OUT_OF_RANGE, "grid: too many tiles");
   return launch_culled(c, r, (unsigned)nblk, q, rel, full, pairs, ratio, sep, 0.0, tc);
+}
+
+// Exact sums at every point of g. Tiles of 16 points of a separable kernel are summed as
+// 32-point ones, on the FP32 pipe as they would be (kGridWideMin's comment).
+int grid_exact_all(bbkde_ctx *c, const Resolved &r, const GridDesc &g, DevBuf &order, double rel,
+                   bool full, double *out, double *pairs, double *ratio, bool pair_form,
+                   int tensor_cores) {
+  const bool wide = g.tile == 16 && !pair_form && op_separable(r.op);
+  const GridDesc gw = wide ? make_grid(g.nx, g.ny, g.x0, g.dx, g.y0, g.dy, 32) : g;
+  TRY(tile_order(c, gw, order));
+  return grid_exact(c, r, gw, order.as<int>(), (int64_t)gw.ntx * gw.nty, rel, full, out, pairs,
+                    ratio, pair_form, wide ? 1 : tensor_cores);
+}
+
+// The entries of order[0, n) with a flag, in order, into list; *count of them (waits).
+int select_flagged(bbkde_ctx *c, const int *order, const int *flag, int *list, int64_t n,
+                   int *count) {
+  size_t tmp = 0;
+  CUDA_TRY(c, cub::DeviceSelect::Flagged(nullptr, tmp, order, flag, list, c->gr_nsel.as<int>(),
+                                         (int)n, c->stream));
+  TRY(ensure(c, c->ms_tmp, tmp));
+  CUDA_TRY(c, cub::DeviceSelect::Flagged(c->ms_tmp.p, tmp, order, flag, list,
+                                         c->gr_nsel.as<int>(), (int)n, c->stream));
+  c->launch_total += 2;
+  CUDA_TRY(c, cudaMemcpyAsync(count, c->gr_nsel.p, sizeof(int), cudaMemcpyDeviceToHost,
+                              c->stream));
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  return BBKDE_OK;
 }
 
 }  // namespace
@@ -2336,10 +2378,9 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
                                   h * g.dx, g.y0, h * g.dy, LT);
     const int64_t n_lat = gl.nx * gl.ny;
     TRY(ensure(c, c->gr_lat_exact, (size_t)n_lat * sizeof(double)));
-    TRY(tile_order(c, gl, c->gr_lat_order));
-    TRY(grid_exact(c, r, gl, c->gr_lat_order.as<int>(), (int64_t)gl.ntx * gl.nty,
-                   cfg->cull_rel, full, c->gr_lat_exact.as<double>(), &st.pairs,
-                   &st.max_bound_ratio, cfg->pair_form != 0, cfg->tensor_cores));
+    TRY(grid_exact_all(c, r, gl, c->gr_lat_order, cfg->cull_rel, full,
+                       c->gr_lat_exact.as<double>(), &st.pairs, &st.max_bound_ratio,
+                       cfg->pair_form != 0, cfg->tensor_cores));
     auto lattice_net = [&]() -> int {
       TRY(ensure(c, c->gr_lat_net, (size_t)n_lat * sizeof(float)));
       TRY(bbkde::surrogate_infer(sur, c->stream, n_lat, nullptr, gl.nx, gl.x0, gl.dx, gl.y0,
@@ -2369,10 +2410,9 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
     if (P == 9) {
       n_q = gq.nx * gq.ny;
       TRY(ensure(c, c->gr_q_exact, (size_t)n_q * sizeof(double)));
-      TRY(tile_order(c, gq, c->gr_q_order));
-      TRY(grid_exact(c, r, gq, c->gr_q_order.as<int>(), (int64_t)gq.ntx * gq.nty, cfg->cull_rel,
-                     full, c->gr_q_exact.as<double>(), &st.pairs, &st.max_bound_ratio,
-                     cfg->pair_form != 0, cfg->tensor_cores));
+      TRY(grid_exact_all(c, r, gq, c->gr_q_order, cfg->cull_rel, full,
+                         c->gr_q_exact.as<double>(), &st.pairs, &st.max_bound_ratio,
+                         cfg->pair_form != 0, cfg->tensor_cores));
       if (net_all) {
         TRY(quarter_net());
         q_net = c->gr_q_net.as<float>();
@@ -2434,19 +2474,9 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
       TRY(ensure(c, c->gr_cand_ord, (size_t)ntiles * sizeof(int)));
       k_rescue_mark<<<grid1d(ntiles), 256, 0, c->stream>>>(fa, c->gr_cand_ord.as<int>());
       COUNT_LAUNCH(c);
-      size_t tmp = 0;
-      CUDA_TRY(c, cub::DeviceSelect::Flagged(nullptr, tmp, c->gr_order.as<int>(),
-                                             c->gr_cand_ord.as<int>(), c->gr_list.as<int>(),
-                                             c->gr_nsel.as<int>(), (int)ntiles, c->stream));
-      TRY(ensure(c, c->ms_tmp, tmp));
-      CUDA_TRY(c, cub::DeviceSelect::Flagged(c->ms_tmp.p, tmp, c->gr_order.as<int>(),
-                                             c->gr_cand_ord.as<int>(), c->gr_list.as<int>(),
-                                             c->gr_nsel.as<int>(), (int)ntiles, c->stream));
-      c->launch_total += 2;
       int ncand = 0;
-      CUDA_TRY(c, cudaMemcpyAsync(&ncand, c->gr_nsel.p, sizeof(int), cudaMemcpyDeviceToHost,
-                                  c->stream));
-      CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+      TRY(select_flagged(c, c->gr_order.as<int>(), c->gr_cand_ord.as<int>(), c->gr_list.as<int>(),
+                         ntiles, &ncand));
       if (ncand > 0) {
         const int *cand = c->gr_list.as<int>();
         // The network on the lattice points the candidates read (their anchors
@@ -2518,22 +2548,39 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
   }
   // 7. Exact fallback on the flagged tiles.
   CUDA_TRY(c, cudaGetLastError());
-  size_t tmp = 0;
-  CUDA_TRY(c, cub::DeviceSelect::Flagged(nullptr, tmp, c->gr_order.as<int>(),
-                                         c->gr_flag_ord.as<int>(), c->gr_list.as<int>(),
-                                         c->gr_nsel.as<int>(), (int)ntiles, c->stream));
-  TRY(ensure(c, c->ms_tmp, tmp));
-  CUDA_TRY(c, cub::DeviceSelect::Flagged(c->ms_tmp.p, tmp, c->gr_order.as<int>(),
-                                         c->gr_flag_ord.as<int>(), c->gr_list.as<int>(),
-                                         c->gr_nsel.as<int>(), (int)ntiles, c->stream));
-  c->launch_total += 2;
   int nsel = 0;
   unsigned long long counts[3] = {0, 0, 0};
-  CUDA_TRY(c, cudaMemcpyAsync(&nsel, c->gr_nsel.p, sizeof(int), cudaMemcpyDeviceToHost,
-                              c->stream));
   CUDA_TRY(c, cudaMemcpyAsync(counts, c->gr_counts.p, sizeof(counts), cudaMemcpyDeviceToHost,
                               c->stream));
-  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  TRY(select_flagged(c, c->gr_order.as<int>(), c->gr_flag_ord.as<int>(), c->gr_list.as<int>(),
+                     ntiles, &nsel));
+  if (mode == BBKDE_GRID_EXACT) {
+    TRY(grid_exact_all(c, r, g, c->gr_quad_order, cfg->cull_rel, full, out, &st.pairs,
+                       &st.max_bound_ratio, cfg->pair_form != 0, cfg->tensor_cores));
+    nsel = 0;
+  } else if (T == 16 && !cfg->pair_form && op_separable(r.op) && nsel >= kGridWideMin) {
+    // 2 x 2 blocks of (nearly) all flagged tiles leave the list of single tiles
+    const GridDesc g32 = make_grid(g.nx, g.ny, g.x0, g.dx, g.y0, g.dy, 32);
+    const int64_t nquads = (int64_t)g32.ntx * g32.nty;
+    TRY(tile_order(c, g32, c->gr_quad_order));
+    TRY(ensure(c, c->gr_quad_flag, (size_t)nquads * sizeof(int)));
+    TRY(ensure(c, c->gr_quad_list, (size_t)nquads * sizeof(int)));
+    k_quads<<<grid1d(nquads), 256, 0, c->stream>>>(g, g32, c->gr_quad_order.as<int>(),
+                                                   c->gr_flag.as<int>(), kGridQuadMin,
+                                                   c->gr_quad_flag.as<int>());
+    k_single_flags<<<grid1d(ntiles), 256, 0, c->stream>>>(
+        g, g32, c->gr_order.as<int>(), c->gr_flag.as<int>(), kGridQuadMin,
+        c->gr_flag_ord.as<int>());
+    c->launch_total += 2;
+    CUDA_TRY(c, cudaGetLastError());
+    int n32 = 0;
+    TRY(select_flagged(c, c->gr_quad_order.as<int>(), c->gr_quad_flag.as<int>(),
+                       c->gr_quad_list.as<int>(), nquads, &n32));
+    TRY(select_flagged(c, c->gr_order.as<int>(), c->gr_flag_ord.as<int>(),
+                       c->gr_list.as<int>(), ntiles, &nsel));
+    TRY(grid_exact(c, r, g32, c->gr_quad_list.as<int>(), n32, cfg->cull_rel, full, out,
+                   &st.pairs, &st.max_bound_ratio));
+  }
   TRY(grid_exact(c, r, g, c->gr_list.as<int>(), nsel, cfg->cull_rel, full, out, &st.pairs,
                  &st.max_bound_ratio, cfg->pair_form != 0, cfg->tensor_cores));
   CUDA_TRY(c, cudaEventRecord(c->ev3, c->stream));

@@ -223,31 +223,35 @@ __device__ __forceinline__ int block_append(bool pred, int value, int *dst, int 
 }
 
 // One culling pass over the tiles, two levels. Each batch, thread tid < GR tests
-// one group (group_needed; it also books the bound of a group it skips); the
-// needed groups are listed in order (s_glist, GR entries), and the block then
-// tests their members in parallel (tile_needed), BLOCK at a time. The needed
-// tiles of the batch are listed in ascending order in s_list[0, total) (capacity
-// cull_list_len(BLOCK)) and handed to sum_list(total), which every thread calls.
-// With parts > 1 the block takes every parts-th batch from batch `part` on (the
-// blocks of one tile then share its reference groups). Returns the number of
-// tiles listed.
+// one group (group_needed(group, own); it also books the bound of a group it skips, if
+// the group is its own); the needed groups are listed in order (s_glist, GR entries),
+// and the block then tests their members in parallel (tile_needed), BLOCK at a time.
+// The needed tiles of the batch are listed in ascending order in s_list[0, total)
+// (capacity cull_list_len(BLOCK)) and handed to sum_list(total), which every thread
+// calls. With parts > 1 (a divisor of kGroupTiles) the blocks of one tile share its
+// references: part `part` tests the members ti with ti % parts == part of every needed
+// group, and owns the groups gi with gi % parts == part, so that neighbouring tiles,
+// which tend to be needed together, go to different parts. Returns the number of tiles
+// listed.
 template <int BLOCK, class GroupNeeded, class TileNeeded, class SumList>
 __device__ __forceinline__ int cull_pass(const CullArgs &a, int *s_list, int *s_glist, int *s_wc,
                                          GroupNeeded group_needed, TileNeeded tile_needed,
                                          SumList sum_list, int part = 0, int parts = 1) {
   constexpr int GR = cull_groups_per_batch(BLOCK);
   const int tid = threadIdx.x;
+  const int members = kGroupTiles / parts;   // of a group, tested here
   int summed = 0;
-  for (int g0 = part * GR; g0 < a.n_groups; g0 += parts * GR) {
+  for (int g0 = 0; g0 < a.n_groups; g0 += GR) {
     const int gi = g0 + tid;
-    const bool gneed = tid < GR && gi < a.n_groups && group_needed(a.groups[gi]);
+    const bool gneed =
+        tid < GR && gi < a.n_groups && group_needed(a.groups[gi], gi % parts == part);
     const int ng = block_append<BLOCK>(gneed, gi, s_glist, s_wc);
     int total = 0;
-    for (int m0 = 0; m0 < ng * kGroupTiles; m0 += BLOCK) {
+    for (int m0 = 0; m0 < ng * members; m0 += BLOCK) {
       const int m = m0 + tid;
       int ti = -1;
-      if (m < ng * kGroupTiles) {
-        ti = s_glist[m / kGroupTiles] * kGroupTiles + m % kGroupTiles;
+      if (m < ng * members) {
+        ti = s_glist[m / members] * kGroupTiles + (m % members) * parts + part;
         if (ti >= a.n_tiles || !tile_needed(a.tiles[ti])) ti = -1;
       }
       total += block_append<BLOCK>(ti >= 0, ti, s_list + total, s_wc);
@@ -407,7 +411,7 @@ __global__ void __launch_bounds__(32 * kCullWarps, 4) k_pair_sum_culled(CullArgs
 
   auto pass = [&](int phase) {
     summed += cull_pass<BLOCK>(
-        a, s_list, s_glist, s_wc, [&](const RefTile &g) { return needed(g, phase, true); },
+        a, s_list, s_glist, s_wc, [&](const RefTile &g, bool) { return needed(g, phase, true); },
         [&](const RefTile &t) { return needed(t, phase, false); }, sum_list);
   };
   // The warps' sums of query tid (tid < kCullQpb) added in warp order.

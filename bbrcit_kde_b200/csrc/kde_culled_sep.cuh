@@ -56,8 +56,8 @@ __host__ __device__ constexpr bool op_separable(int op) {
 
 // Split tiles (S > 1, launched as clusters of S blocks per tile): for short tile
 // lists, where one block per tile would leave most SMs idle while the densest
-// tiles finish, block `part` of a tile's cluster sums every S-th batch of tile
-// groups. Every part scans all groups for the largest bound (the same near/far
+// tiles finish, block `part` of a tile's cluster sums every S-th reference tile of
+// the needed groups. Every part scans all groups for the largest bound (the same near/far
 // split), the parts exchange their near-field sums through distributed shared
 // memory so that all of them use the thresholds of the total near-field sum, and
 // part 0 adds the parts' point sums in rank order. The skipped units of the
@@ -184,8 +184,9 @@ __global__ void __launch_bounds__(T *T / 8, T == 32 ? 4 : 16)
   for (int k = 0; k < NS; ++k) skipped[k] = 0.f;
   int summed = 0;
 
-  // Is tile (or group) rt needed? (as in k_pair_sum_culled)
-  auto needed = [&](const RefTile &rt, int phase, bool group) -> bool {
+  // Is tile (or group) rt needed? (as in k_pair_sum_culled; `book`: count it as skipped
+  // here if it is not)
+  auto needed = [&](const RefTile &rt, int phase, bool group, bool book) -> bool {
     if (!kGauss) {
       bool need = false;
 #pragma unroll
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(T *T / 8, T == 32 ? 4 : 16)
       const float pk = tile_peak<OP, 2>(rt, s_box[k][0], s_box[k][1], s_box[k][2], s_box[k][3]);
       need |= pk >= kFlushExp && rt.lm + pk >= s_th[k];
     }
-    if (!need) {
+    if (!need && book) {
 #pragma unroll
       for (int k = 0; k < NS; ++k) {
         const float pk = tile_peak<OP, 2>(rt, s_box[k][0], s_box[k][1], s_box[k][2], s_box[k][3]);
@@ -337,8 +338,9 @@ __global__ void __launch_bounds__(T *T / 8, T == 32 ? 4 : 16)
 
   auto pass = [&](int phase) {
     summed += cull_pass<BLOCK>(
-        a, s_list, s_glist, s_wc, [&](const RefTile &g) { return needed(g, phase, true); },
-        [&](const RefTile &rt) { return needed(rt, phase, false); }, sum_list, part, S);
+        a, s_list, s_glist, s_wc,
+        [&](const RefTile &g, bool own) { return needed(g, phase, true, own); },
+        [&](const RefTile &rt) { return needed(rt, phase, false, true); }, sum_list, part, S);
   };
 
   // Point k = 4 kr + kc of this lane: row own(rg, kr), column own(cg, kc).

@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(NT, 4) k_pair_sum_culled_sep_tc(CullArgs a) {
 
   auto pass = [&](int phase) {
     summed += cull_pass<BLOCK>(
-        a, s_list, s_glist, s_wc, [&](const RefTile &g) { return needed(g, phase, true); },
+        a, s_list, s_glist, s_wc, [&](const RefTile &g, bool) { return needed(g, phase, true); },
         [&](const RefTile &rt) { return needed(rt, phase, false); }, sum_list);
     drain();
   };

@@ -331,6 +331,38 @@ __global__ void k_flag_tiles(FlagArgs a) {
   flag_counts_add(a.counts, low, f != 0, eb);
 }
 
+// Flagged tiles of g in its 2 x 2 block `t32` (a tile of g32, the same grid in tiles of
+// twice the edge).
+__device__ __forceinline__ int quad_flags(const GridDesc &g, const GridDesc &g32, int t32,
+                                          const int *flag) {
+  const int tx = 2 * (t32 % g32.ntx), ty = 2 * (t32 / g32.ntx);
+  int n = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int x = tx + (k & 1), y = ty + (k >> 1);
+    if (x < g.ntx && y < g.nty) n += flag[(int64_t)y * g.ntx + x] != 0;
+  }
+  return n;
+}
+
+// Which 2 x 2 blocks (per position of order32) have at least `least` flagged tiles.
+__global__ void k_quads(GridDesc g, GridDesc g32, const int *order32, const int *flag, int least,
+                        int *quad_ord) {
+  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+  if (o < g32.ntx * g32.nty)
+    quad_ord[o] = quad_flags(g, g32, order32[o], flag) >= least;
+}
+
+// Which tiles (per position of order) are flagged and not in such a block.
+__global__ void k_single_flags(GridDesc g, GridDesc g32, const int *order, const int *flag,
+                               int least, int *flag_ord) {
+  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+  if (o >= g.ntx * g.nty) return;
+  const int t = order[o];
+  const int t32 = (t / g.ntx / 2) * g32.ntx + (t % g.ntx) / 2;
+  flag_ord[o] = flag[t] && quad_flags(g, g32, t32, flag) < least;
+}
+
 // Rescue candidates: tiles flagged by their probes alone (not low, no
 // non-finite prediction), per Morton position.
 __global__ void k_rescue_mark(FlagArgs a, int *cand_ord) {

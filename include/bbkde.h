@@ -328,7 +328,7 @@ BBKDE_API int bbkde_surrogate_load(bbkde_surrogate *s, const char *path);
 /* ---- culled direct evaluation and dense grids ------------------------------ */
 
 /* Culled direct evaluation: the QUERY set against every REFERENCE point, summing
- * only the reference tiles (256 Morton-ordered points) that can contribute. For
+ * only the reference tiles (64 points in curve order) that can contribute. For
  * the Gaussian kernels the part left out is bounded, per block of queries, by
  * rel_tol times the smallest sum in that block, so every result is within
  * rel_tol (plus the FP32-compensated arithmetic error) of the full sum; for the
@@ -417,12 +417,13 @@ typedef struct {
   int lattice_tile;  /* tile edge (in lattice points) of the factored exact sums on the
                         anchor/probe lattices: 16 or 32; 0 = automatic: 32 while a
                         32-point lattice tile spans at most 16 narrowest kernel widths,
-                        else 16. A larger tile shares each kernel factor among more
-                        points but culls over a larger box */
+                        else 16. 16-point tiles of a separable kernel are summed two
+                        by two, as 32-point ones on the FP32 pipe */
   int tensor_cores;  /* factored sums on 32 x 32 tiles (lattices, exact tiles): 0 =
                         automatic: on the tcgen05 tensor cores (each factor split into
                         two TF32 terms, up to ~1e-6 relative error against FP64) when
-                        the sums are culled with cull_rel >= 1e-5, else on the FP32
+                        the sums are culled with cull_rel >= 1e-5 and the list fills
+                        the chip (592 tiles on 148 SMs), else on the FP32
                         pipe (FP32-compensated); 1 = always the FP32 pipe; 2 = always
                         the tensor cores */
 } bbkde_grid_config;
