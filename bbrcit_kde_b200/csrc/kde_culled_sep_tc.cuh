@@ -165,7 +165,8 @@ __global__ void __launch_bounds__(NT, 4) k_pair_sum_culled_sep_tc(CullArgs a) {
   __shared__ int s_glist[cull_groups_per_batch(BLOCK)];
   __shared__ int s_wc[NW];
   __shared__ float s_box[NS][4];
-  __shared__ float s_th[NS];
+  __shared__ float s_la[NS];           // log2 of the slot allowances
+  __shared__ int s_bins[kFarBins];
   __shared__ unsigned s_min[NS];
   __shared__ float s_red[NW];
   __shared__ double s_d[NS][NW];
@@ -260,6 +261,7 @@ __global__ void __launch_bounds__(NT, 4) k_pair_sum_culled_sep_tc(CullArgs a) {
   float skipped[NS];
 #pragma unroll
   for (int k = 0; k < NS; ++k) skipped[k] = 0.f;
+  float t0 = 0.f, tn = 0.f;   // far thresholds relative to the allowances (groups, tiles)
   int summed = 0;
 
   auto needed = [&](const RefTile &rt, int phase, bool group) -> bool {
@@ -279,13 +281,13 @@ __global__ void __launch_bounds__(NT, 4) k_pair_sum_culled_sep_tc(CullArgs a) {
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
       const float pk = tile_peak<OP, 2>(rt, s_box[k][0], s_box[k][1], s_box[k][2], s_box[k][3]);
-      need |= pk >= kFlushExp && rt.lm + pk >= s_th[k];
+      need |= pk >= kFlushExp && rt.lm + pk - s_la[k] >= (group ? t0 : tn);
     }
     if (!need) {
 #pragma unroll
       for (int k = 0; k < NS; ++k) {
         const float pk = tile_peak<OP, 2>(rt, s_box[k][0], s_box[k][1], s_box[k][2], s_box[k][3]);
-        if (pk >= kFlushExp) skipped[k] += ex2_approx(rt.lm + pk - s_th[k]);
+        if (pk >= kFlushExp) skipped[k] += ex2_approx(rt.lm + pk - s_la[k] - tn);
       }
     }
     return need;
@@ -456,10 +458,24 @@ __global__ void __launch_bounds__(NT, 4) k_pair_sum_culled_sep_tc(CullArgs a) {
     if (tid < NS) {
       const double mk = (double)__uint_as_float(s_min[tid]);
       const double allow = fmax(a.rel * mk, a.abs_n);
-      s_th[tid] = allow > 0.0 ? (float)(log2(allow) - log2((double)a.n_tiles)) - 1.0f
-                              : -INFINITY;
+      s_la[tid] = allow > 0.0 ? (float)log2(allow) : -INFINITY;
     }
     __syncthreads();
+    t0 = -log2f((float)a.n_tiles) - 2.0f;
+    tn = cull_far_level<BLOCK>(
+        a, s_bins, t0,
+        [&](const RefTile &rt, bool group) {
+          const float pb = tile_peak<OP, 2>(rt, qx0, qx1, qy0, qy1);
+          if (pb < kFlushExp || (!group && rt.lm + pb >= t_a)) return -INFINITY;
+          float e = -INFINITY;
+#pragma unroll
+          for (int k = 0; k < NS; ++k) {
+            const float pk =
+                tile_peak<OP, 2>(rt, s_box[k][0], s_box[k][1], s_box[k][2], s_box[k][3]);
+            if (pk >= kFlushExp) e = fmaxf(e, rt.lm + pk - s_la[k]);
+          }
+          return e;
+        });
     pass(2);   // far field, bound of the rest
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
@@ -482,7 +498,7 @@ __global__ void __launch_bounds__(NT, 4) k_pair_sum_culled_sep_tc(CullArgs a) {
       const double mk = (double)__uint_as_float(s_min[k]);
       smin_all = fmin(smin_all, mk);
       if (s_b[k] > 0.0)
-        ratio = fmax(ratio, s_b[k] * exp2((double)s_th[k]) / fmax(a.rel * mk, a.abs_n));
+        ratio = fmax(ratio, s_b[k] * exp2((double)tn));
     }
   } else {
     pass(0);
