@@ -723,6 +723,17 @@ int self_checks(bbkde_ctx *c, const bbkde_kernel_desc *k, int precision, Resolve
   return BBKDE_OK;
 }
 
+// The same unnormalised sums: the Gaussian product's convolution kernel keeps the
+// product kernel's exponent by default (KernelTraits.h:444-446), so that one pass over
+// the pairs serves both terms of the least-squares score.
+bool same_sums(const Resolved &a, const Resolved &b) {
+  return a.op == b.op && a.dim == b.dim && a.h1 == b.h1 && a.h2 == b.h2 &&
+         a.c1_f64 == b.c1_f64 && a.c2_f64 == b.c2_f64;
+}
+
+// FP64 sum of w_i m_i over the REFERENCE set in a fixed order -> *dst (device).
+int weighted_mass(bbkde_ctx *c, double *dst);
+
 int conv_kind_of(int kind, int dim) {
   if (dim == 1 && kind == BBKDE_GAUSSIAN) return BBKDE_GAUSSIAN_CONV_1D;
   if (dim == 1 && kind == BBKDE_EPANECHNIKOV) return BBKDE_EPANECHNIKOV_CONV_1D;
@@ -1046,6 +1057,17 @@ int bbkde_lsq_conv_cv(bbkde_ctx *c, const bbkde_kernel_desc *k, int precision, d
                c->out_dev.as<double>(), EPI_W_VALUE, s.weight.as<double>()));
   CUDA_TRY(c, cudaMemcpy(&llo, c->scalars.p, sizeof(double), cudaMemcpyDeviceToHost));
   const double ms = c->last_ms;
+  if (same_sums(r, rc)) {
+    // the same sums with the self terms, w_i m_i each, under the other normalisation
+    double diag = 0;
+    TRY(weighted_mass(c, c->scalars.as<double>()));
+    CUDA_TRY(c, cudaMemcpyAsync(&diag, c->scalars.p, sizeof(double), cudaMemcpyDeviceToHost,
+                                c->stream));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    sq = rc.norm / r.norm * llo + rc.norm * diag;
+    *cv_out = sq - 2 * llo;
+    return BBKDE_OK;
+  }
   // Square-integral term with the convolution kernel, all pairs (:187-205).
   TRY(pair_sum(c, rc, precision, BBKDE_REFERENCE, 0, s.n - 1, 0, s.n - 1, rc.norm, false,
                c->out_dev.as<double>(), EPI_W_VALUE, s.weight.as<double>()));
@@ -2005,6 +2027,11 @@ int wsum(bbkde_ctx *c, const double *f, const double *sub, double C, int mode, i
   return BBKDE_OK;
 }
 
+int weighted_mass(bbkde_ctx *c, double *dst) {
+  const PointSet &s = c->sets[BBKDE_REFERENCE];
+  return wsum(c, s.mass.as<double>(), nullptr, 0.0, 1, s.n, dst);
+}
+
 // Argument checks of the tolerance forms: 0 <= rel_tol < 1, finite abs_tol >= 0
 // (both 0: every tile that does not flush to zero is summed).
 int tol_checks(bbkde_ctx *c, const bbkde_kernel_desc *k, double rel_tol, double abs_tol,
@@ -2120,7 +2147,19 @@ extern "C" int bbkde_lsq_conv_cv_tol(bbkde_ctx *c, const bbkde_kernel_desc *k, d
   TRY(culled_self_sum(c, r, rel_tol, abs_tol, c->out_dev.as<double>(), &pairs, &ms));
   TRY(wsum(c, c->out_dev.as<double>(), s.mass.as<double>(), r.norm, 1, s.n,
            c->scalars.as<double>()));
-  // Square-integral term sum_i w_i f_conv(x_i), self term included (:187-205).
+  // Square-integral term sum_i w_i f_conv(x_i), self term included (:187-205). Where the
+  // sums are the same, the first ones serve under the other normalisation; their
+  // tolerance is the tighter (relative, or absolute before the larger normalisation).
+  if (same_sums(r, rc) && rc.norm <= r.norm) {
+    TRY(wsum(c, c->out_dev.as<double>(), nullptr, 0.0, 1, s.n, c->scalars.as<double>() + 1));
+    CUDA_TRY(c, cudaMemcpyAsync(t, c->scalars.p, 2 * sizeof(double), cudaMemcpyDeviceToHost,
+                                c->stream));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    *cv_out = rc.norm / r.norm * t[1] - 2.0 * t[0];
+    c->last_ms = ms;
+    c->last_pairs = pairs;
+    return BBKDE_OK;
+  }
   TRY(culled_self_sum(c, rc, rel_tol, abs_tol, c->out_dev.as<double>(), &pairs2, &ms2));
   TRY(wsum(c, c->out_dev.as<double>(), nullptr, 0.0, 1, s.n, c->scalars.as<double>() + 1));
   CUDA_TRY(c, cudaMemcpyAsync(t, c->scalars.p, 2 * sizeof(double), cudaMemcpyDeviceToHost,

@@ -129,3 +129,28 @@ def test_lsq_numint_matches_golden(ctx, name):
     assert got == pytest.approx(float(g["cv"]), rel=2e-6)
     with pytest.raises(bk.BBKDEError):
         ctx.lsq_numint_cv(desc, (sx, sy, x0, x1, y0, y1), precision=bk.FP64)
+
+
+@pytest.mark.parametrize("n", [1, 65, 700])
+@pytest.mark.parametrize("flags", [0, bk.FLAG_EXACT_GAUSS_CONV])
+def test_lsq_conv_of_the_gaussian_product(ctx, n, flags):
+    """The default convolution kernel has the product kernel's exponent, so one pass
+    serves both terms; with the exact convolution it does not. Both against sums of
+    evaluated densities (FP64 device path), with attributes that are not the weights."""
+    rng = W.SplitMix64(n)
+    xy = W.f32(rng.normal(2 * n).reshape(n, 2))
+    w = rng.uniform(n, 0.5, 1.5)
+    w /= w.sum()
+    mass, abw = w * rng.uniform(n, 0.7, 1.4), rng.uniform(n, 0.8, 1.3)
+    ctx.upload(bk.REFERENCE, xy, mass=mass, abw=abw, weight=w)
+    ctx.upload(bk.QUERY, xy)
+    h = (0.5, 0.8)
+    desc = bk.kernel_desc(W.GAUSS_PROD2D, 2, h, flags)
+    conv = bk.kernel_desc(W.GAUSS_PROD_CONV2D, 2, h, flags)
+    f = ctx.eval_all(desc, precision=bk.FP64)
+    loo = f - mass / (2 * np.pi * h[0] * h[1])
+    want = np.sum(w * ctx.eval_all(conv, precision=bk.FP64)) - 2 * np.sum(w * loo)
+    size = np.sum(w * f)
+    assert ctx.lsq_conv_cv(desc, bk.FP64) == pytest.approx(want, abs=1e-13 * size)
+    assert ctx.lsq_conv_cv(desc) == pytest.approx(want, abs=2e-6 * size)
+    assert ctx.lsq_conv_cv_tol(desc, 1e-6, 0.0) == pytest.approx(want, abs=4e-6 * size)
