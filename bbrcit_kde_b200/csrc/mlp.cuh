@@ -63,6 +63,18 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
 // z sigmoid(z) with the fast reciprocal (__fdividef, 2 ulp): for z < -88 the
 // denominator is +inf and the result is -0.
 __device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
+// silu(z) and its derivative s (1 + z (1 - s)), s = sigmoid(z), from one exponential.
+__device__ __forceinline__ void silu_both(float z, float &f, float &g) {
+  const float s = __fdividef(1.0f, 1.0f + __expf(-z));
+  f = z * s;
+  g = fmaf(f, 1.0f - s, s);
+}
+// Byte offset of element (r, k) of a 128 x 128 BF16 matrix in the tensor cores' canonical
+// K-major layout without swizzle (8 x 16-byte core matrices).
+__device__ __forceinline__ uint32_t tc_off(int r, int k) {
+  return (uint32_t)((k >> 3) * 2048 + (r >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
+}
+
 // d silu / dz = s (1 + z (1 - s)), s = sigmoid(z)
 __device__ __forceinline__ float silu_grad(float z) {
   float s = __fdividef(1.0f, 1.0f + __expf(-z));
@@ -155,7 +167,8 @@ __device__ __forceinline__ void layer4(const Frag &a3, const float *w4, float b4
 // ---------------------------------------------------------------------------
 struct InferArgs {
   const float *params;          // FP32 master (W1, b's, w4, b4)
-  const __nv_bfloat16 *w2, *w3; // BF16 [128][128]
+  const __nv_bfloat16 *w2, *w3;     // row-major (mma.sync)
+  const __nv_bfloat16 *w2c, *w3c;   // canonical layout (tcgen05)
   Norm norm;
   const float2 *xy;             // query coordinates, or null for a grid:
   int64_t gnx;                  //   point p at (gx0 + (p % gnx) gdx, gy0 + (p / gnx) gdy)
@@ -289,7 +302,8 @@ constexpr int kTrainPts = kTrainWarps * 16;
 
 struct TrainArgs {
   const float *params;
-  const __nv_bfloat16 *w2, *w3;
+  const __nv_bfloat16 *w2, *w3;     // row-major (mma.sync)
+  const __nv_bfloat16 *w2c, *w3c;   // canonical layout (tcgen05)
   Norm norm;
   const float2 *xy;             // training inputs
   const float *target;          // log-density targets
@@ -587,7 +601,8 @@ struct AdamArgs {
   const float *loss_part;
   float *params;                // FP32 master (updated when step > 0)
   float *m, *v;                 // Adam moments
-  __nv_bfloat16 *w2, *w3;       // BF16 copies refreshed from the master
+  __nv_bfloat16 *w2, *w3;       // BF16 copies refreshed from the master, row-major
+  __nv_bfloat16 *w2c, *w3c;     // and in the canonical layout (tc_off)
   float *grad_out;              // summed gradient (may be null)
   float *loss_out;              // summed loss (may be null)
   float lr, beta1, beta2, eps;
@@ -635,8 +650,13 @@ __global__ void __launch_bounds__(kReduceGroups * kReduceParams) k_mlp_reduce(Ad
     a.params[i] -= a.lr * mh / (sqrtf(vh) + a.eps);
   }
   const float p = a.params[i];
-  if (i >= kOffW2 && i < kOffW2 + kH * kH) a.w2[i - kOffW2] = __float2bfloat16_rn(p);
-  if (i >= kOffW3 && i < kOffW3 + kH * kH) a.w3[i - kOffW3] = __float2bfloat16_rn(p);
+  const __nv_bfloat16 pb = __float2bfloat16_rn(p);
+  auto put = [&](int e, __nv_bfloat16 *rm, __nv_bfloat16 *can) {
+    rm[e] = pb;
+    can[tc_off(e / kH, e % kH) / sizeof(__nv_bfloat16)] = pb;
+  };
+  if (i >= kOffW2 && i < kOffW2 + kH * kH) put(i - kOffW2, a.w2, a.w2c);
+  if (i >= kOffW3 && i < kOffW3 + kH * kH) put(i - kOffW3, a.w3, a.w3c);
 }
 constexpr unsigned kReduceBlocks = (kParams + kReduceParams - 1) / kReduceParams;
 

@@ -55,10 +55,6 @@ struct TcSmem {
   static constexpr size_t kBytes = kFail + 4 * kTcWarpgroups;
 };
 
-__device__ __forceinline__ uint32_t tc_off(int r, int k) {
-  return (uint32_t)((k >> 3) * 2048 + (r >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
-}
-
 // Shared-memory matrix descriptor: K-major, no swizzle, LBO 2048 B, SBO 128 B,
 // descriptor version 1 (bit 46).
 __device__ __forceinline__ uint64_t tc_desc(uint32_t saddr) {
@@ -146,22 +142,43 @@ __device__ __forceinline__ void tc_store8(unsigned char *ahi, unsigned char *alo
     *reinterpret_cast<uint4 *>(alo + tc_off(r, k0)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
 }
 
-// The two 128 x 128 BF16 weight matrices (row-major [n][k] in global memory)
-// into the canonical layout, 16 bytes (8 consecutive k of one row n) per copy:
-// consecutive threads take consecutive rows, so a warp's shared-memory stores
-// fill 512 contiguous bytes.
+// The two 128 x 128 BF16 weight matrices, kept in the canonical layout in global memory
+// too (k_mlp_reduce writes them so): a straight copy, 16 bytes a thread.
 __device__ __forceinline__ void tc_stage_weights(unsigned char *W2, unsigned char *W3,
                                                  const __nv_bfloat16 *w2,
                                                  const __nv_bfloat16 *w3, int tid,
                                                  int nthreads) {
-  const uint4 *g2 = reinterpret_cast<const uint4 *>(w2);
-  const uint4 *g3 = reinterpret_cast<const uint4 *>(w3);
   for (int i = tid; i < kH * kH / 8; i += nthreads) {
-    const int n = i % kH, k0 = (i / kH) * 8;
-    const int gi = n * (kH / 8) + k0 / 8;
-    *reinterpret_cast<uint4 *>(W2 + tc_off(n, k0)) = __ldg(g2 + gi);
-    *reinterpret_cast<uint4 *>(W3 + tc_off(n, k0)) = __ldg(g3 + gi);
+    reinterpret_cast<uint4 *>(W2)[i] = __ldg(reinterpret_cast<const uint4 *>(w2) + i);
+    reinterpret_cast<uint4 *>(W3)[i] = __ldg(reinterpret_cast<const uint4 *>(w3) + i);
   }
+}
+
+// 32 KB from global to shared memory as one bulk copy that completes on `mbar`.
+__device__ __forceinline__ void tc_bulk_matrix(uint32_t dst, const __nv_bfloat16 *src,
+                                               uint32_t mbar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+      ::"r"(dst), "l"(src), "r"(kTcMatBytes), "r"(mbar)
+      : "memory");
+}
+
+// 32 floats into this thread's TMEM lane (32 consecutive columns).
+__device__ __forceinline__ void tc_st32(uint32_t taddr, const float (&v)[32]) {
+  uint32_t r[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(v[i]);
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+      "%11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, "
+      "%28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+        "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
+        "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
+        "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+        "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 struct TcArgs {
@@ -183,7 +200,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_infer_tc(TcArgs ta) {
 
   const int tid = threadIdx.x, wg = tid >> 7, row = tid & 127, warp = tid >> 5;
   // Weights into the canonical layout; FP32 vectors.
-  tc_stage_weights(W2, W3, a.w2, a.w3, tid, kTcThreads);
+  tc_stage_weights(W2, W3, a.w2c, a.w3c, tid, kTcThreads);
   for (int i = tid; i < 2 * kH; i += kTcThreads) W1[i] = a.params[kOffW1 + i];
   for (int i = tid; i < kH; i += kTcThreads) {
     b1[i] = a.params[kOffB1 + i];
@@ -305,22 +322,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_infer_tc(TcArgs ta) {
 // lane quarter w % 4). The step is a chain of four products with an element-wise pass
 // between them, so its time is the latency of those passes: four threads per point
 // run each pass over 32 features instead of 128, and the per-feature sums are taken
-// while the next products run. Measured, 8,192 points:
-// 18 us a launch in the step's graph, 33 with one thread per point; MUFU (two operations
-// per SiLU, twice per layer) and the 31-step butterflies of the feature sums are what
-// is left of the passes.
+// while the next products run. Measured, a step of
+// 8,192 points with its reduction: 40 us with one thread per point, 25 with four, 20
+// with the derivatives kept in TMEM, bulk weight copies and the first layer's sums
+// through shared memory; MUFU (two operations per SiLU, three layers: 3 us) and the
+// latency of the four products with their hand-offs are what is left.
 //
 // The four 128 x 128 x 128 products of a step run on the tensor cores from the same
-// stored BF16 matrices (canonical K-major at tc_off), reading them transposed
-// (MN-major) where the product needs it:
+// stored BF16 matrices (canonical K-major at tc_off; the weights arrive as bulk copies
+// while the first layer is computed), reading them transposed (MN-major) where the
+// product needs it:
 //   forward   Z2 = A1 W2^T, Z3 = A2 W3^T                 (A, B K-major)
 //   input     dA2 = dZ3 W3, dA1 = dZ2 W2                  (A K-major, B MN-major)
 //   weights   dW3 = dZ3^T A2, dW2 = dZ2^T A1 (K = points) (A, B MN-major)
-// TMEM (512 columns): [0, 128) Z2, kept for silu'(z2); [128, 256) Z3, then dA2,
-// then dA1; [256, 384) dW3, then dW2. The 2 -> 128 and 128 -> 1 layers and every
+// TMEM (512 columns): [0, 128) Z2, then silu'(z2), then dW2; [128, 256) Z3, then dA2,
+// then dA1; [256, 384) dW3; [384, 512) silu'(z1). Each SiLU and its derivative share one
+// exponential and one reciprocal, so the backward passes need neither. The 2 -> 128 and 128 -> 1 layers and every
 // per-feature sum over the points (bias gradients, dW1, dw4) run in FP32 on the
-// CUDA cores; the sums are warp butterflies then a fixed-order sum over the four
-// lane quarters, so a step is deterministic. Rounding points (the FP64 restatement in
+// CUDA cores; the sums are warp butterflies (beside the running products; the first
+// layer's three go through shared memory, which is free by then) and then a fixed-order
+// sum over the four lane quarters, so a step is deterministic. Rounding points (the FP64 restatement in
 // the tests follows them): A1 = bf16(silu(z1)), A2 = bf16(silu(z2)), dZ3 =
 // bf16(dz3), dZ2 = bf16(dz2); z2, z3, dA and dW stay FP32; bias and vector
 // gradients sum the FP32 dz. Per CTA the gradient partial is written in the
@@ -332,6 +353,7 @@ constexpr int kTcTrainGroups = 4;                        // column groups (warpg
 constexpr int kTcTrainThreads = 128 * kTcTrainGroups;
 constexpr uint32_t kTcTrainCols = 512;
 
+constexpr int kTcTrainPtsSmem = kTcTrainPts;
 struct TcTrainSmem {
   static constexpr size_t kW2 = 0;
   static constexpr size_t kW3 = kW2 + kTcMatBytes;
@@ -341,10 +363,14 @@ struct TcTrainSmem {
   static constexpr size_t kF = kDZ + kTcMatBytes;                // FP32 vectors
   // W1, b1 b2 b3 w4, three feature sums red[3][4 quarters][kH], out[4 groups][128]
   static constexpr size_t kFloats = 2 * kH + 4 * kH + 3 * 4 * kH + 4 * kTcTrainPts;
-  static constexpr size_t kBar = kF + kFloats * sizeof(float);
-  static constexpr size_t kTmem = kBar + 8;
+  static constexpr size_t kBar = kF + kFloats * sizeof(float);   // products, weights
+  static constexpr size_t kTmem = kBar + 16;
   static constexpr size_t kFail = kTmem + 8;
   static constexpr size_t kBytes = kFail + 16;
+  // dz1 as [point][feature], padded (each 8-lane phase of a 16-byte store covers all
+  // banks), over the matrices once the products are done
+  static constexpr int kDzLd = kH + 4;
+  static_assert((size_t)kTcTrainPtsSmem * kDzLd * sizeof(float) <= kF, "fits the matrices");
 };
 
 struct TcTrainArgs {
@@ -397,7 +423,6 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int quarter = warp & 3, row = quarter * 32 + lane, c0 = (warp >> 2) * 32;
 
-  tc_stage_weights(W2, W3, a.w2, a.w3, tid, kTcTrainThreads);
   for (int i = tid; i < 2 * kH; i += kTcTrainThreads) W1[i] = a.params[kOffW1 + i];
   if (tid < kH) {
     b1[tid] = a.params[kOffB1 + tid];
@@ -406,7 +431,15 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
     w4[tid] = a.params[kOffW4 + tid];
   }
   if (tid == 0) {
+    const uint32_t wbar = smem_u32(bar + 1);
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wbar));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(wbar),
+                 "r"(2 * kTcMatBytes)
+                 : "memory");
+    tc_bulk_matrix(smem_u32(W2), a.w2c, wbar);
+    tc_bulk_matrix(smem_u32(W3), a.w3c, wbar);
     fail[0] = 0;
   }
   if (warp == 0) {
@@ -425,15 +458,13 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
     y = (q.y - a.norm.cy) * a.norm.sy;
     target = (a.target[r] - a.norm.mu) / a.norm.sigma;
   }
-  fence_async_smem();
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   // this thread's lane and column group of each accumulator
   const uint32_t mine = ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
-  const uint32_t tZ2 = tmem, tZ3 = tmem + 128, tW = tmem + 256;
+  const uint32_t tZ2 = tmem, tZ3 = tmem + 128, tW = tmem + 256, tG1 = tmem + 384;
   const uint32_t mbar = smem_u32(bar);
   const uint32_t sW2 = smem_u32(W2), sW3 = smem_u32(W3), sA1 = smem_u32(A1),
                  sA2 = smem_u32(A2), sDZ = smem_u32(DZ);
@@ -475,23 +506,26 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
 
   // ---- forward -----------------------------------------------------------
   {
-    float v[32];
+    float v[32], g[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       const int n = c0 + i;
-      v[i] = silu(fmaf(W1[2 * n], x, fmaf(W1[2 * n + 1], y, b1[n])));
+      silu_both(fmaf(W1[2 * n], x, fmaf(W1[2 * n + 1], y, b1[n])), v[i], g[i]);
     }
 #pragma unroll
     for (int j = 0; j < 32; j += 8) tc_store8<false>(A1, nullptr, row, c0 + j, v + j);
+    tc_st32(tG1 + mine, g);
   }
+  if (!tc_wait(smem_u32(bar + 1), 0)) fail[0] = 1;   // the weights are in shared memory
   ok = run([&] { tc_gemm128(tZ2, sA1, false, sW2, false, false); }, nothing);
   if (ok) {
-    float v[32];
+    float v[32], g[32];
     tc_ld32(tZ2 + mine, v);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = silu(v[i] + b2[c0 + i]);
+    for (int i = 0; i < 32; ++i) silu_both(v[i] + b2[c0 + i], v[i], g[i]);
 #pragma unroll
     for (int j = 0; j < 32; j += 8) tc_store8<false>(A2, nullptr, row, c0 + j, v + j);
+    tc_st32(tZ2 + mine, g);
     ok = run([&] { tc_gemm128(tZ3, sA2, false, sW3, false, false); }, nothing);
   }
   // ---- output layer and dz3 ----------------------------------------------
@@ -502,8 +536,7 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
     float part = 0.f;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-      z[i] += b3[c0 + i];
-      s[i] = silu(z[i]);
+      silu_both(z[i] + b3[c0 + i], s[i], z[i]);
       part = fmaf(w4[c0 + i], s[i], part);
     }
     outp[(c0 >> 5) * kTcTrainPts + row] = part;
@@ -514,13 +547,11 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
     dy = 2.f * e * inv_b;   // dL/dy
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-      z[i] = dy * w4[c0 + i] * silu_grad(z[i]);
+      z[i] *= dy * w4[c0 + i];
       s[i] *= dy;
     }
 #pragma unroll
     for (int j = 0; j < 32; j += 8) tc_store8<false>(DZ, nullptr, row, c0 + j, z + j);
-    colsum(0, z);
-    colsum(1, s);
     // dA2 = dZ3 W3 -> [128, 256); dW3 = dZ3^T A2 -> [256, 384)
     ok = run(
         [&] {
@@ -528,50 +559,66 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
           tc_gemm128(tW, sDZ, true, sA2, true, false);
         },
         [&] {
-          if (tid < kH) gp[kOffB3 + tid] = quarters(0, tid);
-          else if (tid < 2 * kH) gp[kOffW4 + tid - kH] = quarters(1, tid - kH);
+          colsum(0, z);
+          colsum(1, s);
         });
   }
   // ---- dz2, dW3 ------------------------------------------------------------
   if (ok) {
-    float d[32], z[32];
+    if (tid < kH) gp[kOffB3 + tid] = quarters(0, tid);
+    else if (tid < 2 * kH) gp[kOffW4 + tid - kH] = quarters(1, tid - kH);
+    float d[32], g[32];
     tc_ld32(tZ3 + mine, d);
-    tc_ld32(tZ2 + mine, z);
+    tc_ld32(tZ2 + mine, g);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) d[i] *= silu_grad(z[i] + b2[c0 + i]);
+    for (int i = 0; i < 32; ++i) d[i] *= g[i];
 #pragma unroll
     for (int j = 0; j < 32; j += 8) tc_store8<false>(DZ, nullptr, row, c0 + j, d + j);
-    colsum(0, d);
-    tc_ld32(tW + mine, z);   // row `row` of dW3
-    store32(gp + kOffW3 + row * kH + c0, z);
-    // dA1 = dZ2 W2 -> [128, 256); dW2 = dZ2^T A1 -> [256, 384)
+    // dA1 = dZ2 W2 -> [128, 256); dW2 = dZ2^T A1 -> [0, 128)
     ok = run(
         [&] {
           tc_gemm128(tZ3, sDZ, false, sW2, true, false);
-          tc_gemm128(tW, sDZ, true, sA1, true, false);
+          tc_gemm128(tZ2, sDZ, true, sA1, true, false);
         },
         [&] {
-          if (tid < kH) gp[kOffB2 + tid] = quarters(0, tid);
+          colsum(2, d);
+          tc_ld32(tW + mine, g);   // row `row` of dW3
+          store32(gp + kOffW3 + row * kH + c0, g);
         });
   }
   // ---- dz1 and the first layer; dW2; db4 and the loss ----------------------
   if (ok) {
-    float d[32], v[32];
-    tc_ld32(tW + mine, d);   // row `row` of dW2
-    store32(gp + kOffW2 + row * kH + c0, d);
+    if (tid < kH) gp[kOffB2 + tid] = quarters(2, tid);
+    float d[32], g[32];
     tc_ld32(tZ3 + mine, d);
+    tc_ld32(tG1 + mine, g);
+    float *dz = reinterpret_cast<float *>(smem);   // the matrices are no longer read
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const int n = c0 + i;
-      d[i] *= silu_grad(fmaf(W1[2 * n], x, fmaf(W1[2 * n + 1], y, b1[n])));
-      v[i] = d[i] * x;
+    for (int i = 0; i < 32; i += 4)
+      *reinterpret_cast<float4 *>(dz + row * L::kDzLd + c0 + i) =
+          make_float4(d[i] * g[i], d[i + 1] * g[i + 1], d[i + 2] * g[i + 2], d[i + 3] * g[i + 3]);
+    if (c0 == 0) {
+      outp[row] = x;
+      outp[kTcTrainPts + row] = y;
     }
-    colsum(1, v);   // dW1[n][0]
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = d[i] * y;
-    colsum(2, v);   // dW1[n][1]
-    colsum(0, d);
+    tc_ld32(tZ2 + mine, g);   // row `row` of dW2
+    store32(gp + kOffW2 + row * kH + c0, g);
+    __syncthreads();
+    // thread (feature n, point quarter q): db1, dW1[n][0], dW1[n][1] over 32 points
+    const int n = tid % kH, q = tid / kH;
+    float s0 = 0.f, sx = 0.f, sy = 0.f;
+#pragma unroll 8
+    for (int i = 32 * q; i < 32 * q + 32; ++i) {
+      const float v = dz[i * L::kDzLd + n];
+      s0 += v;
+      sx = fmaf(v, outp[i], sx);
+      sy = fmaf(v, outp[kTcTrainPts + i], sy);
+    }
+    red[q * kH + n] = s0;
+    red[(4 + q) * kH + n] = sx;
+    red[(8 + q) * kH + n] = sy;
   }
+  float *psum = outp + 2 * kTcTrainPts;
   if (c0 == 0) {   // the first column group's four warps: sums over their points
     float sd = dy, se = e * e;
 #pragma unroll
@@ -580,8 +627,8 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
       se += __shfl_xor_sync(0xffffffffu, se, o);
     }
     if (lane == 0) {
-      outp[quarter] = sd;
-      outp[4 + quarter] = se;
+      psum[quarter] = sd;
+      psum[4 + quarter] = se;
     }
   }
   tc_fence_before();
@@ -592,8 +639,8 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
     gp[k == 0 ? kOffB1 + n : kOffW1 + 2 * n + (k - 1)] = quarters(k, n);
   }
   if (tid == 0) {
-    gp[kOffB4] = ((outp[0] + outp[1]) + outp[2]) + outp[3];
-    a.loss_part[blockIdx.x] = (((outp[4] + outp[5]) + outp[6]) + outp[7]) * inv_b;
+    gp[kOffB4] = ((psum[0] + psum[1]) + psum[2]) + psum[3];
+    a.loss_part[blockIdx.x] = (((psum[4] + psum[5]) + psum[6]) + psum[7]) * inv_b;
     if (!ok) atomicExch(ta.status, 1);
   }
   if (warp == 0)

@@ -24,13 +24,15 @@ struct bbkde_surrogate {
   int device = 0;
   cudaStream_t stream = nullptr;
   Norm norm = {0.f, 0.f, 1.f, 1.f, 0.f, 1.f};
+  void *state = nullptr;   // one allocation: the parameter-sized arrays and flags below
   float *params = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr;
-  __nv_bfloat16 *w2 = nullptr, *w3 = nullptr;
+  __nv_bfloat16 *w2 = nullptr, *w3 = nullptr;     // row-major
+  __nv_bfloat16 *w2c = nullptr, *w3c = nullptr;   // the tensor cores' canonical layout
   float *grad_part = nullptr, *loss_part = nullptr, *loss = nullptr;
   size_t part_cap = 0;
   float2 *xy = nullptr;
   float *target = nullptr;
-  size_t data_cap = 0;
+  size_t data_cap = 0, target_cap = 0;
   float *pred = nullptr;
   size_t pred_cap = 0;
   int64_t adam_step = 0;
@@ -106,6 +108,8 @@ int refresh_bf16(bbkde_surrogate *s) {
   a.params = s->params;
   a.w2 = s->w2;
   a.w3 = s->w3;
+  a.w2c = s->w2c;
+  a.w3c = s->w3c;
   a.nparts = 0;
   a.step = 0;
   k_mlp_reduce<<<kReduceBlocks, kReduceGroups * kReduceParams, 0, s->stream>>>(a);
@@ -120,10 +124,7 @@ int upload_data(bbkde_surrogate *s, int64_t n, const double *xy, const double *t
   S_CUDA(s, cudaMemcpyAsync(s->xy, hxy.data(), n * sizeof(float2), cudaMemcpyHostToDevice,
                             s->stream));
   if (target) {
-    size_t cap = 0;
-    if (s->target) cudaFree(s->target);
-    s->target = nullptr;
-    S_TRY(grow(s, s->target, cap, (size_t)n));
+    S_TRY(grow(s, s->target, s->target_cap, (size_t)n));
     std::vector<float> ht(n);
     for (int64_t i = 0; i < n; ++i) ht[i] = (float)target[i];
     S_CUDA(s, cudaMemcpyAsync(s->target, ht.data(), n * sizeof(float), cudaMemcpyHostToDevice,
@@ -156,6 +157,8 @@ TrainArgs train_args(bbkde_surrogate *s, int64_t batch) {
   t.params = s->params;
   t.w2 = s->w2;
   t.w3 = s->w3;
+  t.w2c = s->w2c;
+  t.w3c = s->w3c;
   t.norm = s->norm;
   t.xy = s->xy;
   t.target = s->target;
@@ -212,16 +215,27 @@ int bbkde_surrogate_create(int device, uint64_t seed, bbkde_surrogate **out) {
       rc = BBKDE_CUDA_ERROR;
       break;
     }
-    if (cudaMalloc(&s->params, kParams * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&s->m, kParams * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&s->v, kParams * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&s->grad, kParams * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&s->loss, sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&s->w2, kH * kH * sizeof(__nv_bfloat16)) != cudaSuccess ||
-        cudaMalloc(&s->w3, kH * kH * sizeof(__nv_bfloat16)) != cudaSuccess ||
-        cudaMalloc(&s->status, sizeof(int)) != cudaSuccess ||
-        cudaMemset(s->status, 0, sizeof(int)) != cudaSuccess) {
+    // One allocation, each array on a 256-byte boundary.
+    const size_t vec = (kParams * sizeof(float) + 255) & ~size_t(255);
+    const size_t mat = kH * kH * sizeof(__nv_bfloat16);
+    const size_t bytes = 4 * vec + 4 * mat + 512;
+    if (cudaMalloc(&s->state, bytes) != cudaSuccess) {
       rc = BBKDE_ALLOC_FAILED;
+      break;
+    }
+    char *at = static_cast<char *>(s->state);
+    for (float **v : {&s->params, &s->m, &s->v, &s->grad}) {
+      *v = reinterpret_cast<float *>(at);
+      at += vec;
+    }
+    for (__nv_bfloat16 **w : {&s->w2, &s->w3, &s->w2c, &s->w3c}) {
+      *w = reinterpret_cast<__nv_bfloat16 *>(at);
+      at += mat;
+    }
+    s->loss = reinterpret_cast<float *>(at);
+    s->status = reinterpret_cast<int *>(at + 256);
+    if (cudaMemsetAsync(s->state, 0, bytes, s->stream) != cudaSuccess) {
+      rc = BBKDE_CUDA_ERROR;
       break;
     }
     if (cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -240,10 +254,8 @@ int bbkde_surrogate_create(int device, uint64_t seed, bbkde_surrogate **out) {
       break;
     }
     std::vector<float> p = init_params(seed);
-    if (cudaMemcpy(s->params, p.data(), kParams * sizeof(float), cudaMemcpyHostToDevice) !=
-            cudaSuccess ||
-        cudaMemset(s->m, 0, kParams * sizeof(float)) != cudaSuccess ||
-        cudaMemset(s->v, 0, kParams * sizeof(float)) != cudaSuccess) {
+    if (cudaMemcpyAsync(s->params, p.data(), kParams * sizeof(float), cudaMemcpyHostToDevice,
+                        s->stream) != cudaSuccess) {   // p outlives the wait below
       rc = BBKDE_CUDA_ERROR;
       break;
     }
@@ -263,10 +275,8 @@ int bbkde_surrogate_destroy(bbkde_surrogate *s) {
   if (!s) return BBKDE_OK;
   cudaSetDevice(s->device);
   if (s->stream) cudaStreamSynchronize(s->stream);
-  for (void *p : {(void *)s->params, (void *)s->m, (void *)s->v, (void *)s->grad,
-                  (void *)s->loss, (void *)s->w2, (void *)s->w3, (void *)s->grad_part,
-                  (void *)s->loss_part, (void *)s->xy, (void *)s->target,
-                  (void *)s->pred, (void *)s->status})
+  for (void *p : {s->state, (void *)s->grad_part, (void *)s->loss_part, (void *)s->xy,
+                  (void *)s->target, (void *)s->pred})
     if (p) cudaFree(p);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
@@ -320,6 +330,8 @@ int bbkde_surrogate_gradient(bbkde_surrogate *s, int64_t n, const double *xy,
   a.params = s->params;
   a.w2 = s->w2;
   a.w3 = s->w3;
+  a.w2c = s->w2c;
+  a.w3c = s->w3c;
   a.grad_out = s->grad;
   a.loss_out = s->loss;
   a.step = 0;
@@ -386,6 +398,8 @@ int bbkde_surrogate_train(bbkde_surrogate *s, int64_t n, const double *xy, const
     a.v = s->v;
     a.w2 = s->w2;
     a.w3 = s->w3;
+    a.w2c = s->w2c;
+    a.w3c = s->w3c;
     a.loss_out = s->loss;
     a.lr = (float)lr;
     a.beta1 = (float)b1;
@@ -438,6 +452,8 @@ int surrogate_infer(bbkde_surrogate *s, cudaStream_t st, int64_t n, const float2
   a.params = s->params;
   a.w2 = s->w2;
   a.w3 = s->w3;
+  a.w2c = s->w2c;
+  a.w3c = s->w3c;
   a.norm = s->norm;
   a.xy = xy;
   a.gnx = gnx > 0 ? gnx : 1;
