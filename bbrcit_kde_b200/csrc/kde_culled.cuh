@@ -269,16 +269,19 @@ __device__ __forceinline__ int cull_pass(const CullArgs &a, int *s_list, int *s_
 //   * Tiles below t0 = -log2(n_tiles) - 2 hold at most a quarter, however many.
 //   * The tiles from t0 up to -2 are counted per bit; the threshold is the highest bit at
 //     which the counted bounds below it (each taken at its bit's upper edge) still hold
-//     at most another quarter (with parts > 1 that share of a quarter, each part for its
-//     own tiles).
+//     at most kFarShare (with parts > 1 that share of it, each part for its own tiles).
+//     A quarter would keep the guarantee; the smaller share keeps the part left out,
+//     which is always missing on the same side, an order below the tolerance asked for
+//     (a 1-D likelihood to 1e-6: off by 4.7e-7 with a quarter).
 // A threshold of -log2(n_tiles) - 1 for every tile, which needs no count, charges each of
-// them as much as the nearest one left out: five to six bits lower. 400,000 x 300,000 at
-// 1e-6 lists 3.43e9 pairs instead of 4.10e9 (1.62 -> 1.51 ms), the flagged tiles of a
-// 4,096^2 pipeline at 1e-5 1.01e11 instead of 1.10e11 (7.8 -> 7.1 ms).
+// them as much as the nearest one left out and lies two to three bits lower: 400,000 x
+// 300,000 at 1e-6 lists 3.71e9 pairs instead of 4.10e9 (1.62 -> 1.57 ms), the flagged
+// tiles of a 4,096^2 pipeline at 1e-5 take 7.0 ms instead of 7.8.
 // level(t): the largest bound of t over the block's slots relative to their allowances,
 // -inf for a tile that is summed already or flushes to zero; a group's is at least its
 // members'. Every thread calls it and gets the result.
 constexpr int kFarBins = 32;
+constexpr float kFarShare = 1.0f / 32.0f;
 template <int BLOCK, class Level>
 __device__ __forceinline__ float cull_far_level(const CullArgs &a, int *s_bins, float t0,
                                                 Level level, int part = 0, int parts = 1) {
@@ -299,7 +302,7 @@ __device__ __forceinline__ float cull_far_level(const CullArgs &a, int *s_bins, 
   float t = t0, held = 0.f;
   for (int b = 0; b < kFarBins && t < -2.0f; ++b) {
     held += (float)s_bins[b] * exp2f(t + 1.0f);
-    if (held > 0.25f / (float)parts) break;
+    if (held > kFarShare / (float)parts) break;
     t += 1.0f;
   }
   return fminf(t, -2.0f);
