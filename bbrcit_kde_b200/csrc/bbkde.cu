@@ -391,7 +391,7 @@ struct Variant {
 };
 constexpr Variant kVariants[] = {{8, 256, 2, 0},  {4, 256, 3, 0},  {8, 128, 4, 0},
                                  {4, 128, 6, 0},  {8, 256, 2, 8},  {8, 128, 4, 8},
-                                 {8, 128, 4, 4},  {4, 128, 6, 8},  {4, 128, 6, 16},
+                                 {4, 128, 6, kPoly3Of16}, {4, 128, 6, 8},  {4, 128, 6, 16},
                                  {4, 128, 6, 32}, {8, 256, 2, 16}};
 constexpr int kNumVariants = 11;
 // Beside them k_pair_sum_split (64 queries per block), the form of small problems.
@@ -405,10 +405,11 @@ constexpr int kBlock64 = 128;
 constexpr double kAutotuneMinPairs = 2.0e10;
 constexpr double kSplitMaxPairs = 3.0e8;
 
-// 1-D Gaussians have so few FP32 operations that every 8th reference's exponentials fit
-// there (50,000 x 50,000: 542 us, every 32nd 566, none 586); 2-D ones take every 32nd
-// (593, 638 with every 8th, 617 with none). The other kernels ignore the split.
-inline int mid_variant(const Resolved &r) { return r.dim == 1 ? 7 : 9; }
+// 1-D Gaussians have so few FP32 operations that three of 16 references' exponentials
+// fit there (50,000 x 50,000: 524 us, every 8th 544, every 32nd 566, none 589); 2-D ones
+// take every 32nd (593, 638 with every 8th, 617 with none). The other kernels ignore the
+// split.
+inline int mid_variant(const Resolved &r) { return r.dim == 1 ? 6 : 9; }
 
 // Queries per block. FP64: `variant` is the queries per thread (1 or 4, f64_qpt).
 inline int queries_per_block(int variant, bool f64) {
@@ -471,7 +472,7 @@ void launch_f32(int variant, dim3 grid, cudaStream_t st, const SumArgs &a) {
     case 3: launch_shape<OP, D, 4, 128, 6>(grid, st, a); break;
     case 4: launch_shape<OP, D, 8, 256, 2, 8>(grid, st, a); break;
     case 5: launch_shape<OP, D, 8, 128, 4, 8>(grid, st, a); break;
-    case 6: launch_shape<OP, D, 8, 128, 4, 4>(grid, st, a); break;
+    case 6: launch_shape<OP, D, 4, 128, 6, kPoly3Of16>(grid, st, a); break;
     case 7: launch_shape<OP, D, 4, 128, 6, 8>(grid, st, a); break;
     case 8: launch_shape<OP, D, 4, 128, 6, 16>(grid, st, a); break;
     case 9: launch_shape<OP, D, 4, 128, 6, 32>(grid, st, a); break;

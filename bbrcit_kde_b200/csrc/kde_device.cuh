@@ -256,10 +256,14 @@ __device__ __forceinline__ void ref_pairs(const float4 *s_r0, const float4 *s_r1
 // its exponentials from exp2_poly2 (FP32 pipe) instead of MUFU.EX2, so that both
 // pipes share the work (1 in 8 balances them: the MUFU bound alone is 16 pairs
 // per clock per SM, the joint bound ~18.3).
+// kPoly3Of16: three of every 16 (the 1-D Gaussian, whose pair has 4 FP32 operations:
+// joint bound 19.7 pairs per clock per SM, 18.3 with 1 in 8 or 1 in 4).
+constexpr int kPoly3Of16 = 316;
 template <int OP, int D, int QPT, int BLOCK, int TILE, int MINB, int POLY_EVERY = 0>
 __global__ void __launch_bounds__(BLOCK, MINB) k_pair_sum_f32x2(SumArgs a) {
   static_assert(QPT % 2 == 0, "queries are processed in pairs");
-  static_assert(kChunk % (POLY_EVERY > 0 ? POLY_EVERY : 1) == 0, "poly stride divides a chunk");
+  static_assert(POLY_EVERY == kPoly3Of16 || kChunk % (POLY_EVERY > 0 ? POLY_EVERY : 1) == 0,
+                "poly stride divides a chunk");
   static_assert(TILE % kChunk == 0 && TILE % BLOCK == 0, "tile shape");
   constexpr int NP = QPT / 2;
   constexpr bool kExt = op_has_extra(OP) && D == 2;
@@ -324,13 +328,18 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pair_sum_f32x2(SumArgs a) {
           for (int j = 0; j < kChunk; ++j)
             ref_pairs<OP, D, NP, false, kExt>(s_r0, s_r1, s_r2, j0 + j, qx, qy, acc);
         } else {
+          // groups of G references, every S-th of them on the FP32 pipe
+          constexpr int G = POLY_EVERY == kPoly3Of16 ? 16 : POLY_EVERY;
+          constexpr int S = POLY_EVERY == kPoly3Of16 ? 5 : POLY_EVERY;
 #pragma unroll 1
-          for (int j = 0; j < kChunk; j += POLY_EVERY) {
+          for (int j = 0; j < kChunk; j += G) {
 #pragma unroll
-            for (int jj = 0; jj < POLY_EVERY - 1; ++jj)
-              ref_pairs<OP, D, NP, false, kExt>(s_r0, s_r1, s_r2, j0 + j + jj, qx, qy, acc);
-            ref_pairs<OP, D, NP, true, kExt>(s_r0, s_r1, s_r2, j0 + j + POLY_EVERY - 1, qx, qy,
-                                             acc);
+            for (int jj = 0; jj < G; ++jj) {
+              if (jj % S == S - 1)
+                ref_pairs<OP, D, NP, true, kExt>(s_r0, s_r1, s_r2, j0 + j + jj, qx, qy, acc);
+              else
+                ref_pairs<OP, D, NP, false, kExt>(s_r0, s_r1, s_r2, j0 + j + jj, qx, qy, acc);
+            }
           }
         }
       } else {
