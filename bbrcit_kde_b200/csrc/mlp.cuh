@@ -63,11 +63,12 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
 // z sigmoid(z) with the fast reciprocal (__fdividef, 2 ulp): for z < -88 the
 // denominator is +inf and the result is -0.
 __device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
-// silu(z) and its derivative s (1 + z (1 - s)), s = sigmoid(z), from one exponential.
+// silu(z) and silu_grad(z) from one exponential and one reciprocal, bit for bit: for every
+// z, z * __fdividef(1, d) is __fdividef(z, d).
 __device__ __forceinline__ void silu_both(float z, float &f, float &g) {
   const float s = __fdividef(1.0f, 1.0f + __expf(-z));
   f = z * s;
-  g = fmaf(f, 1.0f - s, s);
+  g = s * (1.0f + z * (1.0f - s));
 }
 // Byte offset of element (r, k) of a 128 x 128 BF16 matrix in the tensor cores' canonical
 // K-major layout without swizzle (8 x 16-byte core matrices).
@@ -609,36 +610,46 @@ struct AdamArgs {
   int step;                     // 1-based Adam step; 0 = reduce only
 };
 
-// kReduceGroups threads per parameter take the partials in turn and meet in shared
-// memory in group order: one thread per parameter read its 64 partials in one chain on
-// 132 blocks (7.5 us cold, 6.3 now; a step of 8,192 points 40 -> 25 us with both).
+// The partials are added in their order, first to last, so that a network trained from
+// the same seed and rows keeps its bits. kReduceGroups threads per parameter load them,
+// kReduceChunk at a time, and one adds the chunk from shared memory: one thread per
+// parameter waited for its 64 loads in one chain on 132 blocks.
 constexpr int kReduceGroups = 4;
 constexpr int kReduceParams = 64;   // parameters per block
+constexpr int kReduceChunk = 64;    // partials per turn
 __global__ void __launch_bounds__(kReduceGroups * kReduceParams) k_mlp_reduce(AdamArgs a) {
-  __shared__ float s_sum[kReduceGroups][kReduceParams];
+  __shared__ float s_part[kReduceChunk][kReduceParams];
+  __shared__ float s_loss[kReduceChunk];
   __shared__ float s_corr[2];
+  static_assert(kReduceParams == kReduceChunk, "one thread per parameter, one per loss partial");
   const int t = threadIdx.x % kReduceParams, g = threadIdx.x / kReduceParams;
   const int i = blockIdx.x * kReduceParams + t;
-  if (blockIdx.x == 0 && threadIdx.x < 32 && a.loss_out) {
-    float s = 0.f;
-    for (int k = threadIdx.x; k < a.nparts; k += 32) s += a.loss_part[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) *a.loss_out = s;
-  }
-  float gsum = 0.f;
-  if (i < kParams) {
-#pragma unroll 8
-    for (int k = g; k < a.nparts; k += kReduceGroups)
-      gsum += a.grad_part[(int64_t)k * kPartStride + i];
-  }
-  s_sum[g][t] = gsum;
+  const bool loss = blockIdx.x == 0 && a.loss_out != nullptr;
   if (a.step > 0 && threadIdx.x < 2)
     s_corr[threadIdx.x] = 1.f - powf(threadIdx.x == 0 ? a.beta1 : a.beta2, (float)a.step);
-  __syncthreads();
-  if (g != 0 || i >= kParams) return;
+  float gsum = 0.f, lsum = 0.f;   // of thread (g 0, t), of thread (g 1, t 0)
+  for (int k0 = 0; k0 < a.nparts; k0 += kReduceChunk) {
+    const int n = min(kReduceChunk, a.nparts - k0);
+    if (i < kParams) {
 #pragma unroll
-  for (int k = 1; k < kReduceGroups; ++k) gsum += s_sum[k][t];
+      for (int k = g; k < kReduceChunk; k += kReduceGroups)
+        if (k < n) s_part[k][t] = a.grad_part[(int64_t)(k0 + k) * kPartStride + i];
+    }
+    if (loss && g == 1 && t < n) s_loss[t] = a.loss_part[k0 + t];
+    __syncthreads();
+    if (g == 0 && i < kParams) {
+#pragma unroll 16
+      for (int k = 0; k < n; ++k) gsum += s_part[k][t];
+    }
+    if (loss && g == 1 && t == 0) {
+#pragma unroll 16
+      for (int k = 0; k < n; ++k) lsum += s_loss[k];
+    }
+    __syncthreads();
+  }
+  __syncthreads();   // s_corr, where there are no partials
+  if (loss && g == 1 && t == 0) *a.loss_out = lsum;
+  if (g != 0 || i >= kParams) return;
   if (a.grad_out) a.grad_out[i] = gsum;
   if (a.step > 0) {
     float m = a.beta1 * a.m[i] + (1.f - a.beta1) * gsum;

@@ -340,8 +340,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_infer_tc(TcArgs ta) {
 // exponential and one reciprocal, so the backward passes need neither. The 2 -> 128 and 128 -> 1 layers and every
 // per-feature sum over the points (bias gradients, dW1, dw4) run in FP32 on the
 // CUDA cores; the sums are warp butterflies (beside the running products; the first
-// layer's three go through shared memory, which is free by then) and then a fixed-order
-// sum over the four lane quarters, so a step is deterministic. Rounding points (the FP64 restatement in
+// layer's three go through shared memory, which is free by then, in the same order) and
+// then a fixed-order sum over the four lane quarters; the output and its own sums run in
+// feature and point order. So a step is deterministic, and its bits are those of one
+// thread per point. Rounding points (the FP64 restatement in
 // the tests follows them): A1 = bf16(silu(z1)), A2 = bf16(silu(z2)), dZ3 =
 // bf16(dz3), dZ2 = bf16(dz2); z2, z3, dA and dW stay FP32; bias and vector
 // gradients sum the FP32 dz. Per CTA the gradient partial is written in the
@@ -361,7 +363,8 @@ struct TcTrainSmem {
   static constexpr size_t kA2 = kA1 + kTcMatBytes;
   static constexpr size_t kDZ = kA2 + kTcMatBytes;               // dZ3, then dZ2
   static constexpr size_t kF = kDZ + kTcMatBytes;                // FP32 vectors
-  // W1, b1 b2 b3 w4, three feature sums red[3][4 quarters][kH], out[4 groups][128]
+  // W1, b1 b2 b3 w4, three feature sums red[3][4 quarters][kH], per point: the output (then
+  // x), y, dy, e^2
   static constexpr size_t kFloats = 2 * kH + 4 * kH + 3 * 4 * kH + 4 * kTcTrainPts;
   static constexpr size_t kBar = kF + kFloats * sizeof(float);   // products, weights
   static constexpr size_t kTmem = kBar + 16;
@@ -416,7 +419,7 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
   float *fp = reinterpret_cast<float *>(smem + L::kF);
   float *W1 = fp, *b1 = W1 + 2 * kH, *b2 = b1 + kH, *b3 = b2 + kH, *w4 = b3 + kH;
   float *red = w4 + kH;          // [3][4 lane quarters][kH]
-  float *outp = red + 12 * kH;   // [4 column groups][128]
+  float *outp = red + 12 * kH;   // [4][128]
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L::kBar);
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L::kTmem);
   volatile int *fail = reinterpret_cast<volatile int *>(smem + L::kFail);
@@ -533,18 +536,23 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
   if (ok) {
     float z[32], s[32];
     tc_ld32(tZ3 + mine, z);
-    float part = 0.f;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      silu_both(z[i] + b3[c0 + i], s[i], z[i]);
-      part = fmaf(w4[c0 + i], s[i], part);
+    for (int i = 0; i < 32; ++i) silu_both(z[i] + b3[c0 + i], s[i], z[i]);
+    for (int k = 0; k < kTcTrainGroups; ++k) {   // the column groups in turn: feature order
+      if (c0 == 32 * k) {
+        float out = k > 0 ? outp[row] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) out = fmaf(w4[c0 + i], s[i], out);
+        outp[row] = out;
+      }
+      __syncthreads();
     }
-    outp[(c0 >> 5) * kTcTrainPts + row] = part;
-    __syncthreads();
-    const float out = ((outp[row] + outp[kTcTrainPts + row]) + outp[2 * kTcTrainPts + row]) +
-                      outp[3 * kTcTrainPts + row];
-    e = valid ? out + b4 - target : 0.f;
+    e = valid ? outp[row] + b4 - target : 0.f;
     dy = 2.f * e * inv_b;   // dL/dy
+    if (c0 == 0) {
+      outp[2 * kTcTrainPts + row] = dy;
+      outp[3 * kTcTrainPts + row] = e * e;
+    }
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       z[i] *= dy * w4[c0 + i];
@@ -563,7 +571,10 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
           colsum(1, s);
         });
   }
-  // ---- dz2, dW3 ------------------------------------------------------------
+  // ---- dz2, dW3; db4 and the loss ------------------------------------------
+  // lane 0 of the last warp: sum of dy, lane 1: of e^2, in point order
+  const int tail_lane = tid - (kTcTrainThreads - 32);
+  float tail = 0.f;
   if (ok) {
     if (tid < kH) gp[kOffB3 + tid] = quarters(0, tid);
     else if (tid < 2 * kH) gp[kOffW4 + tid - kH] = quarters(1, tid - kH);
@@ -584,9 +595,14 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
           colsum(2, d);
           tc_ld32(tW + mine, g);   // row `row` of dW3
           store32(gp + kOffW3 + row * kH + c0, g);
+          if (tail_lane == 0 || tail_lane == 1) {
+            const float *src = outp + (2 + tail_lane) * kTcTrainPts;
+#pragma unroll 16
+            for (int i = 0; i < kTcTrainPts; ++i) tail += src[i];
+          }
         });
   }
-  // ---- dz1 and the first layer; dW2; db4 and the loss ----------------------
+  // ---- dz1 and the first layer; dW2 ----------------------------------------
   if (ok) {
     if (tid < kH) gp[kOffB2 + tid] = quarters(2, tid);
     float d[32], g[32];
@@ -604,32 +620,30 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
     tc_ld32(tZ2 + mine, g);   // row `row` of dW2
     store32(gp + kOffW2 + row * kH + c0, g);
     __syncthreads();
-    // thread (feature n, point quarter q): db1, dW1[n][0], dW1[n][1] over 32 points
+    // thread (feature n, point quarter q): db1, dW1[n][0], dW1[n][1] over 32 points, as
+    // warp_transpose_sum adds them (points 16 apart first, then 8, 4, 2 and 1)
     const int n = tid % kH, q = tid / kH;
-    float s0 = 0.f, sx = 0.f, sy = 0.f;
-#pragma unroll 8
-    for (int i = 32 * q; i < 32 * q + 32; ++i) {
-      const float v = dz[i * L::kDzLd + n];
-      s0 += v;
-      sx = fmaf(v, outp[i], sx);
-      sy = fmaf(v, outp[kTcTrainPts + i], sy);
-    }
-    red[q * kH + n] = s0;
-    red[(4 + q) * kH + n] = sx;
-    red[(8 + q) * kH + n] = sy;
-  }
-  float *psum = outp + 2 * kTcTrainPts;
-  if (c0 == 0) {   // the first column group's four warps: sums over their points
-    float sd = dy, se = e * e;
+    float s0[16], sx[16], sy[16];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sd += __shfl_xor_sync(0xffffffffu, sd, o);
-      se += __shfl_xor_sync(0xffffffffu, se, o);
+    for (int i = 0; i < 16; ++i) {
+      const int j = 32 * q + i, k = j + 16;
+      const float v = dz[j * L::kDzLd + n], w = dz[k * L::kDzLd + n];
+      s0[i] = v + w;
+      sx[i] = __fadd_rn(__fmul_rn(v, outp[j]), __fmul_rn(w, outp[k]));
+      sy[i] = __fadd_rn(__fmul_rn(v, outp[kTcTrainPts + j]), __fmul_rn(w, outp[kTcTrainPts + k]));
     }
-    if (lane == 0) {
-      psum[quarter] = sd;
-      psum[4 + quarter] = se;
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) {
+#pragma unroll
+      for (int i = 0; i < o; ++i) {
+        s0[i] += s0[i + o];
+        sx[i] += sx[i + o];
+        sy[i] += sy[i + o];
+      }
     }
+    red[q * kH + n] = s0[0];
+    red[(4 + q) * kH + n] = sx[0];
+    red[(8 + q) * kH + n] = sy[0];
   }
   tc_fence_before();
   __syncthreads();
@@ -638,11 +652,9 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
     const int k = tid / kH, n = tid % kH;
     gp[k == 0 ? kOffB1 + n : kOffW1 + 2 * n + (k - 1)] = quarters(k, n);
   }
-  if (tid == 0) {
-    gp[kOffB4] = ((psum[0] + psum[1]) + psum[2]) + psum[3];
-    a.loss_part[blockIdx.x] = (((psum[4] + psum[5]) + psum[6]) + psum[7]) * inv_b;
-    if (!ok) atomicExch(ta.status, 1);
-  }
+  if (tail_lane == 0) gp[kOffB4] = tail;
+  if (tail_lane == 1) a.loss_part[blockIdx.x] = tail * inv_b;
+  if (tid == 0 && !ok) atomicExch(ta.status, 1);
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(kTcTrainCols));
