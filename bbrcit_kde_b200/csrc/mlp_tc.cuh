@@ -378,7 +378,8 @@ struct TcTrainSmem {
 
 struct TcTrainArgs {
   TrainArgs t;
-  int *status;   // set to 1 if a wait expired
+  int *status;          // set to 1 if a wait expired
+  long long limit;      // polls of a wait before it gives up
 };
 
 // Sum over the 32 lanes of a warp, per index: after the call lane j holds
@@ -488,7 +489,7 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
       tc_commit(mbar);
     }
     meanwhile();
-    if (!tc_wait(mbar, phase)) fail[0] = 1;
+    if (!tc_wait(mbar, phase, ta.limit)) fail[0] = 1;
     phase ^= 1u;
     tc_fence_after();
     __syncthreads();
@@ -519,8 +520,8 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
     for (int j = 0; j < 32; j += 8) tc_store8<false>(A1, nullptr, row, c0 + j, v + j);
     tc_st32(tG1 + mine, g);
   }
-  if (!tc_wait(smem_u32(bar + 1), 0)) fail[0] = 1;   // the weights are in shared memory
-  ok = run([&] { tc_gemm128(tZ2, sA1, false, sW2, false, false); }, nothing);
+  ok = __syncthreads_and(tc_wait(smem_u32(bar + 1), 0, ta.limit));   // the weights are here
+  if (ok) ok = run([&] { tc_gemm128(tZ2, sA1, false, sW2, false, false); }, nothing);
   if (ok) {
     float v[32], g[32];
     tc_ld32(tZ2 + mine, v);
@@ -654,7 +655,14 @@ __global__ void __launch_bounds__(kTcTrainThreads, 1) k_mlp_train_tc(TcTrainArgs
   }
   if (tail_lane == 0) gp[kOffB4] = tail;
   if (tail_lane == 1) a.loss_part[blockIdx.x] = tail * inv_b;
-  if (tid == 0 && !ok) atomicExch(ta.status, 1);
+  if (tid == 0 && !ok) {
+    atomicExch(ta.status, 1);
+    // Nothing of this CTA's may be in flight when its shared memory and TMEM go: wait
+    // (again bounded) for the weights and for the last products (at once if none are).
+    tc_wait(smem_u32(bar + 1), 0);
+    tc_wait(mbar, phase ^ 1u);
+  }
+  if (!ok) __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(kTcTrainCols));

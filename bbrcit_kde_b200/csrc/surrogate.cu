@@ -185,6 +185,7 @@ unsigned launch_train(bbkde_surrogate *s, const TrainArgs &targs) {
     TcTrainArgs ta;
     ta.t = targs;
     ta.status = s->status;
+    ta.limit = bbkde::kTcWaitLimit;
     k_mlp_train_tc<<<blocks, kTcTrainThreads, TcTrainSmem::kBytes, s->stream>>>(ta);
   } else {
     k_mlp_train<<<blocks, kTrainWarps * 32, kTrainSmem, s->stream>>>(targs);

@@ -21,8 +21,9 @@ __device__ __forceinline__ void tc_commit(uint32_t mbar) {
 }
 
 // Bounded wait for the mbarrier phase `parity` to complete; false on expiry.
-__device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity) {
-  for (long long i = 0; i < kTcWaitLimit; ++i) {
+__device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity,
+                                        long long limit = kTcWaitLimit) {
+  for (long long i = 0; i < limit; ++i) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
