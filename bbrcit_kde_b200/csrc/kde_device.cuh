@@ -162,22 +162,29 @@ __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 // f = x - n in [-1/2, 1/2] exactly), 2^f by a degree-5 polynomial (coefficients
 // fitted for minimum relative error on [-1/2, 1/2] by Lawson's iteratively
 // reweighted least squares: 7.5e-8 in exact arithmetic, 2.1e-7 evaluated with FP32
-// FMAs), 2^n added into the exponent field (the 0x4B400000 of t shifts out of a
-// 32-bit word, leaving n << 23). x is clamped at -125 so the result is a normal
-// number: a pair that MUFU.EX2 flushes to zero contributes at most 2^-125 * mass.
+// FMAs), times 2^n, whose bits are t << 23 (the shift carries the exponent bias 127; its
+// 0x4B400000 leaves the 32-bit word). As ex2.approx.ftz does, it gives 0 for x < -126 --
+// 2^-127 is 0 here and the product flushes -- and NaN for NaN, so that a sum does not
+// depend on which of its exponentials run here: with every far pair at 2^-125 instead, an
+// isolated point's leave-one-out density was 1e-38 and its likelihood finite.
 __device__ __forceinline__ float2 exp2_poly2(float2 x) {
-  x.x = fmaxf(x.x, -125.0f);
-  x.y = fmaxf(x.y, -125.0f);
-  const float2 t = __fadd2_rn(x, f2(12582912.0f));
-  const float2 n = __fadd2_rn(t, f2(-12582912.0f));
+  asm("max.NaN.f32 %0, %0, 0fC2FE0000;" : "+f"(x.x));   // -127
+  asm("max.NaN.f32 %0, %0, 0fC2FE0000;" : "+f"(x.y));
+  const float2 t = __fadd2_rn(x, f2(12583039.0f));   // 1.5 * 2^23 + 127
+  const float2 n = __fadd2_rn(t, f2(-12583039.0f));
   const float2 f = __ffma2_rn(n, f2(-1.0f), x);
   float2 p = __ffma2_rn(f2(1.327644451521337e-3f), f, f2(9.67553723603487e-3f));
   p = __ffma2_rn(p, f, f2(5.550713464617729e-2f));
   p = __ffma2_rn(p, f, f2(2.4022120237350464e-1f));
   p = __ffma2_rn(p, f, f2(6.931469440460205e-1f));
   p = __ffma2_rn(p, f, f2(1.0000001192092896f));
-  return make_float2(__uint_as_float(__float_as_uint(p.x) + (__float_as_uint(t.x) << 23)),
-                     __uint_as_float(__float_as_uint(p.y) + (__float_as_uint(t.y) << 23)));
+  float2 u;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "mul.rn.ftz.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(u.x), "=f"(u.y)
+      : "f"(p.x), "f"(p.y), "f"(__uint_as_float(__float_as_uint(t.x) << 23)),
+        "f"(__uint_as_float(__float_as_uint(t.y) << 23)));
+  return u;
 }
 
 // max(1 + s d2, 0) for two lanes: two saturating multiply-adds (1 + s d2 <= 1) instead
