@@ -63,11 +63,14 @@ __device__ __forceinline__ float fma_sat(float a, float b, float c) {
 // banks, so a warp's lookups never conflict.
 // The bias keeps every value that the library's exp returns (denormals included) in the
 // normal range, without a slow path; the sum is scaled back once per query. x is
-// clamped at kExpClamp, where the value (2^-1276) is lost in that scaling unless the
-// masses sum to 2^200; the clamp works on the high word and lets a NaN of either sign
-// pass (plus 0x80000 a negative quiet NaN wraps to a small number).
-constexpr int kExpBias = 256;
-constexpr unsigned kExpClamp = 0xC08BA000u;   // high word of -884
+// clamped at kExpClamp, where k = -16 (1023 + kExpBias) takes the exponent field of entry
+// 0, 1.0, to zero: the value is 0, whatever the mass (the binade above it, 2^-1534, is a
+// denormal of too few bits). The clamp works on the high word and lets a NaN of either
+// sign pass (plus 0x80000 a negative quiet NaN wraps to a small number). A biased sum that
+// overflows (2^512, before the scaling) is taken again without the bias
+// (gauss_sum_unbiased).
+constexpr int kExpBias = 512;
+constexpr unsigned kExpClamp = 0xC0909FECu;   // high word of -1063.98: k = -24560
 __device__ constexpr double kExpTab[16] = {
     1.0, 1.0442737824274138, 1.0905077326652577, 1.1387886347566916,
     1.189207115002721, 1.241857812073484, 1.2968395546510096, 1.3542555469368927,
@@ -518,6 +521,25 @@ __global__ void __launch_bounds__(32 * kSplitWarps, 4) k_pair_sum_split(SumArgs 
   }
 }
 
+// Gaussian sum of one query over [lo, hi) with the library's exp, for sums that overflow
+// under exp_neg's bias (masses beyond 2^512, infinities) or are NaN; -1: no self pair.
+template <int OP, int D>
+__device__ __noinline__ double gauss_sum_unbiased(const double4 *refs, const double *ext,
+                                                  int64_t lo, int64_t hi, double qx, double qy,
+                                                  int64_t self) {
+  double total = 0.0;
+  for (int64_t r = lo; r < hi; ++r) {
+    const double4 v = refs[r];
+    const double dx = qx - v.x, dy = D == 2 ? qy - v.y : 0.0;
+    const double m = D == 2 ? v.z : v.y, s = D == 2 ? v.w : v.z;
+    const double x = D == 1 ? dx * dx * s
+                     : OP == OP_GAUSS_ISO ? (dx * dx + dy * dy) * s
+                                          : dx * dx * s + dy * dy * ext[r];
+    total += (r == self ? 0.0 : m) * exp(x);
+  }
+  return total;
+}
+
 // ---------------------------------------------------------------------------
 // FP64 pair sum (reference arithmetic). Thread t of block b owns the queries
 // (b QPT + k) BLOCK + t. The FP64 pipe (64 lanes per clock per SM) is the bound: 18
@@ -590,8 +612,12 @@ __global__ void __launch_bounds__(BLOCK) k_pair_sum_f64(SumArgs a) {
 #pragma unroll
   for (int k = 0; k < QPT; ++k) {
     const int64_t lq = lq0 + k * BLOCK + tid;
-    const double v = kGauss ? ldexp(total[k], -kExpBias) : total[k];
-    if (lq < a.q_count) a.out[(int64_t)blockIdx.y * a.q_count + lq] = a.scale * v;
+    if (lq >= a.q_count) continue;
+    double v = kGauss ? ldexp(total[k], -kExpBias) : total[k];
+    if (kGauss && !isfinite(v))
+      v = gauss_sum_unbiased<OP, D>(refs, ext, r_lo, r_hi, qx[k], qy[k],
+                                    a.exclude_self ? a.q_begin + lq : -1);
+    a.out[(int64_t)blockIdx.y * a.q_count + lq] = a.scale * v;
   }
 }
 
