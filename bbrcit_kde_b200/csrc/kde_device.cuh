@@ -39,7 +39,7 @@ __device__ __forceinline__ float ex2_approx(float x) {
 
 // The Epanechnikov convolution (2 - u)^3 (u^2 + 6u + 4) / 32 on u = |d| / (h a) < 2
 // (KernelTraits.h:338-342) in v = u / 2: (1 - v)^3 (v^2 + 3v + 1), the same value with
-// every power of two folded into the record's scale 1 / (2 h a).
+// every power of two folded into the record's scale 1 / |2 h a|.
 __device__ __forceinline__ double epan_conv_d(double d, double inv) {
   const double v = fabs(d) * inv;
   const double c = 1.0 - v > 0.0 ? 1.0 - v : 0.0;
@@ -636,11 +636,11 @@ struct PackArgs {
 //   GAUSS_*:  s = c1 / (h1 a)^2 (c1 = -log2(e)/2, or -log2(e)/4 for the
 //             Gaussian convolution), e = c2 / (h2 a)^2
 //   EPAN_ISO / EPAN_PROD: s = -1 / (h1 a)^2, e = -1 / (h2 a)^2
-//   EPAN_CONV: s = 1 / (2 h1 a), e = 1 / (2 h2 a)
+//   EPAN_CONV: s = 1 / |2 h1 a|, e = 1 / |2 h2 a| (the kernel is one of |u|)
 __device__ __forceinline__ void pack_scales(const PackArgs &p, double a, double &s, double &e) {
   if (p.op == OP_EPAN_CONV) {
-    s = 0.5 / (p.h1 * a);
-    e = 0.5 / (p.h2 * a);
+    s = 0.5 / fabs(p.h1 * a);
+    e = 0.5 / fabs(p.h2 * a);
   } else {
     s = p.c1 / (p.h1 * p.h1 * a * a);
     e = p.c2 / (p.h2 * p.h2 * a * a);

@@ -78,3 +78,19 @@ def test_fp64_gaussian_far_values(ctx):
     # a thousand far points with large masses add up to nothing
     ctx.upload(bk.REFERENCE, np.full((1000, 1), 100.0), mass=np.full(1000, 1e6))
     assert ctx.eval_range(desc, 0, 999, 4, 4, normalized=False, precision=bk.FP64)[0] == 0.0
+
+
+@pytest.mark.parametrize("kind,dim,h", KINDS)
+@pytest.mark.parametrize("precision", [bk.FP32C, bk.FP64])
+def test_every_kernel_is_one_of_the_bandwidths_size(ctx, oracle, kind, dim, h, precision):
+    """Local bandwidths of either sign: a kernel value depends on |h a| only (same bounds as
+    test_edges)."""
+    refs, q, mass, abw = _problem(3, 600, 130, dim)
+    abw[::3] *= -1.0
+    ctx.upload(bk.REFERENCE, refs, mass=mass, abw=abw, weight=mass)
+    ctx.upload(bk.QUERY, q)
+    want = oracle.direct(kind, dim, h, refs, mass, q, abw=abw)
+    peak = 1.0 / (h[0] * (h[1] if dim == 2 else 1.0)) * mass.max()
+    got = ctx.eval_all(bk.kernel_desc(kind, dim, h), precision=precision)
+    tol = 1e-6 if precision == bk.FP32C else 1e-13
+    assert np.all(np.abs(got - want) <= tol * want + tol * peak)
