@@ -172,10 +172,11 @@ __global__ void __launch_bounds__(T *T / 8, T == 32 ? 4 : 16)
   // Column swizzle of factor row p (see the layout note).
   auto swz = [](int p) { return T == 16 ? (p & 1) << 3 : 0; };
 
+  const CullGroups groups = {nullptr, a.n_groups};
   // Scan 1 (Gaussians): largest tile bound over the block's box.
   float e_max = -INFINITY;
   if (kGauss)
-    e_max = cull_max<BLOCK>(a, s_red, [&](const RefTile &rt) {
+    e_max = cull_max<BLOCK>(a, groups, s_red, [&](const RefTile &rt) {
       return rt.lm + tile_peak<OP, 2>(rt, qx0, qx1, qy0, qy1);
     });
   const float t_a = e_max - a.cut;
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(T *T / 8, T == 32 ? 4 : 16)
 
   auto pass = [&](int phase) {
     summed += cull_pass<BLOCK>(
-        a, s_list, s_glist, s_wc,
+        a, groups, s_list, s_glist, s_wc,
         [&](const RefTile &g, bool own) { return needed(g, phase, true, own); },
         [&](const RefTile &rt) { return needed(rt, phase, false, true); }, sum_list, part, S);
   };
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(T *T / 8, T == 32 ? 4 : 16)
     __syncthreads();
     t0 = -log2f((float)a.n_tiles) - 2.0f;
     tn = cull_far_level<BLOCK>(
-        a, s_bins, t0,
+        a, groups, s_bins, t0,
         [&](const RefTile &rt, bool group) {
           const float pb = tile_peak<OP, 2>(rt, qx0, qx1, qy0, qy1);
           if (pb < kFlushExp || (!group && rt.lm + pb >= t_a)) return -INFINITY;

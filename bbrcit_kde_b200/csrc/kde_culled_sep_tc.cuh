@@ -250,10 +250,11 @@ __global__ void __launch_bounds__(NT, 4) k_pair_sum_culled_sep_tc(CullArgs a) {
   }
   const int foff = half ? 0 : STG;
 
+  const CullGroups groups = {nullptr, a.n_groups};
   // Scan 1 (Gaussians): largest tile bound over the block's box.
   float e_max = -INFINITY;
   if (kGauss)
-    e_max = cull_max<BLOCK>(a, s_red, [&](const RefTile &rt) {
+    e_max = cull_max<BLOCK>(a, groups, s_red, [&](const RefTile &rt) {
       return rt.lm + tile_peak<OP, 2>(rt, qx0, qx1, qy0, qy1);
     });
   const float t_a = e_max - a.cut;
@@ -436,7 +437,8 @@ __global__ void __launch_bounds__(NT, 4) k_pair_sum_culled_sep_tc(CullArgs a) {
 
   auto pass = [&](int phase) {
     summed += cull_pass<BLOCK>(
-        a, s_list, s_glist, s_wc, [&](const RefTile &g, bool) { return needed(g, phase, true); },
+        a, groups, s_list, s_glist, s_wc,
+        [&](const RefTile &g, bool) { return needed(g, phase, true); },
         [&](const RefTile &rt) { return needed(rt, phase, false); }, sum_list);
     drain();
   };
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(NT, 4) k_pair_sum_culled_sep_tc(CullArgs a) {
     __syncthreads();
     t0 = -log2f((float)a.n_tiles) - 2.0f;
     tn = cull_far_level<BLOCK>(
-        a, s_bins, t0,
+        a, groups, s_bins, t0,
         [&](const RefTile &rt, bool group) {
           const float pb = tile_peak<OP, 2>(rt, qx0, qx1, qy0, qy1);
           if (pb < kFlushExp || (!group && rt.lm + pb >= t_a)) return -INFINITY;

@@ -80,3 +80,28 @@ def test_not_a_number(ctx):
     got, _ = ctx.eval_tol(desc, 1e-6, 0.0)
     assert np.isnan(got[:130]).all()
     np.testing.assert_allclose(got[130:], want[130:], rtol=2e-6)
+
+
+@pytest.mark.parametrize("kind,dim", [(W.GAUSS, 1), (W.GAUSS_PROD2D, 2), (W.EPAN, 1)])
+@pytest.mark.parametrize("n", [262_144, 262_145, 300_007, 1_100_000, 8_500_000])
+@pytest.mark.parametrize("h", [1e-4, 0.02, 5.0])
+def test_many_groups(ctx, kind, dim, n, h):
+    """More tile groups (1,024 references each) than a block has threads: its scans go over
+    the groups in reach -- none, some, more than the list holds (1,074 groups at h = 5) --
+    and past 8,192 groups the list is made in two turns. Queries far from all references
+    share blocks with others. Bounds as in test_edges; at h = 1e-4 an FP32 coordinate
+    (step 2^-22 of a few) is off by 2.4e-3 of a bandwidth in both, the same."""
+    refs = W.f32(W.SplitMix64(n).uniform(n * dim, -3.0, 3.0).reshape(n, dim))
+    q = W.f32(W.SplitMix64(8).uniform(100 * dim, -3.0, 3.0).reshape(100, dim))
+    q[::7] = refs[:15]
+    q[50:53] = 40.0
+    ctx.upload(bk.REFERENCE, refs, mass=np.full(n, 1.0 / n))
+    ctx.upload(bk.QUERY, q)
+    desc = bk.kernel_desc(kind, dim, h)
+    want = ctx.eval_all(desc, precision=bk.FP64)
+    got, st = ctx.eval_tol(desc, 1e-6, 0.0)
+    peak = 1.0 / (n * h ** dim)
+    # an FP32 exponent of -e is off by e 2^-23 or two of it; below e = 20 that is 1e-5 of one
+    # pair's value at most, and sums of many pairs are dominated by near ones
+    assert np.all(np.abs(got - want) <= 2e-6 * want + 1e-5 * peak)
+    assert st.max_bound_ratio <= 1e-6
