@@ -399,7 +399,7 @@ constexpr int kSplitVariant = kNumVariants;
 constexpr int kTile = 256;
 constexpr int kBlock64 = 128;
 // Problems below this many pairs skip autotuning: up to kSplitMaxPairs they run
-// k_pair_sum_split, above it a fixed shape (mid_variant). Kernel us, split / fixed:
+// k_pair_sum_split, above it a fixed shape (untuned_variant). Kernel us, split / fixed:
 // 500 x 400 queries 8 / 13, 2,000 x 2,000 9 / 13, 10,000 x 10,000 36 / 36, 50,000 x
 // 50,000 630 / 595 (2-D Gaussian; 28, 30, 48, 633 in the 2,048-query blocks of shape 0).
 constexpr double kAutotuneMinPairs = 2.0e10;
@@ -409,7 +409,9 @@ constexpr double kSplitMaxPairs = 3.0e8;
 // fit there (50,000 x 50,000: 524 us, every 8th 544, every 32nd 566, none 589); 2-D ones
 // take every 32nd (593, 638 with every 8th, 617 with none). The other kernels ignore the
 // split.
-inline int mid_variant(const Resolved &r) { return r.dim == 1 ? 6 : 9; }
+inline int untuned_variant(const Resolved &r, double pairs) {
+  return pairs <= kSplitMaxPairs ? kSplitVariant : r.dim == 1 ? 6 : 9;
+}
 
 // Queries per block. FP64: `variant` is the queries per thread (1 or 4, f64_qpt).
 inline int queries_per_block(int variant, bool f64) {
@@ -568,7 +570,7 @@ int choose_variant(bbkde_ctx *c, const Resolved &r, const void *qx, const void *
   if (c->forced_variant >= 0) { *variant = c->forced_variant; return BBKDE_OK; }
   const double pairs = (double)(r_j - r_i + 1) * (double)(q_j - q_i + 1);
   if (pairs < kAutotuneMinPairs) {
-    *variant = pairs <= kSplitMaxPairs ? kSplitVariant : mid_variant(r);
+    *variant = untuned_variant(r, pairs);
     return BBKDE_OK;
   }
   auto key = std::make_tuple(r.op, r.dim, exclude_self ? 1 : 0, ilog2(r_j - r_i + 1),
@@ -2857,11 +2859,15 @@ extern "C" int bbkde_eval_noalloc(const bbkde_kernel_desc *kernel, int64_t n_ref
     cudaGetLastError();
     return BBKDE_CUDA_ERROR;
   }
-  Plan pl = plan_launch(sm_count, n_ref, n_query, kSplitVariant, false);
+  // The context path's shapes without its tuning, which would wait for the stream (100,000
+  // x 100,000 2-D Gaussian: 2.53 ms in the split form, 2.30 in shape 9).
+  const int variant = untuned_variant(r, (double)n_ref * (double)n_query);
+  const int64_t step = segment_step(variant, false);
+  Plan pl = plan_launch(sm_count, n_ref, n_query, variant, false);
   const int64_t fit = (int64_t)((kNoAllocScratchBytes - off_part) / per_seg);
   if (pl.nseg > fit) {
     pl.seg_len = (n_ref + fit - 1) / fit;
-    pl.seg_len = (pl.seg_len + kSplitStep - 1) / kSplitStep * kSplitStep;
+    pl.seg_len = (pl.seg_len + step - 1) / step * step;
     pl.nseg = (n_ref + pl.seg_len - 1) / pl.seg_len;
   }
 
@@ -2880,8 +2886,8 @@ extern "C" int bbkde_eval_noalloc(const bbkde_kernel_desc *kernel, int64_t n_ref
   a.out = partial;   // every (segment, query) entry is written: nothing to clear
   a.status = nullptr;
   const dim3 grid(pl.gx, (unsigned)pl.nseg);
-  if (dim == 2) dispatch_op<2>(r.op, false, kSplitVariant, grid, st, a);
-  else dispatch_op<1>(r.op, false, kSplitVariant, grid, st, a);
+  if (dim == 2) dispatch_op<2>(r.op, false, variant, grid, st, a);
+  else dispatch_op<1>(r.op, false, variant, grid, st, a);
   launch_combine(st, partial, pl.nseg, n_query, normalized ? r.norm : 1.0, out, EPI_NONE,
                  nullptr, nullptr);
   e = cudaGetLastError();
