@@ -2591,6 +2591,7 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
   // 7. Exact fallback on the flagged tiles.
   CUDA_TRY(c, cudaGetLastError());
   int nsel = 0;
+  bool quads = false;
   unsigned long long counts[3] = {0, 0, 0};
   CUDA_TRY(c, cudaMemcpyAsync(counts, c->gr_counts.p, sizeof(counts), cudaMemcpyDeviceToHost,
                               c->stream));
@@ -2602,6 +2603,7 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
     nsel = 0;
   } else if (T == 16 && !cfg->pair_form && op_separable(r.op) && nsel >= kGridWideMin) {
     // 2 x 2 blocks of (nearly) all flagged tiles leave the list of single tiles
+    quads = true;
     const GridDesc g32 = make_grid(g.nx, g.ny, g.x0, g.dx, g.y0, g.dy, 32);
     const int64_t nquads = (int64_t)g32.ntx * g32.nty;
     TRY(tile_order(c, g32, c->gr_quad_order));
@@ -2626,15 +2628,24 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
   TRY(grid_exact(c, r, g, c->gr_list.as<int>(), nsel, cfg->cull_rel, full, out, &st.pairs,
                  &st.max_bound_ratio, cfg->pair_form != 0, cfg->tensor_cores));
   CUDA_TRY(c, cudaEventRecord(c->ev3, c->stream));
-  // Points in the flagged tiles (edge tiles may be partial).
+  // Tiles summed exactly -- the flagged ones, and the fourth of a block summed whole --
+  // and their points (edge tiles may be partial).
   std::vector<int> flags((size_t)ntiles);
   CUDA_TRY(c, cudaMemcpyAsync(flags.data(), c->gr_flag.p, (size_t)ntiles * sizeof(int),
                               cudaMemcpyDeviceToHost, c->stream));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-  int64_t fb_points = 0;
+  int64_t fb_points = 0, fb_tiles = 0;
   for (int64_t t = 0; t < ntiles; ++t) {
-    if (!flags[(size_t)t]) continue;
     const int64_t tx = t % g.ntx, ty = t / g.ntx;
+    if (!flags[(size_t)t]) {
+      int block = 0;
+      if (quads)
+        for (int64_t y = ty & ~1; y < std::min<int64_t>((ty & ~1) + 2, g.nty); ++y)
+          for (int64_t x = tx & ~1; x < std::min<int64_t>((tx & ~1) + 2, g.ntx); ++x)
+            block += flags[(size_t)(y * g.ntx + x)] != 0;
+      if (!quads || block < kGridQuadMin) continue;
+    }
+    ++fb_tiles;
     fb_points += std::min<int64_t>(T, g.nx - tx * T) * std::min<int64_t>(T, g.ny - ty * T);
   }
   float ms = 0.f;
@@ -2648,7 +2659,7 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
   CUDA_TRY(c, cudaEventElapsedTime(&ms, c->ev2, c->ev3));
   st.ms_fallback = ms;
   st.tiles_low = (int64_t)counts[0];
-  st.tiles_flagged = (int64_t)counts[1];
+  st.tiles_flagged = fb_tiles;
   st.tiles_surrogate = ntiles - st.tiles_flagged;
   st.exact_points += fb_points;
   unsigned eb = (unsigned)counts[2];
