@@ -1198,9 +1198,10 @@ int cv_batch_loop(bbkde_ctx *c, int kind, int n_sets, const bbkde_dataset *sets,
         const int64_t o = ((int64_t)sidx * n_hx + a) * n_hy + b;
         TRY(bbkde_likelihood_cv(c, &k, precision, lik + o));
         ms += c->last_ms;
+        pairs += c->last_pairs;
         TRY(bbkde_lsq_conv_cv(c, &k, precision, lsq + o));
         ms += c->last_ms;
-        pairs += 3.0 * (double)d.n * (double)d.n;
+        pairs += c->last_pairs;
       }
   }
   c->last_ms = ms;

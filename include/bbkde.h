@@ -226,7 +226,8 @@ typedef struct {
  *     bandwidth (moment binning, FP64), captured in a CUDA graph and replayed
  *     for repeated calls of the same shape.
  *   BBKDE_GAUSSIAN_PRODUCT_2D: exact per-bandwidth loop over the pair sum.
- * hx and hy must be strictly increasing, positive, at most 64 values each.
+ * hx and hy must be strictly increasing, positive, at most 64 values each; a dataset has
+ * at least 2 points and at most 2^31 - 1 (OUT_OF_RANGE).
  * Exact-duplicate points are not merged (the reference's Kd-tree merges them). */
 BBKDE_API int bbkde_cv_batch(bbkde_ctx *ctx, int kind, int n_sets, const bbkde_dataset *sets,
                              int n_hx, const double *hx, int n_hy, const double *hy,

@@ -145,3 +145,10 @@ def test_cv_batch_small_items(ctx, sizes, nx, ny, weighted):
                                         hy[pick[1]])
     _close(lik[:, pick[0]][:, :, pick[1]], want_lik, 1e-9)
     _close(lsq[:, pick[0]][:, :, pick[1]], want_lsq, 1e-9)
+
+
+def test_gaussian_loop_counts_the_pairs_it_summed(ctx):
+    """Both scores of the product Gaussian take one pass over the pairs each."""
+    xy = W.config3_datasets(n_sets=1, sizes=[700])[0]
+    ctx.cv_batch(bk.GAUSSIAN_PRODUCT_2D, [(xy, None), (xy[:300], None)], [0.1, 0.2], [0.3])
+    assert ctx.last_launch_stats()[1] == 2 * (2 * 700.0 ** 2 + 2 * 300.0 ** 2)
