@@ -259,12 +259,12 @@ def test_grid_exact_matches_direct(ctx):
 
 @pytest.mark.parametrize("tiles_per_axis", [8, 12, 16, 24, 32])
 def test_grid_exact_split_tiles(ctx, tiles_per_axis):
-    """Short tile-16 lists are summed by clusters of 8, 4 or 2 blocks per tile (each
-    part sums every S-th batch of reference groups; the parts share the thresholds
-    of the total near-field sum through distributed shared memory and part 0 adds
-    them in rank order). On 148 SMs these tile counts (64, 144, 256, 576, 1024) run
-    8, 8, 4, 2 and 1 parts; every one matches the direct sum, keeps the bound, and
-    repeats bitwise."""
+    """Exact grids of 16-point tiles, summed two by two as 32-point ones: lists of 16 to
+    256 of them, in clusters of 8 or (256) 4 blocks per tile (each part sums every S-th
+    reference tile; the parts share the thresholds of the total near-field sum through
+    distributed shared memory and part 0 adds them in rank order). Every one matches the
+    direct sum, keeps the bound, and repeats bitwise (test_grid_parts_gpu.py has the other
+    part counts)."""
     desc = _setup_adaptive(ctx)
     m = 16 * tiles_per_axis
     grid = (m, m, -4.0, 4.0, -4.0, 4.0)
@@ -277,9 +277,9 @@ def test_grid_exact_split_tiles(ctx, tiles_per_axis):
     assert np.array_equal(got, again)
 
 
-@pytest.mark.parametrize("grid,tile", [((100, 70, -3.0, 2.5, -2.0, 3.0), 16),   # 35 ragged tiles: 8 parts
-                                       ((700, 690, -4.0, 4.0, -4.0, 4.0), 16),   # 1,936 tiles: cost order
-                                       ((1000, 990, -4.0, 4.0, -4.0, 4.0), 32)])  # 1,024 tiles: cost order
+@pytest.mark.parametrize("grid,tile", [((100, 70, -3.0, 2.5, -2.0, 3.0), 16),   # 12 ragged 32-point tiles: 8 parts
+                                       ((700, 690, -4.0, 4.0, -4.0, 4.0), 16),   # 484: 2 parts
+                                       ((1000, 990, -4.0, 4.0, -4.0, 4.0), 32)])  # 1,024: cost order
 def test_grid_exact_ragged_split_and_ordered(ctx, grid, tile):
     """Ragged grids (edges that cut tiles) through the two launch forms that long
     and short tile lists take: clusters of parts per tile (short lists) and the

@@ -15,12 +15,6 @@ KERNELS = {"gauss2d": (bk.GAUSSIAN, 2), "gaussprod": (bk.GAUSSIAN_PRODUCT_2D, 2)
 FAR = 200.0
 
 
-@pytest.fixture(scope="module")
-def ctx():
-    with bk.Context(0) as c:
-        yield c
-
-
 def _points(n, dim):
     return W.SplitMix64(77).normal(n * dim).astype(np.float32).astype(np.float64).reshape(n, dim)
 

@@ -11,12 +11,6 @@ from bbrcit_kde_b200 import workloads as W
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(scope="module")
-def ctx():
-    with bk.Context(0) as c:
-        yield c
-
-
 @pytest.mark.parametrize("kind,dim,h", [(W.GAUSS, 2, (0.3, 0.3)), (W.GAUSS_PROD2D, 2, (0.2, 0.5)),
                                         (W.GAUSS, 1, (0.3, 0.3))])
 @pytest.mark.parametrize("n,m", [(300, 200), (3000, 40_000)])   # one and four queries a thread

@@ -80,7 +80,8 @@ def test_tensor_core_tiles_match_direct_and_fp32_pipe(ctx, kind, h):
 
 def test_tensor_core_tiles_long_list_and_automatic_choice(ctx):
     """The automatic setting takes the tensor cores for every culled tile-32 sum at
-    tolerances of 1e-5 and above: 128-thread blocks for lists of at least 16
+    tolerances of 1e-5 and above whose list is at least one wave of blocks
+    (test_grid_parts_gpu.py has shorter ones): 128-thread blocks for lists of at least 16
     waves (a ragged 3200 x 3100 grid, 9,700 tiles, in the most-expensive-first
     launch order), 256-thread blocks for shorter ones (a 1,024-tile list). Both
     are bitwise the forced result and match the direct sum and the FP32-pipe
