@@ -2361,6 +2361,23 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
     if (stats) *stats = st;
     return BBKDE_OK;
   }
+  if (mode == BBKDE_GRID_EXACT) {   // every tile; no prediction, flags or lists
+    CUDA_TRY(c, cudaEventRecord(c->ev0, c->stream));
+    TRY(grid_exact_all(c, r, g, c->gr_order, cfg->cull_rel, full, out, &st.pairs,
+                       &st.max_bound_ratio, cfg->pair_form != 0, cfg->tensor_cores));
+    CUDA_TRY(c, cudaEventRecord(c->ev3, c->stream));
+    CUDA_TRY(c, cudaEventSynchronize(c->ev3));
+    float ms = 0.f;
+    CUDA_TRY(c, cudaEventElapsedTime(&ms, c->ev0, c->ev3));
+    st.tiles_flagged = ntiles;
+    st.exact_points = npts;
+    st.ms_total = st.ms_fallback = ms;
+    c->last_ms = st.ms_total;
+    c->last_pairs = st.pairs;
+    c->last_launches = 0;
+    if (stats) *stats = st;
+    return BBKDE_OK;
+  }
   TRY(tile_order(c, g, c->gr_order));
   TRY(ensure(c, c->gr_flag, (size_t)ntiles * sizeof(int)));
   TRY(ensure(c, c->gr_flag_ord, (size_t)ntiles * sizeof(int)));
@@ -2384,7 +2401,6 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
   fa.gmax = c->gr_gmax.as<float>();
   fa.log_low = cfg->low_frac > 0 ? (float)std::log(cfg->low_frac) : -INFINITY;
   fa.rel_tol = (float)cfg->rel_tol;
-  fa.all = mode == BBKDE_GRID_EXACT;
   fa.flag = c->gr_flag.as<int>();
   fa.flag_ord = c->gr_flag_ord.as<int>();
   fa.counts = c->gr_counts.as<unsigned long long>();
@@ -2392,203 +2408,196 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
   // Rescue mode: the network runs after the probes, on the missed tiles only.
   const bool rescue =
       mode == BBKDE_GRID_ANCHORED && sur && cfg->net_scope != BBKDE_NET_EVERYWHERE;
-  const bool net_all = mode != BBKDE_GRID_EXACT && sur && !rescue;
-  if (mode == BBKDE_GRID_EXACT) {
-    CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
-    CUDA_TRY(c, cudaEventRecord(c->ev2, c->stream));
-    k_flag_tiles<<<grid1d(ntiles), 256, 0, c->stream>>>(fa);
+  const bool net_all = sur && !rescue;
+  // 1. Prediction at every point (log-density): the network, or zero.
+  bool pred_zero = false;
+  TRY(ensure(c, c->gr_pred, (size_t)npts * sizeof(float)));
+  float *pred = c->gr_pred.as<float>();
+  if (net_all) {
+    TRY(bbkde::surrogate_infer(sur, c->stream, npts, nullptr, g.nx, g.x0, g.dx, g.y0, g.dy,
+                               pred) == BBKDE_OK
+            ? BBKDE_OK
+            : fail(c, BBKDE_CUDA_ERROR, "grid: surrogate inference failed"));
     COUNT_LAUNCH(c);
   } else {
-    // 1. Prediction at every point (log-density): the network, or zero.
-    bool pred_zero = false;
-    TRY(ensure(c, c->gr_pred, (size_t)npts * sizeof(float)));
-    float *pred = c->gr_pred.as<float>();
-    if (net_all) {
-      TRY(bbkde::surrogate_infer(sur, c->stream, npts, nullptr, g.nx, g.x0, g.dx, g.y0, g.dy,
-                                 pred) == BBKDE_OK
-              ? BBKDE_OK
-              : fail(c, BBKDE_CUDA_ERROR, "grid: surrogate inference failed"));
-      COUNT_LAUNCH(c);
-    } else {
-      pred_zero = true;   // written by the interpolation below, never read as zeros
-    }
-    if (!rescue) CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
-    // 2. Exact values on the half-pitch lattice (anchors and probes; one regular
-    //    grid of pitch T/2 from the grid's origin, past its end by one pitch) and,
-    //    for 9 probes, on the quarter lattice; network values there.
-    const int h = T / 2;
-    const GridDesc gl = make_grid(2 * (int64_t)g.ntx + 1, 2 * (int64_t)g.nty + 1, g.x0,
-                                  h * g.dx, g.y0, h * g.dy, LT);
-    const int64_t n_lat = gl.nx * gl.ny;
-    TRY(ensure(c, c->gr_lat_exact, (size_t)n_lat * sizeof(double)));
-    TRY(grid_exact_all(c, r, gl, c->gr_lat_order, cfg->cull_rel, full,
-                       c->gr_lat_exact.as<double>(), &st.pairs, &st.max_bound_ratio,
+    pred_zero = true;   // written by the interpolation below, never read as zeros
+  }
+  if (!rescue) CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
+  // 2. Exact values on the half-pitch lattice (anchors and probes; one regular
+  //    grid of pitch T/2 from the grid's origin, past its end by one pitch) and,
+  //    for 9 probes, on the quarter lattice; network values there.
+  const int h = T / 2;
+  const GridDesc gl = make_grid(2 * (int64_t)g.ntx + 1, 2 * (int64_t)g.nty + 1, g.x0,
+                                h * g.dx, g.y0, h * g.dy, LT);
+  const int64_t n_lat = gl.nx * gl.ny;
+  TRY(ensure(c, c->gr_lat_exact, (size_t)n_lat * sizeof(double)));
+  TRY(grid_exact_all(c, r, gl, c->gr_lat_order, cfg->cull_rel, full,
+                     c->gr_lat_exact.as<double>(), &st.pairs, &st.max_bound_ratio,
+                     cfg->pair_form != 0, cfg->tensor_cores));
+  auto lattice_net = [&]() -> int {
+    TRY(ensure(c, c->gr_lat_net, (size_t)n_lat * sizeof(float)));
+    TRY(bbkde::surrogate_infer(sur, c->stream, n_lat, nullptr, gl.nx, gl.x0, gl.dx, gl.y0,
+                               gl.dy, c->gr_lat_net.as<float>()) == BBKDE_OK
+            ? BBKDE_OK
+            : fail(c, BBKDE_CUDA_ERROR, "grid: surrogate inference failed"));
+    COUNT_LAUNCH(c);
+    return BBKDE_OK;
+  };
+  const float *lat_net = nullptr, *q_net = nullptr;
+  if (net_all) {
+    TRY(lattice_net());
+    lat_net = c->gr_lat_net.as<float>();
+  }
+  int64_t n_q = 0;
+  const GridDesc gq = make_grid(2 * (int64_t)g.ntx, 2 * (int64_t)g.nty, g.x0 + (T / 4) * g.dx,
+                                h * g.dx, g.y0 + (T / 4) * g.dy, h * g.dy, LT);
+  auto quarter_net = [&]() -> int {
+    TRY(ensure(c, c->gr_q_net, (size_t)n_q * sizeof(float)));
+    TRY(bbkde::surrogate_infer(sur, c->stream, n_q, nullptr, gq.nx, gq.x0, gq.dx, gq.y0,
+                               gq.dy, c->gr_q_net.as<float>()) == BBKDE_OK
+            ? BBKDE_OK
+            : fail(c, BBKDE_CUDA_ERROR, "grid: surrogate inference failed"));
+    COUNT_LAUNCH(c);
+    return BBKDE_OK;
+  };
+  if (P == 9) {
+    n_q = gq.nx * gq.ny;
+    TRY(ensure(c, c->gr_q_exact, (size_t)n_q * sizeof(double)));
+    TRY(grid_exact_all(c, r, gq, c->gr_q_order, cfg->cull_rel, full,
+                       c->gr_q_exact.as<double>(), &st.pairs, &st.max_bound_ratio,
                        cfg->pair_form != 0, cfg->tensor_cores));
-    auto lattice_net = [&]() -> int {
-      TRY(ensure(c, c->gr_lat_net, (size_t)n_lat * sizeof(float)));
-      TRY(bbkde::surrogate_infer(sur, c->stream, n_lat, nullptr, gl.nx, gl.x0, gl.dx, gl.y0,
-                                 gl.dy, c->gr_lat_net.as<float>()) == BBKDE_OK
-              ? BBKDE_OK
-              : fail(c, BBKDE_CUDA_ERROR, "grid: surrogate inference failed"));
-      COUNT_LAUNCH(c);
-      return BBKDE_OK;
-    };
-    const float *lat_net = nullptr, *q_net = nullptr;
     if (net_all) {
-      TRY(lattice_net());
-      lat_net = c->gr_lat_net.as<float>();
+      TRY(quarter_net());
+      q_net = c->gr_q_net.as<float>();
     }
-    int64_t n_q = 0;
-    const GridDesc gq = make_grid(2 * (int64_t)g.ntx, 2 * (int64_t)g.nty, g.x0 + (T / 4) * g.dx,
-                                  h * g.dx, g.y0 + (T / 4) * g.dy, h * g.dy, LT);
-    auto quarter_net = [&]() -> int {
-      TRY(ensure(c, c->gr_q_net, (size_t)n_q * sizeof(float)));
-      TRY(bbkde::surrogate_infer(sur, c->stream, n_q, nullptr, gq.nx, gq.x0, gq.dx, gq.y0,
-                                 gq.dy, c->gr_q_net.as<float>()) == BBKDE_OK
+  }
+  // 3. Anchored mode: residual at the anchors, interpolated onto the grid.
+  const int64_t n_anchor = ((int64_t)g.ntx + 1) * (g.nty + 1);
+  const float *resid = nullptr;
+  if (mode == BBKDE_GRID_ANCHORED) {
+    TRY(ensure(c, c->gr_resid, (size_t)n_anchor * sizeof(float)));
+    k_anchor_residual<<<grid1d(n_anchor), 256, 0, c->stream>>>(
+        c->gr_lat_exact.as<double>(), lat_net, g.ntx, g.nty, c->gr_resid.as<float>());
+    COUNT_LAUNCH(c);
+    resid = c->gr_resid.as<float>();
+  }
+  if (pred_zero && !resid) {
+    CUDA_TRY(c, cudaMemsetAsync(pred, 0, (size_t)npts * sizeof(float), c->stream));
+    pred_zero = false;
+  }
+  k_tile_reduce<<<(unsigned)((ntiles + kTileReduceWarps - 1) / kTileReduceWarps),
+                  32 * kTileReduceWarps, 0, c->stream>>>(g, pred, resid, interp, pred_zero ? 1 : 0,
+                                                         c->gr_tmin.as<float>(),
+                                                         c->gr_tmax.as<float>(),
+                                                         c->gr_bad.as<int>());
+  COUNT_LAUNCH(c);
+  {
+    const unsigned nb = std::min<unsigned>(grid1d(ntiles), (unsigned)c->sm_count * 4);
+    TRY(ensure(c, c->gr_part, (size_t)nb * sizeof(double)));
+    k_max_finite<<<nb, 256, 0, c->stream>>>(c->gr_tmax.as<float>(), (int)ntiles,
+                                            c->gr_part.as<float>());
+    k_max_finite<<<1, 1024, 0, c->stream>>>(c->gr_part.as<float>(), (int)nb,
+                                            c->gr_gmax.as<float>());
+    c->launch_total += 2;
+  }
+  // 4. Held-out probes: every tile's interpolant against the exact lattice values.
+  ProbeArgs pa;
+  pa.g = g;
+  pa.list = nullptr;
+  pa.n_list = 0;
+  pa.lat_exact = c->gr_lat_exact.as<double>();
+  pa.lat_net = lat_net;
+  pa.q_exact = P == 9 ? c->gr_q_exact.as<double>() : nullptr;
+  pa.q_net = q_net;
+  pa.resid = resid;
+  pa.interp = interp;
+  pa.probes = P;
+  pa.terr = c->gr_terr.as<unsigned>();
+  k_probe_check<<<grid1d(ntiles), 256, 0, c->stream>>>(pa);
+  COUNT_LAUNCH(c);
+  k_flag_tiles<<<grid1d(ntiles), 256, 0, c->stream>>>(fa);
+  COUNT_LAUNCH(c);
+  CUDA_TRY(c, cudaGetLastError());
+  CUDA_TRY(c, cudaEventRecord(rescue ? c->ev1 : c->ev2, c->stream));
+  st.exact_points = n_lat + n_q;
+
+  // 5. Rescue: the network + its own residual on the tiles whose probes missed;
+  //    a tile keeps that prediction when its probes pass.
+  if (rescue) {
+    TRY(ensure(c, c->gr_cand_ord, (size_t)ntiles * sizeof(int)));
+    k_rescue_mark<<<grid1d(ntiles), 256, 0, c->stream>>>(fa, c->gr_cand_ord.as<int>());
+    COUNT_LAUNCH(c);
+    int ncand = 0;
+    TRY(select_flagged(c, c->gr_order.as<int>(), c->gr_cand_ord.as<int>(), c->gr_list.as<int>(),
+                       ntiles, &ncand));
+    if (ncand > 0) {
+      const int *cand = c->gr_list.as<int>();
+      // The network on the lattice points the candidates read (their anchors
+      // and probes), not on the whole lattice; NaN elsewhere (read by nothing).
+      const int64_t nl = (int64_t)ncand * kRescueSlots;
+      TRY(ensure(c, c->gr_lat_net, (size_t)n_lat * sizeof(float)));
+      TRY(ensure(c, c->gr_rl_idx, (size_t)nl * sizeof(int64_t)));
+      TRY(ensure(c, c->gr_rl_xy, (size_t)nl * sizeof(float2)));
+      TRY(ensure(c, c->gr_rl_net, (size_t)nl * sizeof(float)));
+      CUDA_TRY(c, cudaMemsetAsync(c->gr_lat_net.p, 0xff, (size_t)n_lat * sizeof(float),
+                                  c->stream));
+      k_rescue_lattice_points<<<grid1d(nl), 256, 0, c->stream>>>(
+          g, gl, cand, ncand, c->gr_rl_idx.as<int64_t>(), c->gr_rl_xy.as<float2>());
+      COUNT_LAUNCH(c);
+      TRY(bbkde::surrogate_infer(sur, c->stream, nl, c->gr_rl_xy.as<float2>(), 0, 0.0, 0.0,
+                                 0.0, 0.0, c->gr_rl_net.as<float>()) == BBKDE_OK
               ? BBKDE_OK
               : fail(c, BBKDE_CUDA_ERROR, "grid: surrogate inference failed"));
       COUNT_LAUNCH(c);
-      return BBKDE_OK;
-    };
-    if (P == 9) {
-      n_q = gq.nx * gq.ny;
-      TRY(ensure(c, c->gr_q_exact, (size_t)n_q * sizeof(double)));
-      TRY(grid_exact_all(c, r, gq, c->gr_q_order, cfg->cull_rel, full,
-                         c->gr_q_exact.as<double>(), &st.pairs, &st.max_bound_ratio,
-                         cfg->pair_form != 0, cfg->tensor_cores));
-      if (net_all) {
+      k_scatter_net<<<grid1d(nl), 256, 0, c->stream>>>(
+          c->gr_rl_idx.as<int64_t>(), c->gr_rl_net.as<float>(), nl, c->gr_lat_net.as<float>());
+      COUNT_LAUNCH(c);
+      lat_net = c->gr_lat_net.as<float>();
+      if (P == 9) {
         TRY(quarter_net());
         q_net = c->gr_q_net.as<float>();
       }
-    }
-    // 3. Anchored mode: residual at the anchors, interpolated onto the grid.
-    const int64_t n_anchor = ((int64_t)g.ntx + 1) * (g.nty + 1);
-    const float *resid = nullptr;
-    if (mode == BBKDE_GRID_ANCHORED) {
-      TRY(ensure(c, c->gr_resid, (size_t)n_anchor * sizeof(float)));
       k_anchor_residual<<<grid1d(n_anchor), 256, 0, c->stream>>>(
           c->gr_lat_exact.as<double>(), lat_net, g.ntx, g.nty, c->gr_resid.as<float>());
       COUNT_LAUNCH(c);
-      resid = c->gr_resid.as<float>();
-    }
-    if (pred_zero && !resid) {
-      CUDA_TRY(c, cudaMemsetAsync(pred, 0, (size_t)npts * sizeof(float), c->stream));
-      pred_zero = false;
-    }
-    k_tile_reduce<<<(unsigned)((ntiles + kTileReduceWarps - 1) / kTileReduceWarps),
-                    32 * kTileReduceWarps, 0, c->stream>>>(g, pred, resid, interp, pred_zero ? 1 : 0,
-                                                           c->gr_tmin.as<float>(),
-                                                           c->gr_tmax.as<float>(),
-                                                           c->gr_bad.as<int>());
-    COUNT_LAUNCH(c);
-    {
-      const unsigned nb = std::min<unsigned>(grid1d(ntiles), (unsigned)c->sm_count * 4);
-      TRY(ensure(c, c->gr_part, (size_t)nb * sizeof(double)));
-      k_max_finite<<<nb, 256, 0, c->stream>>>(c->gr_tmax.as<float>(), (int)ntiles,
-                                              c->gr_part.as<float>());
-      k_max_finite<<<1, 1024, 0, c->stream>>>(c->gr_part.as<float>(), (int)nb,
-                                              c->gr_gmax.as<float>());
-      c->launch_total += 2;
-    }
-    // 4. Held-out probes: every tile's interpolant against the exact lattice values.
-    ProbeArgs pa;
-    pa.g = g;
-    pa.list = nullptr;
-    pa.n_list = 0;
-    pa.lat_exact = c->gr_lat_exact.as<double>();
-    pa.lat_net = lat_net;
-    pa.q_exact = P == 9 ? c->gr_q_exact.as<double>() : nullptr;
-    pa.q_net = q_net;
-    pa.resid = resid;
-    pa.interp = interp;
-    pa.probes = P;
-    pa.terr = c->gr_terr.as<unsigned>();
-    k_probe_check<<<grid1d(ntiles), 256, 0, c->stream>>>(pa);
-    COUNT_LAUNCH(c);
-    k_flag_tiles<<<grid1d(ntiles), 256, 0, c->stream>>>(fa);
-    COUNT_LAUNCH(c);
-    CUDA_TRY(c, cudaGetLastError());
-    CUDA_TRY(c, cudaEventRecord(rescue ? c->ev1 : c->ev2, c->stream));
-    st.exact_points = n_lat + n_q;
-
-    // 5. Rescue: the network + its own residual on the tiles whose probes missed;
-    //    a tile keeps that prediction when its probes pass.
-    if (rescue) {
-      TRY(ensure(c, c->gr_cand_ord, (size_t)ntiles * sizeof(int)));
-      k_rescue_mark<<<grid1d(ntiles), 256, 0, c->stream>>>(fa, c->gr_cand_ord.as<int>());
+      const int64_t np = (int64_t)ncand * T * T;
+      TRY(ensure(c, c->gr_cand_xy, (size_t)np * sizeof(float2)));
+      TRY(ensure(c, c->gr_cand_net, (size_t)np * sizeof(float)));
+      k_tile_points<<<grid1d(np), 256, 0, c->stream>>>(g, cand, np,
+                                                      c->gr_cand_xy.as<float2>());
       COUNT_LAUNCH(c);
-      int ncand = 0;
-      TRY(select_flagged(c, c->gr_order.as<int>(), c->gr_cand_ord.as<int>(), c->gr_list.as<int>(),
-                         ntiles, &ncand));
-      if (ncand > 0) {
-        const int *cand = c->gr_list.as<int>();
-        // The network on the lattice points the candidates read (their anchors
-        // and probes), not on the whole lattice; NaN elsewhere (read by nothing).
-        const int64_t nl = (int64_t)ncand * kRescueSlots;
-        TRY(ensure(c, c->gr_lat_net, (size_t)n_lat * sizeof(float)));
-        TRY(ensure(c, c->gr_rl_idx, (size_t)nl * sizeof(int64_t)));
-        TRY(ensure(c, c->gr_rl_xy, (size_t)nl * sizeof(float2)));
-        TRY(ensure(c, c->gr_rl_net, (size_t)nl * sizeof(float)));
-        CUDA_TRY(c, cudaMemsetAsync(c->gr_lat_net.p, 0xff, (size_t)n_lat * sizeof(float),
-                                    c->stream));
-        k_rescue_lattice_points<<<grid1d(nl), 256, 0, c->stream>>>(
-            g, gl, cand, ncand, c->gr_rl_idx.as<int64_t>(), c->gr_rl_xy.as<float2>());
-        COUNT_LAUNCH(c);
-        TRY(bbkde::surrogate_infer(sur, c->stream, nl, c->gr_rl_xy.as<float2>(), 0, 0.0, 0.0,
-                                   0.0, 0.0, c->gr_rl_net.as<float>()) == BBKDE_OK
-                ? BBKDE_OK
-                : fail(c, BBKDE_CUDA_ERROR, "grid: surrogate inference failed"));
-        COUNT_LAUNCH(c);
-        k_scatter_net<<<grid1d(nl), 256, 0, c->stream>>>(
-            c->gr_rl_idx.as<int64_t>(), c->gr_rl_net.as<float>(), nl, c->gr_lat_net.as<float>());
-        COUNT_LAUNCH(c);
-        lat_net = c->gr_lat_net.as<float>();
-        if (P == 9) {
-          TRY(quarter_net());
-          q_net = c->gr_q_net.as<float>();
-        }
-        k_anchor_residual<<<grid1d(n_anchor), 256, 0, c->stream>>>(
-            c->gr_lat_exact.as<double>(), lat_net, g.ntx, g.nty, c->gr_resid.as<float>());
-        COUNT_LAUNCH(c);
-        const int64_t np = (int64_t)ncand * T * T;
-        TRY(ensure(c, c->gr_cand_xy, (size_t)np * sizeof(float2)));
-        TRY(ensure(c, c->gr_cand_net, (size_t)np * sizeof(float)));
-        k_tile_points<<<grid1d(np), 256, 0, c->stream>>>(g, cand, np,
-                                                        c->gr_cand_xy.as<float2>());
-        COUNT_LAUNCH(c);
-        TRY(bbkde::surrogate_infer(sur, c->stream, np, c->gr_cand_xy.as<float2>(), 0, 0.0, 0.0,
-                                   0.0, 0.0, c->gr_cand_net.as<float>()) == BBKDE_OK
-                ? BBKDE_OK
-                : fail(c, BBKDE_CUDA_ERROR, "grid: surrogate inference failed"));
-        COUNT_LAUNCH(c);
-        k_tile_predict_list<<<(unsigned)ncand, 256, 0, c->stream>>>(
-            g, cand, c->gr_cand_net.as<float>(), resid, interp, pred, c->gr_bad.as<int>());
-        COUNT_LAUNCH(c);
-        pa.list = cand;
-        pa.n_list = ncand;
-        pa.lat_net = lat_net;
-        pa.q_net = q_net;
-        k_probe_check<<<grid1d(ncand), 256, 0, c->stream>>>(pa);
-        COUNT_LAUNCH(c);
-        k_rescue_update<<<grid1d(ncand), 256, 0, c->stream>>>(
-            cand, ncand, c->gr_bad.as<int>(), c->gr_terr.as<unsigned>(), (float)cfg->rel_tol,
-            c->gr_flag.as<int>());
-        COUNT_LAUNCH(c);
-        CUDA_TRY(c, cudaMemsetAsync(c->gr_counts.as<unsigned long long>() + 1, 0,
-                                    2 * sizeof(unsigned long long), c->stream));
-        k_flag_recount<<<grid1d(ntiles), 256, 0, c->stream>>>(fa);
-        COUNT_LAUNCH(c);
-        CUDA_TRY(c, cudaGetLastError());
-      }
-      CUDA_TRY(c, cudaEventRecord(c->ev2, c->stream));
+      TRY(bbkde::surrogate_infer(sur, c->stream, np, c->gr_cand_xy.as<float2>(), 0, 0.0, 0.0,
+                                 0.0, 0.0, c->gr_cand_net.as<float>()) == BBKDE_OK
+              ? BBKDE_OK
+              : fail(c, BBKDE_CUDA_ERROR, "grid: surrogate inference failed"));
+      COUNT_LAUNCH(c);
+      k_tile_predict_list<<<(unsigned)ncand, 256, 0, c->stream>>>(
+          g, cand, c->gr_cand_net.as<float>(), resid, interp, pred, c->gr_bad.as<int>());
+      COUNT_LAUNCH(c);
+      pa.list = cand;
+      pa.n_list = ncand;
+      pa.lat_net = lat_net;
+      pa.q_net = q_net;
+      k_probe_check<<<grid1d(ncand), 256, 0, c->stream>>>(pa);
+      COUNT_LAUNCH(c);
+      k_rescue_update<<<grid1d(ncand), 256, 0, c->stream>>>(
+          cand, ncand, c->gr_bad.as<int>(), c->gr_terr.as<unsigned>(), (float)cfg->rel_tol,
+          c->gr_flag.as<int>());
+      COUNT_LAUNCH(c);
+      CUDA_TRY(c, cudaMemsetAsync(c->gr_counts.as<unsigned long long>() + 1, 0,
+                                  2 * sizeof(unsigned long long), c->stream));
+      k_flag_recount<<<grid1d(ntiles), 256, 0, c->stream>>>(fa);
+      COUNT_LAUNCH(c);
+      CUDA_TRY(c, cudaGetLastError());
     }
-    // 6. Predicted values on the tiles that keep them.
-    const dim3 ab((unsigned)std::min<int64_t>((g.nx + 1023) / 1024, 16),
-                  (unsigned)std::min<int64_t>(g.ny, (int64_t)c->sm_count * 8));
-    k_apply<<<ab, 256, 0, c->stream>>>(g, T == 32 ? 5 : 4, c->gr_pred.as<float>(),
-                                       c->gr_flag.as<int>(), out);
-    COUNT_LAUNCH(c);
+    CUDA_TRY(c, cudaEventRecord(c->ev2, c->stream));
   }
+  // 6. Predicted values on the tiles that keep them.
+  const dim3 ab((unsigned)std::min<int64_t>((g.nx + 1023) / 1024, 16),
+                (unsigned)std::min<int64_t>(g.ny, (int64_t)c->sm_count * 8));
+  k_apply<<<ab, 256, 0, c->stream>>>(g, T == 32 ? 5 : 4, c->gr_pred.as<float>(),
+                                     c->gr_flag.as<int>(), out);
+  COUNT_LAUNCH(c);
   // 7. Exact fallback on the flagged tiles.
   CUDA_TRY(c, cudaGetLastError());
   int nsel = 0;
@@ -2598,11 +2607,7 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
                               c->stream));
   TRY(select_flagged(c, c->gr_order.as<int>(), c->gr_flag_ord.as<int>(), c->gr_list.as<int>(),
                      ntiles, &nsel));
-  if (mode == BBKDE_GRID_EXACT) {
-    TRY(grid_exact_all(c, r, g, c->gr_quad_order, cfg->cull_rel, full, out, &st.pairs,
-                       &st.max_bound_ratio, cfg->pair_form != 0, cfg->tensor_cores));
-    nsel = 0;
-  } else if (T == 16 && !cfg->pair_form && op_separable(r.op) && nsel >= kGridWideMin) {
+  if (T == 16 && !cfg->pair_form && op_separable(r.op) && nsel >= kGridWideMin) {
     // 2 x 2 blocks of (nearly) all flagged tiles leave the list of single tiles
     quads = true;
     const GridDesc g32 = make_grid(g.nx, g.ny, g.x0, g.dx, g.y0, g.dy, 32);
@@ -2666,12 +2671,12 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
   unsigned eb = (unsigned)counts[2];
   float pe = 0.f;
   std::memcpy(&pe, &eb, sizeof(pe));
-  st.max_probe_err = mode == BBKDE_GRID_EXACT ? 0.0 : (double)pe;
+  st.max_probe_err = (double)pe;
   c->last_ms = st.ms_total;
   c->last_pairs = st.pairs;
   c->last_launches = 0;
   if (stats) *stats = st;
-  if (mode != BBKDE_GRID_EXACT && sur && bbkde::surrogate_check(sur) != BBKDE_OK)
+  if (sur && bbkde::surrogate_check(sur) != BBKDE_OK)
     return fail(c, BBKDE_TIMEOUT, "grid: surrogate inference wait expired");
   return BBKDE_OK;
 }

@@ -291,7 +291,6 @@ struct FlagArgs {
   const float *gmax;
   float log_low;          // log(low_frac)
   float rel_tol;
-  int all;                // flag every tile
   int *flag;              // per tile
   int *flag_ord;          // per Morton position
   unsigned long long *counts;   // [0] low, [1] flagged, [2] max probe error bits (non-low)
@@ -318,13 +317,10 @@ __global__ void k_flag_tiles(FlagArgs a) {
   unsigned eb = 0;
   if (in) {
     const int t = a.order[o];
-    f = a.all;
-    if (!f) {
-      low = !(a.tmin[t] >= *a.gmax + a.log_low);
-      const float err = a.terr ? __uint_as_float(a.terr[t]) : 0.f;
-      f = a.bad[t] || low || !(err <= a.rel_tol);
-      if (!low) eb = __float_as_uint(err);
-    }
+    low = !(a.tmin[t] >= *a.gmax + a.log_low);
+    const float err = a.terr ? __uint_as_float(a.terr[t]) : 0.f;
+    f = a.bad[t] || low || !(err <= a.rel_tol);
+    if (!low) eb = __float_as_uint(err);
     a.flag[t] = f;
     a.flag_ord[o] = f;
   }
