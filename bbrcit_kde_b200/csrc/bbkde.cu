@@ -1782,9 +1782,15 @@ int sep_schedule(bbkde_ctx *c, CullArgs &a, unsigned nblk) {
 // Parts per tile for a factored launch of nblk tiles of edge `tile`: enough for two waves
 // of blocks (1,089 tile-16 lattice tiles of a 4,096^2 pipeline, one wave: 5.6 ms in one
 // part, 3.7 in two, 3.4 in four; 8,714 flagged tiles 7.7 in one, 8.1 in two).
+// Below kSepSplitRefTiles reference tiles a part has too few of them to pay for a second
+// wave (2-D Gaussian, 300 x 300 points: 6,000 references 94 us in one wave, 117 in two;
+// lattice of a 4,096^2 pipeline, 1,000 references: 140 / 170; but 100,000 references on a
+// 2,048^2 pipeline's 510 / 390).
 constexpr double kSepSplitWaves = 2.0;
-int sep_parts(const bbkde_ctx *c, int tile, unsigned nblk) {
-  const double per = kSepSplitWaves * c->sm_count * sep_resident(tile) / (double)nblk;
+constexpr int kSepSplitRefTiles = 64;
+int sep_parts(const bbkde_ctx *c, int tile, unsigned nblk, int ref_tiles) {
+  const double waves = ref_tiles < kSepSplitRefTiles ? 1.0 : kSepSplitWaves;
+  const double per = waves * c->sm_count * sep_resident(tile) / (double)nblk;
   return per >= 8 ? 8 : per >= 4 ? 4 : per >= 2 ? 2 : 1;
 }
 
@@ -1829,7 +1835,7 @@ int launch_culled(bbkde_ctx *c, const Resolved &r, unsigned nblk, const CullQuer
   if (tc) CUDA_TRY(c, cudaMemsetAsync(a.status, 0, sizeof(int), c->stream));
   const bool d2 = r.dim == 2;
   if (sep_tile > 0) {
-    const int parts = tc ? 1 : sep_parts(c, sep_tile, nblk);
+    const int parts = tc ? 1 : sep_parts(c, sep_tile, nblk, lv.n_tiles);
     // More than one wave: launch the tiles most expensive first.
     if (parts == 1 && q.mode == 1 &&
         (int64_t)nblk > (int64_t)c->sm_count * sep_resident(sep_tile)) {
