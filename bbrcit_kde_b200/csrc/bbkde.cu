@@ -1588,10 +1588,17 @@ constexpr double kGridLatticeSpan = 16.0;
 // Exact 16-point tiles of a separable kernel run as 32-point ones: an exact grid always
 // (262,144 references, ms in 16- / 32-point tiles: 1,000 x 900 points 1.44 / 1.08, 500 x
 // 450 1.18 / 0.53, 250 x 225 0.51 / 0.32, 64 x 64 0.44 / 0.38), the pipeline's flagged
-// tiles from this many on (building the list of 2 x 2 blocks is ten small launches,
-// about 50 us) in blocks with at least kGridQuadMin of their tiles flagged (the 32-point
-// kernel sums about 1.7x the pairs per second; 8,714 tiles 8.8 -> 7.7 ms).
-constexpr int kGridWideMin = 1024;
+// tiles in blocks with at least kGridQuadMin of their tiles flagged (the 32-point kernel
+// sums about 1.7x the pairs per second; 8,714 tiles of 10^6 references 8.8 -> 7.7 ms)
+// where that is worth the list of blocks: sorting and selecting it are a dozen launches
+// and two waits, 100-150 us. A flagged tile takes about 0.5 ns sqrt(n) with n references
+// (0.02 us at 1,000, 0.3 at 400,000), so that a fifth of the list's time exceeds that from
+// tiles x sqrt(n) = kGridQuadWork on, about 0.75 ms. Fallback us without / with blocks:
+// 1,000 references 14,100 tiles 351 / 377, 48,162 tiles 881 / 825; 25,000 references 3,844
+// tiles 365 / 424, 13,749 tiles 948 / 775; 400,000 references 3,347 tiles 1,360 / 1,245,
+// 9,791 tiles 3,948 / 3,384.
+constexpr int64_t kGridQuadTiles = 1024;   // never below: the parts of short lists are better
+constexpr double kGridQuadWork = 1.5e6;
 constexpr int kGridQuadMin = 3;
 
 // Curve order of n points (x[i * stride], y[i * stride]; y null for 1-D) into
@@ -2253,7 +2260,7 @@ int grid_exact(bbkde_ctx *c, const Resolved &r, const GridDesc &g, const int *li
 }
 
 // Exact sums at every point of g. Tiles of 16 points of a separable kernel are summed as
-// 32-point ones, on the FP32 pipe as they would be (kGridWideMin's comment).
+// 32-point ones, on the FP32 pipe as they would be (kGridQuadWork's comment).
 int grid_exact_all(bbkde_ctx *c, const Resolved &r, const GridDesc &g, DevBuf &order, double rel,
                    bool full, double *out, double *pairs, double *ratio, bool pair_form,
                    int tensor_cores) {
@@ -2613,7 +2620,8 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
                               c->stream));
   TRY(select_flagged(c, c->gr_order.as<int>(), c->gr_flag_ord.as<int>(), c->gr_list.as<int>(),
                      ntiles, &nsel));
-  if (T == 16 && !cfg->pair_form && op_separable(r.op) && nsel >= kGridWideMin) {
+  if (T == 16 && !cfg->pair_form && op_separable(r.op) && nsel >= kGridQuadTiles &&
+      nsel * std::sqrt((double)rs.n) >= kGridQuadWork) {
     // 2 x 2 blocks of (nearly) all flagged tiles leave the list of single tiles
     quads = true;
     const GridDesc g32 = make_grid(g.nx, g.ny, g.x0, g.dx, g.y0, g.dy, 32);
@@ -2640,23 +2648,23 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
   TRY(grid_exact(c, r, g, c->gr_list.as<int>(), nsel, cfg->cull_rel, full, out, &st.pairs,
                  &st.max_bound_ratio, cfg->pair_form != 0, cfg->tensor_cores));
   CUDA_TRY(c, cudaEventRecord(c->ev3, c->stream));
-  // Tiles summed exactly -- the flagged ones, and the fourth of a block summed whole --
-  // and their points (edge tiles may be partial).
+  // Tiles summed exactly -- the flagged ones, and the fourth of a block summed whole (a
+  // block at an edge has two tiles at most) -- and their points (edge tiles may be partial).
   std::vector<int> flags((size_t)ntiles);
   CUDA_TRY(c, cudaMemcpyAsync(flags.data(), c->gr_flag.p, (size_t)ntiles * sizeof(int),
                               cudaMemcpyDeviceToHost, c->stream));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  if (quads)
+    for (int64_t y = 0; y + 1 < g.nty; y += 2) {
+      int *lo = flags.data() + y * g.ntx, *hi = lo + g.ntx;
+      for (int64_t x = 0; x + 1 < g.ntx; x += 2)
+        if (lo[x] + lo[x + 1] + hi[x] + hi[x + 1] >= kGridQuadMin)
+          lo[x] = lo[x + 1] = hi[x] = hi[x + 1] = 1;
+    }
   int64_t fb_points = 0, fb_tiles = 0;
   for (int64_t t = 0; t < ntiles; ++t) {
+    if (!flags[(size_t)t]) continue;
     const int64_t tx = t % g.ntx, ty = t / g.ntx;
-    if (!flags[(size_t)t]) {
-      int block = 0;
-      if (quads)
-        for (int64_t y = ty & ~1; y < std::min<int64_t>((ty & ~1) + 2, g.nty); ++y)
-          for (int64_t x = tx & ~1; x < std::min<int64_t>((tx & ~1) + 2, g.ntx); ++x)
-            block += flags[(size_t)(y * g.ntx + x)] != 0;
-      if (!quads || block < kGridQuadMin) continue;
-    }
     ++fb_tiles;
     fb_points += std::min<int64_t>(T, g.nx - tx * T) * std::min<int64_t>(T, g.ny - ty * T);
   }

@@ -432,10 +432,11 @@ typedef struct {
 enum { BBKDE_NET_RESCUE = 0, BBKDE_NET_EVERYWHERE = 1 };
 
 typedef struct {
-  /* tiles_flagged: tiles summed exactly. From 1,024 flagged 16-point tiles of a separable
-   * kernel on, a 2 x 2 block with three flagged tiles is summed whole: its fourth tile
-   * counts as flagged, and its predicted values give way to the exact ones. The others
-   * (tiles_surrogate) keep their predicted values. */
+  /* tiles_flagged: tiles summed exactly. In long lists of flagged 16-point tiles of a
+   * separable kernel (at least 1,024, and 1.5e6 / sqrt(references)) a 2 x 2 block with
+   * three flagged tiles is summed whole: its fourth tile counts as flagged, and its
+   * predicted values give way to the exact ones. The others (tiles_surrogate) keep their
+   * predicted values. */
   int64_t tiles, tiles_low, tiles_flagged, tiles_surrogate;
   int64_t exact_points;       /* points evaluated by an exact sum (lattices, fallback) */
   double pairs;               /* reference-query pairs of those sums (tile granularity) */
