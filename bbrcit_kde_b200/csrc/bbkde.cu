@@ -1797,7 +1797,8 @@ constexpr double kSepSplitWaves = 2.0;
 constexpr int kSepSplitRefTiles = 64;
 int sep_parts(const bbkde_ctx *c, int tile, unsigned nblk, int ref_tiles) {
   const double waves = ref_tiles < kSepSplitRefTiles ? 1.0 : kSepSplitWaves;
-  const double per = waves * c->sm_count * sep_resident(tile) / (double)nblk;
+  const double per = std::min(waves * c->sm_count * sep_resident(tile) / (double)nblk,
+                              0.5 * ref_tiles);   // two reference tiles a part at least
   return per >= 8 ? 8 : per >= 4 ? 4 : per >= 2 ? 2 : 1;
 }
 

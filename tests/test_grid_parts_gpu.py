@@ -83,9 +83,10 @@ def test_long_list_of_single_16_point_tiles(ctx):
 
 @pytest.mark.parametrize("tx,ty,cut", [(3, 2, 9), (12, 12, 0), (13, 12, 1), (17, 17, 0), (18, 17, 5),
                                        (24, 24, 0), (25, 24, 31)])   # 8, 8, 4, 4, 2, 2, 1 parts
-@pytest.mark.parametrize("tile,n", [(16, 60_000), (32, 60_000), (32, 5_000)])
+@pytest.mark.parametrize("tile,n", [(16, 60_000), (32, 60_000), (32, 5_000), (32, 1_300)])
 def test_exact_grids_in_32_point_tiles(ctx, tx, ty, cut, tile, n):
-    """Half as many parts, or one, with fewer than 64 reference tiles (5,000 points)."""
+    """Half as many parts, or one, with fewer than 64 reference tiles (5,000 points); two
+    with six of them."""
     desc = _refs(ctx, n)
     grid = (32 * tx - cut, 32 * ty - cut, -4.0, 4.0, -4.0, 4.0)
     want = _direct(ctx, desc, grid)
