@@ -426,11 +426,15 @@ inline int segment_step(int variant, bool f64) {
 }
 
 // Four queries per FP64 thread while that still makes two blocks per SM (segments of
-// one staging tile at the least), else one.
+// one staging tile at the least) and does not fill too much of its blocks with no query:
+// a 512-query block takes 10/3 of a 128-query one (2 * 10^6 references, us with one / four:
+// 1 query 361 / 1,162, 257 1,054 / 1,167, 400 1,404 / 1,168, 513 1,745 / 2,318, 800 2,439 /
+// 2,319).
 inline int f64_qpt(const bbkde_ctx *c, int64_t n_ref, int64_t q_count) {
-  const int64_t blocks = ((q_count + 4 * kBlock64 - 1) / (4 * kBlock64)) *
-                         ((n_ref + kBlock64 - 1) / kBlock64);
-  return blocks >= 2 * c->sm_count ? 4 : 1;
+  const int64_t one = (q_count + kBlock64 - 1) / kBlock64;
+  const int64_t four = (q_count + 4 * kBlock64 - 1) / (4 * kBlock64);
+  const int64_t blocks = four * ((n_ref + kBlock64 - 1) / kBlock64);
+  return blocks >= 2 * c->sm_count && 3 * one >= 10 * four ? 4 : 1;
 }
 
 struct Plan {

@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 KINDS = [(W.GAUSS, 2, (0.3, 0.3)), (W.GAUSS_PROD2D, 2, (0.2, 0.5)), (W.EPAN, 2, (0.8, 0.8)),
          (W.EPAN_PROD2D, 2, (0.9, 0.6)), (W.EPAN_PROD_CONV2D, 2, (0.5, 0.7)),
          (W.GAUSS, 1, (0.3, 0.3)), (W.EPAN, 1, (0.6, 0.6)), (W.EPAN_CONV1D, 1, (0.4, 0.4))]
-SIZES = [(1, 1), (63, 65), (64, 64), (65, 127), (511, 129), (513, 63), (4097, 517), (300, 40_000)]
+SIZES = [(1, 1), (63, 65), (64, 64), (65, 127), (511, 129), (513, 63), (4097, 517), (300, 40_000),
+         (40_000, 257), (40_000, 385), (20_000, 641), (20_000, 801)]   # FP64: 1, 4, 1, 4 a thread
 
 
 def _problem(seed, n, m, dim):
