@@ -922,15 +922,18 @@ int bbkde_upload(bbkde_ctx *c, int role, int dim, int64_t n, const double *coord
       CUDA_TRY(c, cudaMemcpyAsync(c->staging.p, coords, (size_t)n * dim * sizeof(double),
                                   cudaMemcpyHostToDevice, c->stream));
       in.coords = c->staging.as<double>();
-      for (int k = 0; k < 3; ++k) {
-        if (!cols[k]) continue;
-        CUDA_TRY(c, cudaMemcpyAsync(home[k], cols[k], nb, cudaMemcpyHostToDevice, c->stream));
-        *to[k] = home[k];
-      }
+      for (int k = 0; k < 3; ++k)
+        if (cols[k]) *to[k] = home[k];
+      if (mass && !weight)   // read by the kernel: the weight is the mass
+        CUDA_TRY(c, cudaMemcpyAsync(in.m, mass, nb, cudaMemcpyHostToDevice, c->stream));
     }
     k_ingest<<<grid1d(n, 128), 128, 0, c->stream>>>(in);
     COUNT_LAUNCH(c);
     CUDA_TRY(c, cudaGetLastError());
+    // The other columns go home while it runs (the host stages pageable memory meanwhile).
+    for (int k = 0; !host && k < 3; ++k)
+      if (cols[k] && !(k == 0 && !weight))
+        CUDA_TRY(c, cudaMemcpyAsync(home[k], cols[k], nb, cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   }
   s.dim = dim;
