@@ -441,14 +441,15 @@ constexpr int kTile = 256;
 constexpr int kBlock64 = 128;
 // Problems below this many pairs skip autotuning: up to kSplitMaxPairs they run
 // k_pair_sum_split, above it a fixed shape (untuned_variant). Kernel us, split / fixed:
-// 500 x 400 queries 8 / 13, 2,000 x 2,000 9 / 13, 10,000 x 10,000 36 / 36, 50,000 x
-// 50,000 630 / 595 (2-D Gaussian; 28, 30, 48, 633 in the 2,048-query blocks of shape 0).
+// 500 x 400 queries 7 / 11, 2,000 x 2,000 7 / 11, 10,000 x 10,000 35 / 34, 17,300 x 17,300
+// 85 / 78, 50,000 x 50,000 630 / 583 (2-D Gaussian; 25, 25, 44, 99, 631 in the 2,048-query
+// blocks of shape 0).
 constexpr double kAutotuneMinPairs = 2.0e10;
 constexpr double kSplitMaxPairs = 3.0e8;
 
 // 1-D Gaussians have so few FP32 operations that three of 16 references' exponentials
-// fit there (50,000 x 50,000: 524 us, every 8th 544, every 32nd 566, none 589); 2-D ones
-// take every 32nd (593, 638 with every 8th, 617 with none). The other kernels ignore the
+// fit there (50,000 x 50,000: 531 us, every 8th 538, every 32nd 564, none 584); 2-D ones
+// take every 32nd (583, 626 with every 8th, 603 with none). The other kernels ignore the
 // split.
 inline int untuned_variant(const Resolved &r, double pairs) {
   return pairs <= kSplitMaxPairs ? kSplitVariant : r.dim == 1 ? 6 : 9;
@@ -1175,7 +1176,8 @@ namespace {
 // end of the launch; larger ones pay the per-item histogram set-up and flush less
 // often. A call with few points takes smaller items whatever the plan: about
 // kCvItemsPerSm of each kind per SM (500 points at 64 x 48: 5.2 ms in
-// one item of 500 queries, 0.09 ms in items of two).
+// one item of 500 queries, 0.09 ms in items of two). So the plans differ from 38,000
+// points in all on (convolution items), and in their likelihood items from 1.2 million on.
 constexpr int kCvItemsPerSm = 8;
 constexpr int kCvMinQueries = 16;   // least queries of a convolution item
 // A likelihood query's histogram and scores cost as much as this many candidates.
@@ -1627,11 +1629,13 @@ constexpr float kCullCutPair = 10.0f;
 // while the tile span is at most this many narrowest kernel widths, else 9.
 constexpr double kGridProbeSpan = 0.75;
 // Automatic lattice tile (bbkde_grid_config.lattice_tile = 0): 32 while a 32-point
-// lattice tile spans at most this many narrowest kernel widths, else 16. The
-// 32-point tile halves the kernel factors per point (1.44x the pairs per second);
-// its larger box adds the references near its edge, which costs more than that
-// saves on coarse lattices (measured on the Gaussian mixture: a 32-point tile of
-// 10 narrowest widths 20% faster, of 33 and 80 widths 5-7% slower).
+// lattice tile spans at most this many narrowest kernel widths, else 16. Of a separable
+// kernel both are summed in 32-point tiles (grid_exact_all); the setting says whether the
+// tensor cores may take them (culled to 1e-5, lists of a wave and more), whose blocks hold
+// one tile each: a wide tile's longer lists end unevenly. 10^6 adaptive references, exact
+// lattices of an 8,192^2 pipeline, ms as 16 (FP32 pipe) / 32: span 4.9 4.47 / 4.21, 10.1
+// 2.20 / 2.08, 20.6 1.17 / 1.17, 54 0.75 / 0.78; of a 6,400^2 one, span 12.9 1.97 / 1.95,
+// 26.4 1.06 / 1.13, 69 0.75 / 0.78; smaller lattices are the same either way.
 constexpr double kGridLatticeSpan = 16.0;
 // Exact 16-point tiles of a separable kernel run as 32-point ones: an exact grid always
 // (262,144 references, ms in 16- / 32-point tiles: 1,000 x 900 points 1.44 / 1.08, 500 x

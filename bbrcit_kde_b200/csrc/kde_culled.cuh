@@ -63,8 +63,8 @@ constexpr int kGroupTiles = 16;    // tiles per tile group (two-level scan)
 // warps 0.19 (3.3e8); 32 references 0.23 (2.7e8: staging per pair); 128
 // references 0.22 (4.1e8); 128 queries 0.29 (3.7e8); 4 warps 0.23. The former
 // shape, 1,024 queries in eight strips x 256 references, 128 threads: 2.86
-// (1.35e9), on 59 blocks. 300,000 x 300,000 (h = 0.2): 4.3 ms, 3.6e12 pairs/s (77%
-// of the bound); 17.7 ms before.
+// (1.35e9), on 59 blocks. 300,000 x 300,000 (h = 0.2, 1e-5): 4.23 ms, 3.4e12 pairs/s
+// (74% of the bound); 17.7 ms before.
 constexpr int kCullQpb = 64;
 constexpr int kCullWarps = 8;
 constexpr int kCullUnit = 64;
@@ -332,9 +332,10 @@ __device__ __forceinline__ int cull_pass(const CullArgs &a, const CullGroups &gr
 //   * The tiles from t0 up to -2 are counted per bit; the threshold is the highest bit at
 //     which the counted bounds below it (each taken at its bit's upper edge) still hold
 //     at most kFarShare (with parts > 1 that share of it, each part for its own tiles).
-//     A quarter would keep the guarantee; the smaller share keeps the part left out,
-//     which is always missing on the same side, an order below the tolerance asked for
-//     (a 1-D likelihood to 1e-6: off by 4.7e-7 with a quarter).
+//     A quarter would keep the guarantee too; what is left out is always missing on the
+//     same side, so the nearer tiles, whose bounds are the sharper ones, are given less
+//     (a 1-D likelihood to 1e-6: off by 4.7e-7 with a quarter, 6.8e-8 with this).
+//   Together at most 1/4 + 1/32 = 9/32 of the allowance.
 // A threshold of -log2(n_tiles) - 1 for every tile, which needs no count, charges each of
 // them as much as the nearest one left out and lies two to three bits lower: 400,000 x
 // 300,000 at 1e-6 lists 3.71e9 pairs instead of 4.10e9 (1.62 -> 1.57 ms), the flagged

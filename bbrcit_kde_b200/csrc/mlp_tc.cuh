@@ -323,8 +323,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_infer_tc(TcArgs ta) {
 // between them, so its time is the latency of those passes: four threads per point
 // run each pass over 32 features instead of 128, and the per-feature sums are taken
 // while the next products run. Measured, a step of
-// 8,192 points with its reduction: 40 us with one thread per point, 25 with four, 20
-// with the derivatives kept in TMEM, bulk weight copies and the first layer's sums
+// 8,192 points with its reduction: 37 us with one thread per point, 19 with four, the
+// derivatives kept in TMEM, bulk weight copies and the first layer's sums
 // through shared memory; MUFU (two operations per SiLU, three layers: 3 us) and the
 // latency of the four products with their hand-offs are what is left.
 //

@@ -54,10 +54,10 @@ def pair_sum_bound_per_clk_per_sm(poly: int, fma_cycles: float = 12.0) -> tuple[
     per 64 pairs (two queries per packed instruction) the main path issues
     fma_cycles / 2 packed FP32 instructions (2 FMA-pipe cycles each: 12 cycles for
     the 2-D isotropic kernel, 8 in 1-D) and 2 MUFU.EX2 (8 cycles each on a
-    4-lane-per-clock unit: 16 cycles); the polynomial exp2 costs 8 packed
-    instructions (16 cycles) instead of the 2 MUFU operations. 4 SMSPs per SM."""
+    4-lane-per-clock unit: 16 cycles); the polynomial exp2 costs 9 packed
+    instructions (18 cycles) instead of the 2 MUFU operations. 4 SMSPs per SM."""
     mufu = 4 * 64 / (16.0 * (1 - 1 / poly)) if poly else 4 * 64 / 16.0
-    fma = 4 * 64 / (fma_cycles + (16.0 / poly if poly else 0.0))
+    fma = 4 * 64 / (fma_cycles + (18.0 / poly if poly else 0.0))
     bound = "sfu" if mufu <= fma else "fma"
     if poly:
         bound = "sfu+fma (exp2 split: MUFU and FP32 polynomial)"
@@ -734,13 +734,14 @@ def run_surrogate_grid(a, world, rank, local):
         ce = results["culled_exact"]
         peak = sm_count * FP32_FMA_PER_CLK_PER_SM * sm_max * 1e6
         ach = ce["pairs"] / (ce["ms_total"] / 1e3)
-        roofline = {"bound": "fp32", "kernel": f"k_pair_sum_culled_sep<GAUSS_ISO,{lt}> "
+        roofline = {"bound": "fp32", "kernel": "k_pair_sum_culled_sep<GAUSS_ISO,32> "
                                                "(factored culled exact grid; the pipeline's "
                                                "lattice launch)",
                     "achieved": ach / 1e9, "peak": peak / 1e9, "unit": "Gpair/s",
                     "frac": ach / peak, "traffic": None,
                     "peak_basis": f"{sm_count} SMs x 128 FP32 FMA/clk x {sm_max:.0f} MHz "
-                                  f"(MUFU allows {8 * lt} pairs/clk/SM at tile {lt}); "
+                                  "(MUFU allows 256 pairs/clk/SM at tile 32, in which "
+                                  "16-point lattice tiles are summed); "
                                   "compute-bound, DRAM traffic negligible"}
     cpu = None
     if rank == 0 and not a.no_cpu_baseline:

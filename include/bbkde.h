@@ -419,7 +419,8 @@ typedef struct {
                         anchor/probe lattices: 16 or 32; 0 = automatic: 32 while a
                         32-point lattice tile spans at most 16 narrowest kernel widths,
                         else 16. 16-point tiles of a separable kernel are summed two
-                        by two, as 32-point ones on the FP32 pipe */
+                        by two, as 32-point ones on the FP32 pipe, so that there the
+                        setting is whether tensor_cores = 0 may take the tensor cores */
   int tensor_cores;  /* factored sums on 32 x 32 tiles (lattices, exact tiles): 0 =
                         automatic: on the tcgen05 tensor cores (each factor split into
                         two TF32 terms, up to ~1e-6 relative error against FP64) when
@@ -448,7 +449,9 @@ typedef struct {
                         probe = exact lattices, residual interpolation and probe
                         check; fallback = exact tiles */
   int64_t probes_used;        /* the probe set the call ran (resolves probes = 0) */
-  int64_t lattice_tile_used;  /* the lattice tile the call ran (resolves lattice_tile = 0) */
+  int64_t lattice_tile_used;  /* the lattice_tile setting that the call ran with (resolves
+                                 0); at 16, separable kernels are summed in 32-point
+                                 tiles on the FP32 pipe */
 } bbkde_grid_stats;
 
 /* Normalised density of the REFERENCE set (with its current attributes, e.g.
