@@ -1747,7 +1747,7 @@ void launch_cull_op(unsigned nblk, cudaStream_t st, const CullArgs &a) {
 // clusters measured slower: 1.57 vs 1.31 ms on the 8192^2 fallback).
 constexpr int kSepResidentPerSm = 12;
 
-template <int OP, int T, int S>
+template <int OP, int T, int S, bool FINE>
 cudaError_t launch_cull_sep_split(unsigned nblk, cudaStream_t st, const CullArgs &a) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nblk * S);
@@ -1761,7 +1761,7 @@ cudaError_t launch_cull_sep_split(unsigned nblk, cudaStream_t st, const CullArgs
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_pair_sum_culled_sep<OP, T, S>, a);
+  return cudaLaunchKernelEx(&cfg, k_pair_sum_culled_sep<OP, T, S, FINE>, a);
 }
 
 // Tensor-core form of the tile-32 factored sum: the dynamic shared memory it
@@ -1788,23 +1788,24 @@ cudaError_t launch_cull_sep_tc(unsigned nblk, cudaStream_t st, const CullArgs &a
 
 // parts = 1: one block per tile; 2, 4, 8: clusters of that many.
 // tc: tile 32 on the tensor cores (k_pair_sum_culled_sep_tc).
-template <int OP, int T>
+template <int OP, int T, bool FINE = false>
 cudaError_t launch_cull_sep_tile(int parts, unsigned nblk, cudaStream_t st, const CullArgs &a) {
   switch (parts) {
-    case 2: return launch_cull_sep_split<OP, T, 2>(nblk, st, a);
-    case 4: return launch_cull_sep_split<OP, T, 4>(nblk, st, a);
-    case 8: return launch_cull_sep_split<OP, T, 8>(nblk, st, a);
+    case 2: return launch_cull_sep_split<OP, T, 2, FINE>(nblk, st, a);
+    case 4: return launch_cull_sep_split<OP, T, 4, FINE>(nblk, st, a);
+    case 8: return launch_cull_sep_split<OP, T, 8, FINE>(nblk, st, a);
     default:
-      k_pair_sum_culled_sep<OP, T><<<nblk, T * T / 8, 0, st>>>(a);
+      k_pair_sum_culled_sep<OP, T, 1, FINE><<<nblk, T * T / 8, 0, st>>>(a);
       return cudaGetLastError();
   }
 }
 template <int OP>
 cudaError_t launch_cull_sep(int tile, int parts, unsigned nblk, cudaStream_t st,
-                            const CullArgs &a, bool tc = false, bool long_list = false) {
+                            const CullArgs &a, bool tc, bool long_list, bool fine) {
   if (tile == 32 && tc) return launch_cull_sep_tc<OP>(nblk, st, a, long_list);
-  return tile == 32 ? launch_cull_sep_tile<OP, 32>(parts, nblk, st, a)
-                    : launch_cull_sep_tile<OP, 16>(parts, nblk, st, a);
+  if (tile == 16) return launch_cull_sep_tile<OP, 16>(parts, nblk, st, a);
+  return fine ? launch_cull_sep_tile<OP, 32, true>(parts, nblk, st, a)
+              : launch_cull_sep_tile<OP, 32>(parts, nblk, st, a);
 }
 
 // Resident factored blocks per SM: 4 at tile 32 (registers), 12 at tile 16.
@@ -1862,9 +1863,10 @@ int sep_parts(const bbkde_ctx *c, int tile, unsigned nblk, int ref_tiles) {
 // part stays below max(rel * S, abs_n) / 2, and *ratio is then the worst skipped
 // bound over that allowance; with abs_n = 0 it is the worst bound over S.
 // sep_tc: a tile-32 factored sum runs on the tensor cores (k_pair_sum_culled_sep_tc).
+// fine: tile-32 sums in partials of 16 references (k_pair_sum_culled_sep's FINE).
 int launch_culled(bbkde_ctx *c, const Resolved &r, unsigned nblk, const CullQueries &q,
                   double rel, bool full, double *pairs, double *ratio,
-                  int sep_tile = 0, double abs_n = 0.0, bool sep_tc = false) {
+                  int sep_tile = 0, double abs_n = 0.0, bool sep_tc = false, bool fine = false) {
   if (nblk == 0) return BBKDE_OK;
   const int level = sep_tile > 0 ? 0 : 1;
   TRY(ensure_culled(c, r, level));
@@ -1909,15 +1911,15 @@ int launch_culled(bbkde_ctx *c, const Resolved &r, unsigned nblk, const CullQuer
     switch (r.op) {
       case OP_GAUSS_ISO:
         CUDA_TRY(c, launch_cull_sep<OP_GAUSS_ISO>(sep_tile, parts, nblk, c->stream, a, tc,
-                                              tc_long));
+                                              tc_long, fine));
         break;
       case OP_GAUSS_PROD:
         CUDA_TRY(c, launch_cull_sep<OP_GAUSS_PROD>(sep_tile, parts, nblk, c->stream, a, tc,
-                                              tc_long));
+                                              tc_long, fine));
         break;
       case OP_EPAN_PROD:
         CUDA_TRY(c, launch_cull_sep<OP_EPAN_PROD>(sep_tile, parts, nblk, c->stream, a, tc,
-                                              tc_long));
+                                              tc_long, fine));
         break;
       default: return fail(c, BBKDE_UNSUPPORTED, "culled sum: kernel does not factor");
     }
@@ -2283,10 +2285,11 @@ GridDesc make_grid(int64_t nx, int64_t ny, double x0, double dx, double y0, doub
 // Exact sums at the points of every listed tile of g (results row-major into out),
 // in the factored form where the kernel factors over the axes unless pair_form.
 // tensor_cores (bbkde_grid_config.tensor_cores): 0 = tile-32 factored sums on the
-// tensor cores when rel >= kSepTcMinRel (culled), 1 = never, 2 = always.
+// tensor cores when rel >= kSepTcMinRel (culled), 1 = never, 2 = always. fine: 32-point
+// tiles in the place of 16-point ones, with those's partials.
 int grid_exact(bbkde_ctx *c, const Resolved &r, const GridDesc &g, const int *list, int64_t n,
                double rel, bool full, double *out, double *pairs, double *ratio,
-               bool pair_form = false, int tensor_cores = 1) {
+               bool pair_form = false, int tensor_cores = 1, bool fine = false) {
   CullQueries q = {};
   q.mode = 1;
   q.tile_list = list;
@@ -2309,7 +2312,7 @@ int grid_exact(bbkde_ctx *c, const Resolved &r, const GridDesc &g, const int *li
   const int64_t pieces = (int64_t)(g.tile / kCullPiece) * (g.tile / kCullPiece);
   const int64_t nblk = sep > 0 ? n : n * pieces;
   if (nblk > INT32_MAX) return fail(c, BBKDE_OUT_OF_RANGE, "grid: too many tiles");
-  return launch_culled(c, r, (unsigned)nblk, q, rel, full, pairs, ratio, sep, 0.0, tc);
+  return launch_culled(c, r, (unsigned)nblk, q, rel, full, pairs, ratio, sep, 0.0, tc, fine);
 }
 
 // Exact sums at every point of g. Tiles of 16 points of a separable kernel are summed as
@@ -2321,7 +2324,7 @@ int grid_exact_all(bbkde_ctx *c, const Resolved &r, const GridDesc &g, DevBuf &o
   const GridDesc gw = wide ? make_grid(g.nx, g.ny, g.x0, g.dx, g.y0, g.dy, 32) : g;
   TRY(tile_order(c, gw, order));
   return grid_exact(c, r, gw, order.as<int>(), (int64_t)gw.ntx * gw.nty, rel, full, out, pairs,
-                    ratio, pair_form, wide ? 1 : tensor_cores);
+                    ratio, pair_form, wide ? 1 : tensor_cores, wide);
 }
 
 // The entries of order[0, n) with a flag, in order, into list; *count of them (waits).
@@ -2696,7 +2699,7 @@ extern "C" int bbkde_eval_grid(bbkde_ctx *c, bbkde_surrogate *sur, const bbkde_k
     TRY(select_flagged(c, c->gr_order.as<int>(), c->gr_flag_ord.as<int>(),
                        c->gr_list.as<int>(), ntiles, &nsel));
     TRY(grid_exact(c, r, g32, c->gr_quad_list.as<int>(), n32, cfg->cull_rel, full, out,
-                   &st.pairs, &st.max_bound_ratio));
+                   &st.pairs, &st.max_bound_ratio, false, 1, true));
   }
   TRY(grid_exact(c, r, g, c->gr_list.as<int>(), nsel, cfg->cull_rel, full, out, &st.pairs,
                  &st.max_bound_ratio, cfg->pair_form != 0, cfg->tensor_cores));
