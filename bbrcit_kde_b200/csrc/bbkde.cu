@@ -1641,14 +1641,14 @@ constexpr double kGridLatticeSpan = 16.0;
 // (262,144 references, ms in 16-point tiles / as 32-point ones with those's partials:
 // 1,000 x 900 points 1.44 / 0.96, 500 x 450 1.18 / 0.42, 250 x 225 0.51 / 0.28, 64 x 64
 // 0.44 / 0.47), the pipeline's flagged tiles in blocks with at least kGridQuadMin of their
-// tiles flagged (the 32-point kernel sums about 1.7x the pairs per second; 8,714 tiles of
-// 10^6 references 8.8 -> 7.7 ms) where that is worth the list of blocks: sorting and
-// selecting it are a dozen launches and two waits, 100-150 us. A flagged tile takes about
-// 0.5 ns sqrt(n) with n references (0.02 us at 1,000, 0.3 at 400,000), so that a fifth of
-// the list's time exceeds that from tiles x sqrt(n) = kGridQuadWork on, about 0.75 ms.
-// Fallback us without / with blocks: 1,000 references 14,100 tiles 351 / 377, 48,162 tiles
-// 881 / 825; 25,000 references 3,844 tiles 365 / 424, 13,749 tiles 948 / 775; 400,000
-// references 3,347 tiles 1,360 / 1,245, 9,791 tiles 3,948 / 3,384.
+// tiles flagged (the 32-point kernel sums about 1.5x the pairs per second) where that is
+// worth the list of blocks: sorting and selecting it are a dozen launches and two waits,
+// 100-150 us. A flagged tile takes about 0.5 ns sqrt(n) with n references (0.02 us at
+// 1,000, 0.35 at 400,000), so that a fifth of the list's time exceeds that from tiles x
+// sqrt(n) = kGridQuadWork on, about 0.75 ms. Fallback us without / with blocks: 1,000
+// references 14,099 tiles 354 / 358, 52,340 tiles 937 / 827; 25,000 references 3,844 tiles
+// 359 / 427, 13,749 tiles 952 / 810; 400,000 references 3,893 tiles 1,394 / 1,280, 13,478
+// tiles 4,213 / 3,306, but 4,016 tiles of nearly empty regions 476 / 600.
 constexpr int64_t kGridQuadTiles = 1024;   // never below: the parts of short lists are better
 constexpr double kGridQuadWork = 1.5e6;
 constexpr int kGridQuadMin = 3;
