@@ -214,6 +214,8 @@ void *pinned_buffer(bbkde_ctx *c) {
       if (cudaPointerGetAttributes(&at, pool.kept.back()) == cudaSuccess &&
           at.type == cudaMemoryTypeHost)
         c->pinned = pool.kept.back();
+      else
+        cudaGetLastError();
       pool.kept.pop_back();
     }
   }
