@@ -22,9 +22,9 @@
 //   1. M = the largest e over the block's box;
 //   2. sum every tile with e >= M - cut (the near field);
 //   3. with S = the smallest near-field sum of the block's queries and the allowance
-//      A = max(rel * S, abs), also sum every remaining tile that reaches e >= T, the
-//      largest threshold (on a grid of whole bits) at which the bounds of the tiles left
-//      out add up to no more than A / 2 (cull_far_level).
+//      A = max(rel * S, abs), also sum every remaining tile that reaches e >= T =
+//      log2(A / n_tiles) - kFarMargin: all the tiles left out hold at most A / 64. (The
+//      factored grid kernels count the bounds instead: cull_far_level, at most 9/32.)
 // So the skipped part of every query q of the block is below A / 2 <= max(rel * S_q,
 // abs) / 2:
 // every culled sum is within rel of the full sum, or within abs of it, whichever
@@ -337,9 +337,8 @@ __device__ __forceinline__ int cull_pass(const CullArgs &a, const CullGroups &gr
 //     (a 1-D likelihood to 1e-6: off by 4.7e-7 with a quarter, 6.8e-8 with this).
 //   Together at most 1/4 + 1/32 = 9/32 of the allowance.
 // A threshold of -log2(n_tiles) - 1 for every tile, which needs no count, charges each of
-// them as much as the nearest one left out and lies two to three bits lower: 400,000 x
-// 300,000 at 1e-6 lists 3.71e9 pairs instead of 4.10e9 (1.62 -> 1.57 ms), the flagged
-// tiles of a 4,096^2 pipeline at 1e-5 take 7.0 ms instead of 7.8.
+// them as much as the nearest one left out and lies two to three bits lower: the flagged
+// tiles of a 4,096^2 pipeline at 1e-5 take 7.8 ms instead of 7.0.
 // level(t): the largest bound of t over the block's slots relative to their allowances,
 // -inf for a tile that is summed already or flushes to zero; a group's is at least its
 // members'. Every thread calls it and gets the result.
@@ -373,6 +372,15 @@ __device__ __forceinline__ float cull_far_level(const CullArgs &a, const CullGro
   return fminf(t, -2.0f);
 }
 
+// Far threshold of the pair form: bits below the allowance's share of one tile. What is
+// left out is always missing on the same side, so it adds up over a likelihood's points,
+// and blocks of 64 queries have few tiles beyond the needed ones to make up for it. Error
+// of a 1-D likelihood (51,330 points) and an adaptive density (123,398 references) to 1e-6:
+// 5.5e-8 and 9.1e-8 with the counted threshold, 5.9e-9 and 7.7e-8 with 3 bits, 3.4e-9 and
+// 7.7e-8 with 6 (256-reference tiles in blocks of 1,024 queries: 3.8e-9 and 7.7e-8); 0.93,
+// 0.95 and 0.93 ms, 2.03, 2.13 and 2.23 ms.
+constexpr float kFarMargin = 6.0f;
+
 template <int OP, int D>
 __global__ void __launch_bounds__(32 * kCullWarps, 4) k_pair_sum_culled(CullArgs a) {
   constexpr int BLOCK = 32 * kCullWarps;
@@ -393,7 +401,6 @@ __global__ void __launch_bounds__(32 * kCullWarps, 4) k_pair_sum_culled(CullArgs
   __shared__ double s_sum[NW][kCullQpb];
   __shared__ double s_min[kCullQpb / 32];
   __shared__ double s_skip[NW];
-  __shared__ int s_bins[kFarBins];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float2 qx[QPT], qy[QPT];   // (x, x), (y, y): two references per packed operation
@@ -441,7 +448,8 @@ __global__ void __launch_bounds__(32 * kCullWarps, 4) k_pair_sum_culled(CullArgs
   // Skipped bound relative to the threshold: 2^(e - T) < 1 per skipped unit (terms below
   // 2^-126 of the threshold flush; they are negligible). ex2.approx errs by ~2^-22
   // relative, inside the 1% mass slack.
-  float skipped = 0.f, la = 0.f, t0 = 0.f, tn = 0.f;   // log2 A; relative thresholds
+  float skipped = 0.f, la = 0.f;   // log2 A
+  const float tn = -log2f((float)a.n_tiles) - kFarMargin;   // threshold relative to A
   int summed = 0;
 
   // Is tile (or group) t needed? phase 0: Epanechnikov (support of the box);
@@ -457,7 +465,7 @@ __global__ void __launch_bounds__(32 * kCullWarps, 4) k_pair_sum_culled(CullArgs
     const bool near = e >= t_a;
     if (phase == 1) return near;
     if (near && !group) return false;   // already summed
-    if (e - la >= (group ? t0 : tn)) return true;
+    if (e - la >= tn) return true;
     skipped += ex2_approx(e - la - tn);
     return false;
   };
@@ -568,11 +576,6 @@ __global__ void __launch_bounds__(32 * kCullWarps, 4) k_pair_sum_culled(CullArgs
     // allowance 0 (smin <= 0 and no abs): every tile that does not flush to zero
     const double allow = fmax(a.rel * smin, a.abs_n);
     la = allow > 0.0 ? (float)log2(allow) : -INFINITY;
-    t0 = -log2f((float)a.n_tiles) - 2.0f;
-    tn = cull_far_level<BLOCK>(a, groups, s_bins, t0, [&](const RefTile &t, bool group) {
-      const float pb = tile_peak<OP, D>(t, qx0, qx1, qy0, qy1), e = t.lm + pb;
-      return pb < kFlushExp || (!group && e >= t_a) ? -INFINITY : e - la;
-    });
     pass(2);   // scan 3: far field, bound of the rest
     // Bound of the skipped part (fixed-order reduction) over the allowance.
     double sk = skipped;
